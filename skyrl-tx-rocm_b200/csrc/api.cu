@@ -36,34 +36,36 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-static int encode(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t rank, const void* base, const cuuint64_t* dims,
-                  const cuuint64_t* strides, const cuuint32_t* box) {
+static int encode(CUtensorMap* map, CUtensorMapDataType dtype, int elem_bytes, uint32_t rank, const void* base,
+                  const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return fail(SKYRL_ERR_DRIVER, "cuTensorMapEncodeTiled is not available from the CUDA driver");
   const cuuint32_t estr[3] = {1, 1, 1};
+  const uint32_t width = box[0] * static_cast<uint32_t>(elem_bytes);  // the swizzle spans the box's inner extent
+  const CUtensorMapSwizzle swizzle = width >= 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                     : width >= 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                   : CU_TENSOR_MAP_SWIZZLE_32B;
   CUresult r = fn(map, dtype, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(SKYRL_ERR_INVALID_ARGUMENT, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return SKYRL_OK;
 }
 
 int encode_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, int elem_bytes, const void* base, uint64_t inner,
                    uint64_t outer, uint64_t row_pitch_bytes, uint32_t box_inner, uint32_t box_outer) {
-  (void)elem_bytes;
   const cuuint64_t dims[2] = {inner, outer};
   const cuuint64_t strides[1] = {row_pitch_bytes};
   const cuuint32_t box[2] = {box_inner, box_outer};
-  return encode(map, dtype, 2, base, dims, strides, box);
+  return encode(map, dtype, elem_bytes, 2, base, dims, strides, box);
 }
 
 int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dtype, int elem_bytes, const void* base, uint64_t d0,
                    uint64_t d1, uint64_t d2, uint64_t pitch1_bytes, uint64_t pitch2_bytes, uint32_t box0,
                    uint32_t box1, uint32_t box2) {
-  (void)elem_bytes;
   const cuuint64_t dims[3] = {d0, d1, d2};
   const cuuint64_t strides[2] = {pitch1_bytes, pitch2_bytes};
   const cuuint32_t box[3] = {box0, box1, box2};
-  return encode(map, dtype, 3, base, dims, strides, box);
+  return encode(map, dtype, elem_bytes, 3, base, dims, strides, box);
 }
 
 int sm_count() {
@@ -82,19 +84,13 @@ int sm_count() {
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 constexpr int MAX_CHUNKS = 16;
-constexpr int SCHED_WORDS = 8;  // room for four {claimed, finished} pairs of the GEMMs' dynamic tile scheduler
+constexpr int SCHED_WORDS = ZERO_WORDS;  // room for four {claimed, finished} pairs of the GEMMs' dynamic tile scheduler
 
-// Tiles one chunk of `rows` sorted rows can hold: every adapter may end a partial tile inside it.
-static inline int tile_cap(int rows, int num_adapters) {
-  return (rows + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS + (num_adapters > 0 ? num_adapters : 1) + 1;
-}
-static inline int max_tiles_for(int m, int num_adapters) { return tile_cap(m, num_adapters); }
-// Capacity of the tile buffer: the unchunked list, or MAX_CHUNKS per-chunk lists, whichever is larger.
-static inline size_t tile_buffer_slots(int m, int num_adapters) {
-  const size_t whole = static_cast<size_t>(max_tiles_for(m, num_adapters));
-  const size_t chunked = static_cast<size_t>(m) / SKYRL_TILE_ROWS + 2 * MAX_CHUNKS +
-                         static_cast<size_t>(MAX_CHUNKS) * ((num_adapters > 0 ? num_adapters : 1) + 1);
-  return whole > chunked ? whole : chunked;
+// Dense tiles of the sorted rows (tiles.cuh): tile i is rows 128 i ...; segments (tile, adapter) never number more than
+// tiles + adapters.
+static inline int dense_tiles(int rows) { return (rows + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS; }
+static inline size_t segment_slots(int m, int num_adapters) {
+  return static_cast<size_t>(dense_tiles(m)) + (num_adapters > 0 ? num_adapters : 1);
 }
 
 struct Carver {
@@ -114,10 +110,36 @@ struct Carver {
 // Batches of at most this many rows take the row-wise LoRA path (no adapter sort, one M tile).
 constexpr int ROWS_PATH_MAX_M = SKYRL_TILE_ROWS;
 
-struct LinearWs {
+struct RouteWs {
   int32_t* perm;
   int32_t* tiles;
-  int32_t* num_tiles;
+  int32_t* seg_mask;
+  int32_t* seg_adapter;
+};
+static RouteWs carve_route(Carver& c, int m, int num_adapters) {
+  RouteWs r;
+  r.perm = c.take<int32_t>(m);
+  r.tiles = c.take<int32_t>(4 * static_cast<size_t>(dense_tiles(m)));
+  r.seg_mask = c.take<int32_t>(4 * segment_slots(m, num_adapters));
+  r.seg_adapter = c.take<int32_t>(segment_slots(m, num_adapters));
+  return r;
+}
+// Tiles of sorted rows [row0, row0 + rows), row0 a multiple of 128; without routing they are computed, not listed.
+static TileSource tile_source(const RouteWs& r, bool routed, int row0, int rows) {
+  TileSource t = {};
+  t.count = dense_tiles(rows);
+  t.row0 = row0;
+  t.row_end = row0 + rows;
+  if (routed) {
+    t.tiles = reinterpret_cast<const int4*>(r.tiles) + row0 / SKYRL_TILE_ROWS;
+    t.seg_mask = reinterpret_cast<const int4*>(r.seg_mask);
+    t.seg_adapter = r.seg_adapter;
+  }
+  return t;
+}
+
+struct LinearWs {
+  RouteWs route;
   int8_t* xq;
   float* sx;
   uint16_t* xn;
@@ -130,10 +152,7 @@ struct LinearWs {
 static LinearWs carve_linear(void* ws, int m, int n, int k, int num_adapters) {
   Carver c(ws);
   LinearWs w;
-  const int mt = max_tiles_for(m, num_adapters);
-  w.perm = c.take<int32_t>(m);
-  w.tiles = c.take<int32_t>(4 * static_cast<size_t>(mt));
-  w.num_tiles = c.take<int32_t>(4);
+  w.route = carve_route(c, m, num_adapters);
   w.sched = c.take<int32_t>(SCHED_WORDS);
   w.xq = c.take<int8_t>(static_cast<size_t>(m) * k);
   w.sx = c.take<float>(m);
@@ -150,9 +169,7 @@ static LinearWs carve_linear(void* ws, int m, int n, int k, int num_adapters) {
 }
 
 struct MlpWs {
-  int32_t* perm;
-  int32_t* tiles;
-  int32_t* num_tiles;
+  RouteWs route;
   int8_t* xq;
   float* sx;
   uint16_t* xn;
@@ -169,11 +186,7 @@ struct MlpWs {
 static MlpWs carve_mlp(void* ws, int m, int hidden, int inter, int num_adapters) {
   Carver c(ws);
   MlpWs w;
-  const int mt = max_tiles_for(m, num_adapters);
-  w.perm = c.take<int32_t>(m);
-  (void)mt;
-  w.tiles = c.take<int32_t>(4 * tile_buffer_slots(m, num_adapters));
-  w.num_tiles = c.take<int32_t>(MAX_CHUNKS + 4);
+  w.route = carve_route(c, m, num_adapters);
   w.sched = c.take<int32_t>(SCHED_WORDS);
   w.xq = c.take<int8_t>(static_cast<size_t>(m) * hidden);
   w.sx = c.take<float>(m);
@@ -215,13 +228,15 @@ struct Projection {
   float eps;
   const int32_t* gather;  // row gather for the quantiser (sorted route) or NULL
   bool keep_xn;           // sorted route: x must be re-laid out (gathered / normalised) for the projection MMA
-  int m, n, k, rank, na, mt;
+  int m, n, k, rank, na;
   int q_row0, q_rows;     // sorted rows the quantiser stage covers (a chunk of the block, or all m rows)
   int list_row0;          // first sorted row of the tile list `tiles` (0, or the first row of the call's chunk)
   bool skip_quant;        // the quantiser stage of these rows already ran (its outputs are in xq / sx / z_parts)
   int gemm_variant;       // SKYRL_GEMM_VARIANT_* forced on the GEMM (0: the library chooses)
   bool two_step_rows;     // row-wise route: GEMM to an int32 accumulator in memory + finalize kernel (default)
   const float* known_amax;  // absmax of every source row, if the producer of x collected it (sorted route)
+  float* zero_amax;         // quantiser stage: row absmax words it clears for the GEMM behind it (nullable)
+  int32_t* zero_words;      // quantiser stage: scheduler words it clears where no routing kernel runs (nullable)
   float* row_amax;          // SwiGLU epilogue: collect the absmax of every output row here
   int cta_limit;
   void* const* scatter_bases;  // row scatter of the fp32 partial sums (see SkyrlW8A8GemmArgs) or NULL
@@ -240,8 +255,7 @@ struct Projection {
   uint16_t* xn;
   uint16_t* z_parts;
   int32_t* acc;
-  const int32_t* tiles;
-  const int32_t* num_tiles;
+  TileSource src;
   int epilogue;
   const int32_t* out_row_map;
   const void* residual;
@@ -274,13 +288,14 @@ static int run_quant_stage(const Projection& q, cudaStream_t stream) {
   } else if ((rc = launch_rms_quant(xsrc, q.x_stride, q.rms_delta, q.eps,
                                     q.gather != nullptr ? q.gather + r0 : nullptr, rows, q.k,
                                     q.xq + static_cast<size_t>(r0) * q.k, q.sx + r0,
-                                    need_xn ? q.xn + static_cast<size_t>(r0) * q.k : nullptr, stream))) {
+                                    need_xn ? q.xn + static_cast<size_t>(r0) * q.k : nullptr, stream,
+                                    q.zero_amax != nullptr ? q.zero_amax + r0 : nullptr, q.zero_words))) {
     return rc;
   }
   if (lora) {
     const void* xa = need_xn ? static_cast<const void*>(q.xn) : q.x;
-    if ((rc = launch_lora_a_proj(xa, q.m, q.k, q.a_packed, q.scaling, q.na, q.rank, q.tiles, q.num_tiles, q.mt,
-                                 q.z_parts, q.status, stream, r0, r0 + rows, nullptr, 0, q.list_row0)))
+    if ((rc = launch_lora_a_proj(xa, q.m, q.k, q.a_packed, q.scaling, q.na, q.rank, q.src, q.src.count, q.z_parts, q.status,
+                                 stream, r0, r0 + rows, nullptr, 0, q.list_row0)))
       return rc;
   }
   return SKYRL_OK;
@@ -305,15 +320,11 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
     g.n = q.n;
     g.k = q.k;
     g.num_adapters = q.na;
-    g.max_tiles = q.mt;
     g.xq = q.xq;
     g.sx = q.sx;
     g.wq = q.wq;
     g.sw = q.sw;
-    g.tiles = q.tiles;
-    g.num_tiles = q.num_tiles;
     g.status = q.status;
-    g.sched = q.sched;
     g.prefetch = q.prefetch;
     g.prefetch_bytes = q.prefetch_bytes;
     if (!q.two_step_rows) {
@@ -330,7 +341,7 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
       g.out = q.out;
       g.out_row_stride = q.out_stride;
       if (q.ev_begin != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_begin), stream);
-      rc = launch_gemm(g, stream, chain);
+      rc = launch_gemm(g, stream, chain, &q.src);
       if (q.ev_end != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_end), stream);
       return rc;
     }
@@ -343,7 +354,7 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
     g.out = q.acc;
     g.out_row_stride = q.n;
     if (q.ev_begin != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_begin), stream);
-    rc = launch_gemm(g, stream, chain);
+    rc = launch_gemm(g, stream, chain, &q.src);
     if (q.ev_end != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_end), stream);
     if (rc) return rc;
     return launch_finalize_rows(q.epilogue, q.acc, slabs, q.sx, q.sw, z_rows, q.ids, q.na,
@@ -361,14 +372,15 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
   g.n = q.n;
   g.k = q.k;
   g.num_adapters = q.na;
-  g.max_tiles = q.mt;
   g.xq = q.xq;
   g.sx = q.sx;
   g.wq = q.wq;
   g.sw = q.sw;
   g.lora_b_packed = q.b_packed;
-  g.tiles = q.tiles;
-  g.num_tiles = q.num_tiles;
+  if (lora && q.b_rows != nullptr) {
+    g.lora_b_rows = q.b_rows;
+    g.lora_b_rows_rank = q.b_rows_rank;
+  }
   g.out_row_map = q.out_row_map;
   g.residual = q.residual;
   g.out = q.out;
@@ -379,9 +391,11 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
   g.variant = q.gemm_variant;
   g.cta_limit = q.cta_limit;
   if (q.row_amax != nullptr && q.epilogue == SKYRL_EPI_SWIGLU) {
-    const int r0 = q.q_row0, rows = q.q_rows > 0 ? q.q_rows : q.m;
-    cudaError_t e = cudaMemsetAsync(q.row_amax + r0, 0, static_cast<size_t>(rows) * sizeof(float), stream);
-    if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "row_amax memset: %s", cudaGetErrorString(e));
+    if (q.skip_quant) {  // no quantiser stage in this call to clear it
+      const int r0 = q.q_row0, rows = q.q_rows > 0 ? q.q_rows : q.m;
+      cudaError_t e = cudaMemsetAsync(q.row_amax + r0, 0, static_cast<size_t>(rows) * sizeof(float), stream);
+      if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "row_amax memset: %s", cudaGetErrorString(e));
+    }
     g.row_amax = q.row_amax;
   }
   if (q.scatter_bases != nullptr && q.scatter_rows > 0) {
@@ -390,7 +404,9 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
     g.scatter_rows = q.scatter_rows;
   }
   if (q.ev_begin != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_begin), stream);
-  rc = launch_gemm(g, stream);
+  // launched programmatically behind this call's own quantiser stage: what it reads before its wait (the tile list)
+  // then comes from at least two kernels back
+  rc = launch_gemm(g, stream, !q.skip_quant && q.ev_begin == nullptr && q.ev_end == nullptr, &q.src);
   if (q.ev_end != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_end), stream);
   return rc;
 }
@@ -433,19 +449,18 @@ extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, sk
   const LinearWs w = carve_linear(a->workspace, a->m, a->n, a->k, na);
   int rc = check_ws(a->workspace, a->workspace_bytes, w.bytes, "linear");
   if (rc) return rc;
-  const int mt = max_tiles_for(a->m, na);
   const bool rows_path = a->m <= ROWS_PATH_MAX_M;
   const bool routed = a->adapter_ids != nullptr && !rows_path;
 
-  if ((rc = launch_route(routed ? a->adapter_ids : nullptr, a->m, na, w.perm, w.tiles, w.num_tiles, mt, a->status,
-                         stream, 0, 0, w.sched, SCHED_WORDS)))
+  if (routed && (rc = launch_route_dense(a->adapter_ids, a->m, na, w.route.perm, w.route.tiles, w.route.seg_mask,
+                                         w.route.seg_adapter, a->status, stream, w.sched, SCHED_WORDS)))
     return rc;
   Projection q = {};
   q.x = a->x;
   q.x_stride = a->x_row_stride;
   q.rms_delta = a->rms_delta;
   q.eps = a->rms_eps;
-  q.gather = routed ? w.perm : nullptr;
+  q.gather = routed ? w.route.perm : nullptr;
   q.keep_xn = routed || a->rms_delta != nullptr || a->x_row_stride != a->k;
   q.two_step_rows = (a->flags & SKYRL_LINEAR_FUSED_ROWS) == 0;
   q.gemm_variant = static_cast<int>((a->flags >> SKYRL_FLAGS_GEMM_VARIANT_SHIFT) & 7u);
@@ -454,7 +469,6 @@ extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, sk
   q.k = a->k;
   q.rank = a->rank;
   q.na = na;
-  q.mt = mt;
   q.wq = a->wq;
   q.sw = a->sw;
   q.a_packed = a->lora_a_packed;
@@ -468,16 +482,16 @@ extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, sk
   q.acc = w.acc;
   q.b_rows = a->lora_b_rows;
   q.b_rows_rank = a->lora_b_rows_rank;
-  q.tiles = w.tiles;
-  q.num_tiles = w.num_tiles;
+  q.src = tile_source(w.route, routed, 0, a->m);
   q.epilogue = a->epilogue;
-  q.out_row_map = routed ? w.perm : nullptr;
+  q.out_row_map = routed ? w.route.perm : nullptr;
   q.residual = a->residual;
   q.residual_stride = a->residual_row_stride;
   q.out = a->out;
   q.out_stride = a->out_row_stride;
   q.status = a->status;
-  q.sched = w.sched;
+  if (!rows_path) q.sched = w.sched;
+  if (!routed && !rows_path) q.zero_words = w.sched;
   q.ev_begin = a->timing_events[0];
   q.ev_end = a->timing_events[1];
   return run_projection(q, stream);
@@ -516,9 +530,8 @@ struct MlpPlan {
   int na;
   bool rows_path, routed, chunked;
   const int32_t* perm;
-  int chunk_rows, chunk_cap, mt, row0, rows;
-  const int32_t* tiles;
-  const int32_t* num_tiles;
+  int chunk_rows, row0, rows;
+  TileSource src;
 };
 
 static int plan_mlp(const SkyrlW8A8MlpArgs* a, const char* who, MlpPlan* pl) {
@@ -546,27 +559,24 @@ static int plan_mlp(const SkyrlW8A8MlpArgs* a, const char* who, MlpPlan* pl) {
   if (rc) return rc;
   pl->rows_path = a->m <= ROWS_PATH_MAX_M;
   pl->routed = a->adapter_ids != nullptr && !pl->rows_path;
-  pl->perm = pl->routed ? pl->w.perm : nullptr;
+  pl->perm = pl->routed ? pl->w.route.perm : nullptr;
   pl->chunked = a->num_chunks > 1 && !pl->rows_path;
   if (pl->chunked && (a->num_chunks > MAX_CHUNKS || a->chunk_index < 0 || a->chunk_index >= a->num_chunks))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "%s: num_chunks must be <= %d and chunk_index inside it", who, MAX_CHUNKS);
   pl->chunk_rows = pl->chunked ? ((a->m + a->num_chunks - 1) / a->num_chunks + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS *
                                      SKYRL_TILE_ROWS
                                : 0;
-  pl->chunk_cap = pl->chunked ? tile_cap(pl->chunk_rows, pl->na) : 0;
-  pl->mt = pl->chunked ? pl->chunk_cap : max_tiles_for(a->m, pl->na);
   pl->row0 = pl->chunked ? a->chunk_index * pl->chunk_rows : 0;
   pl->rows = pl->chunked ? (a->m - pl->row0 < pl->chunk_rows ? a->m - pl->row0 : pl->chunk_rows) : a->m;
-  pl->tiles = pl->chunked ? pl->w.tiles + 4 * static_cast<size_t>(a->chunk_index) * pl->chunk_cap : pl->w.tiles;
-  pl->num_tiles = pl->chunked ? pl->w.num_tiles + a->chunk_index : pl->w.num_tiles;
+  pl->src = tile_source(pl->w.route, pl->routed, pl->row0, pl->rows > 0 ? pl->rows : 0);
   return SKYRL_OK;
 }
 
 static int route_mlp(const SkyrlW8A8MlpArgs* a, const MlpPlan& pl, cudaStream_t stream) {
-  if ((a->flags & SKYRL_MLP_REUSE_ROUTING) != 0) return SKYRL_OK;
-  return launch_route(pl.routed ? a->adapter_ids : nullptr, a->m, pl.na, pl.w.perm, pl.w.tiles, pl.w.num_tiles,
-                      static_cast<int>(tile_buffer_slots(a->m, pl.na)), a->status, stream, pl.chunk_rows, pl.chunk_cap,
-                      pl.w.sched, SCHED_WORDS);
+  if ((a->flags & SKYRL_MLP_REUSE_ROUTING) != 0 || !pl.routed) return SKYRL_OK;
+  const RouteWs& r = pl.w.route;
+  return launch_route_dense(a->adapter_ids, a->m, pl.na, r.perm, r.tiles, r.seg_mask, r.seg_adapter, a->status, stream,
+                            pl.w.sched, SCHED_WORDS);
 }
 
 // front half: RMSNorm -> quant -> gate_up W8A8 LoRA -> SwiGLU; h keeps the row order of the GEMM
@@ -587,7 +597,6 @@ static Projection front_projection(const SkyrlW8A8MlpArgs* a, const MlpPlan& pl)
   q.k = a->hidden;
   q.rank = a->rank;
   q.na = pl.na;
-  q.mt = pl.mt;
   q.q_row0 = pl.row0;
   q.q_rows = pl.rows;
   q.list_row0 = pl.row0;
@@ -605,8 +614,7 @@ static Projection front_projection(const SkyrlW8A8MlpArgs* a, const MlpPlan& pl)
   q.acc = w.acc;
   q.b_rows = a->gu_b_rows;
   q.b_rows_rank = a->b_rows_rank;
-  q.tiles = pl.tiles;
-  q.num_tiles = pl.num_tiles;
+  q.src = pl.src;
   q.epilogue = SKYRL_EPI_SWIGLU;
   q.out_row_map = nullptr;
   q.out = w.h;
@@ -614,7 +622,9 @@ static Projection front_projection(const SkyrlW8A8MlpArgs* a, const MlpPlan& pl)
   q.status = a->status;
   // odd and even chunks claim tiles through counter pairs of their own, so that two chunks of one block may run
   // on two streams at the same time
-  q.sched = w.sched + (pl.chunked ? (a->chunk_index & 1) * 4 : 0);
+  // (Without adapter ids no routing kernel runs to clear the words: a whole block's quantiser does, the chunks of a
+  // block without ids take their tiles with a fixed stride.)
+  if (pl.routed || (!pl.rows_path && !pl.chunked)) q.sched = w.sched + (pl.chunked ? (a->chunk_index & 1) * 4 : 0);
   q.ev_begin = a->timing_events[0];
   q.ev_end = a->timing_events[1];
   return q;
@@ -640,6 +650,11 @@ extern "C" int skyrl_w8a8_mlp_block_sm100_v1(const SkyrlW8A8MlpArgs* a, skyrl_st
   // streaming pass (SKYRL_MLP_NO_ROW_AMAX keeps the two-pass quantiser; the two must agree bit for bit)
   const bool collect = !pl.rows_path && (a->flags & SKYRL_MLP_NO_ROW_AMAX) == 0;
   q.row_amax = collect ? w.h_amax : nullptr;
+  q.zero_amax = q.row_amax;
+  if (!pl.routed && !pl.rows_path && !pl.chunked) {
+    if (prepared) q.sched = nullptr;  // the rows were prepared by a call of their own
+    else q.zero_words = w.sched;
+  }
   if (pl.rows_path && a->prefetch_down_bytes > 0) {
     // the down weights travel to L2 while the row-wise kernels behind gate_up run
     const int64_t dn_bytes = static_cast<int64_t>((a->inter + SKYRL_WEIGHT_KBLOCK - 1) / SKYRL_WEIGHT_KBLOCK) * a->hidden * SKYRL_WEIGHT_KBLOCK;
@@ -651,6 +666,8 @@ extern "C" int skyrl_w8a8_mlp_block_sm100_v1(const SkyrlW8A8MlpArgs* a, skyrl_st
   // back half: quant(h) -> down W8A8 LoRA -> + residual, rows scattered back to token order
   q.skip_quant = false;
   q.row_amax = nullptr;
+  q.zero_amax = nullptr;
+  q.zero_words = nullptr;
   q.known_amax = collect ? w.h_amax : nullptr;
   q.x = w.h;
   q.x_stride = a->inter;
@@ -667,7 +684,7 @@ extern "C" int skyrl_w8a8_mlp_block_sm100_v1(const SkyrlW8A8MlpArgs* a, skyrl_st
   q.scaling = a->dn_scaling;
   q.xq = w.hq;
   q.sx = w.sh;
-  q.sched += 2;
+  if (q.sched != nullptr) q.sched += 2;
   q.prefetch = nullptr;
   q.prefetch_bytes = 0;
   if (pl.rows_path && a->prefetch_next != nullptr && a->prefetch_next_bytes > 0) {
@@ -805,7 +822,7 @@ extern "C" int skyrl_w8a8_mlp_tp_exchange_sm100_v1(const SkyrlW8A8MlpArgs* blk, 
     }
     if (extra_count > 7) return fail(SKYRL_ERR_INVALID_ARGUMENT, "tp_exchange: this rank's workspace is not among peer_workspaces");
     if ((rc = launch_lora_a_proj(np.w.xn, next->m, next->hidden, next->gu_a_packed, next->gu_scaling, np.na, next->rank,
-                                 np.tiles, np.num_tiles, np.mt, np.w.z_parts, next->status, stream, x->row_begin,
+                                 np.src, np.src.count, np.w.z_parts, next->status, stream, x->row_begin,
                                  x->row_begin + x->row_count, extra, extra_count, np.row0)))
       return rc;
   }
@@ -821,7 +838,7 @@ extern "C" int skyrl_w8a8_mlp_workspace_stage_regions(int32_t m, int32_t hidden,
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "workspace_stage_regions: bad argument");
   unsigned char* const base = reinterpret_cast<unsigned char*>(static_cast<uintptr_t>(1024));
   const MlpWs w = carve_mlp(base, m, hidden, inter, num_adapters > 0 ? num_adapters : 1);
-  offsets[0] = static_cast<size_t>(reinterpret_cast<unsigned char*>(w.perm) - base);
+  offsets[0] = static_cast<size_t>(reinterpret_cast<unsigned char*>(w.route.perm) - base);
   offsets[1] = static_cast<size_t>(reinterpret_cast<unsigned char*>(w.h) - base);
   offsets[2] = static_cast<size_t>(reinterpret_cast<unsigned char*>(w.hq) - base);
   offsets[3] = static_cast<size_t>(reinterpret_cast<unsigned char*>(w.sh) - base);
@@ -854,7 +871,7 @@ extern "C" int skyrl_w8a8_mlp_tp_finalize_sm100_v1(const SkyrlW8A8MlpArgs* a, co
   if (rc) return rc;
   const void* residual = a->residual != nullptr ? a->residual : a->x;
   const bool routed = a->adapter_ids != nullptr && a->m > ROWS_PATH_MAX_M;
-  return launch_tp_finalize(reduced, routed ? w.perm : nullptr, residual, out, a->hidden, row_begin, row_count, stream,
+  return launch_tp_finalize(reduced, routed ? w.route.perm : nullptr, residual, out, a->hidden, row_begin, row_count, stream,
                             (a->flags & SKYRL_MLP_FINALIZE_SORTED) != 0);
 }
 
@@ -876,7 +893,7 @@ extern "C" int skyrl_w8a8_mlp_tp_finalize_slabs_sm100_v1(const SkyrlW8A8MlpArgs*
   if (rc) return rc;
   const void* residual = a->residual != nullptr ? a->residual : a->x;
   const bool routed = a->adapter_ids != nullptr && a->m > ROWS_PATH_MAX_M;
-  return launch_tp_finalize_slabs(slabs, num_slabs, routed ? w.perm : nullptr, residual, out, a->hidden, row_begin,
+  return launch_tp_finalize_slabs(slabs, num_slabs, routed ? w.route.perm : nullptr, residual, out, a->hidden, row_begin,
                                   row_count, stream, (a->flags & SKYRL_MLP_FINALIZE_SORTED) != 0);
 }
 
@@ -933,10 +950,6 @@ extern "C" int skyrl_w8a8_lora_forward_noalloc_sm100_v1(const SkyrlW8A8LinearArg
                 "noalloc linear: m=%d, n=%d, k=%d needs %zu bytes of scratch, the built-in array holds %zu "
                 "(SKYRL_NOALLOC_SCRATCH_BYTES = %u); use skyrl_w8a8_lora_forward_sm100_v1 with a workspace",
                 a->m, a->n, a->k, w.bytes, avail, SKYRL_NOALLOC_SCRATCH_BYTES);
-  // The array keeps the previous call's contents.  Nothing in it is accumulated into, but the
-  // tile count is cleared so that a failed routing pass can never expose a stale count.
-  cudaError_t e = cudaMemsetAsync(w.num_tiles, 0, 4 * sizeof(int32_t), static_cast<cudaStream_t>(stream_));
-  if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "noalloc linear: memset: %s", cudaGetErrorString(e));
   SkyrlW8A8LinearArgs b = *a;
   b.workspace = base;
   b.workspace_bytes = avail;

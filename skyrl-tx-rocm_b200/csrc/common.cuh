@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "../../include/skyrl_w8a8_sm100.h"
+#include "tiles.cuh"
 
 namespace skyrl {
 
@@ -14,7 +15,7 @@ int fail(int code, const char* fmt, ...);
 
 // cuTensorMapEncodeTiled resolved through the runtime (no link-time libcuda
 // dependency, so the library loads on a machine without a driver).
-// 2-D / 3-D row-major tensors, 128-byte swizzle, zero fill out of bounds.
+// 2-D / 3-D row-major tensors, swizzle of the box's inner extent (32, 64 or 128 bytes), zero fill out of bounds.
 int encode_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, int elem_bytes, const void* base, uint64_t inner,
                    uint64_t outer, uint64_t row_pitch_bytes, uint32_t box_inner, uint32_t box_outer);
 int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dtype, int elem_bytes, const void* base, uint64_t d0,
@@ -66,16 +67,20 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, int bytes, bool (&done)[MA
 int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* num_tiles,
                  int max_tiles, int32_t* status, cudaStream_t stream, int chunk_rows = 0, int chunk_cap = 0,
                  int32_t* zero_words = nullptr, int zero_count = 0);
+int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* seg_mask,
+                       int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count);
 int launch_grad_quant(const void* dy, int64_t dy_row_stride, const float* col_scale, const int32_t* row_map, int m, int n,
                       void* q1, float* s1, void* q2, float* s2, cudaStream_t stream);
+constexpr int ZERO_WORDS = 8;  // scheduler words of a workspace: {claimed, finished} of up to four GEMM launches
 int launch_rms_quant(const void* x, int64_t x_row_stride, const void* rms_delta, float eps, const int32_t* row_map,
-                     int m, int k, void* xq, float* sx, void* xn, cudaStream_t stream);
+                     int m, int k, void* xq, float* sx, void* xn, cudaStream_t stream, float* zero_amax = nullptr,
+                     int32_t* zero_words = nullptr);  // fp32 [m] / ZERO_WORDS words cleared for kernels behind this one
 // rows [m, k] contiguous (row pitch k) with their absmax known: codes and scales in one streaming pass
 int launch_quant_stream(const void* x, const float* row_amax, int m, int k, void* xq, float* sx, cudaStream_t stream);
 int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const float* scaling, int num_adapters,
-                       int rank, const int32_t* tiles, const int32_t* num_tiles, int max_tiles, void* z_parts,
-                       int32_t* status, cudaStream_t stream, int row_lo = 0, int row_hi = -1,
-                       void* const* extra_dests = nullptr, int extra_count = 0, int list_row0 = -1);  // extra copies of the rows written
+                       int rank, const TileSource& src, int max_tiles, void* z_parts, int32_t* status,
+                       cudaStream_t stream, int row_lo = 0, int row_hi = -1, void* const* extra_dests = nullptr,
+                       int extra_count = 0, int list_row0 = -1);  // extra copies of the rows written
 // Tile width and K split the GEMM launcher chooses for a shape (deterministic per device).
 struct GemmPlan {
   int bn_eff;
@@ -84,7 +89,8 @@ struct GemmPlan {
 };
 GemmPlan plan_gemm(int m, int n, int k, int epilogue, int max_slabs);
 constexpr int MAX_SPLIT_K_SLABS = 16;
-int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic = false);
+// `src`: the M tiles, where they are not the two-adapter list in `a` (nullptr: a.tiles / a.num_tiles).
+int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic = false, const TileSource* src = nullptr);
 // `programmatic`: launch with programmatic stream serialization (small-batch chain of short kernels)
 // Adapter ids outside [0, num_adapters) are clamped and STATUS_BAD_ADAPTER_ID is recorded in `status`.
 int launch_rms_quant_rows(const void* x, int64_t x_row_stride, const void* rms_delta, float eps, const int32_t* ids,

@@ -154,6 +154,209 @@ int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int
 }
 
 // ----------------------------------------------------------------------------
+// Routing of the operators: the same stable order as dense tiles (tiles.cuh).
+// One CTA, every phase parallel (the serial scatter of route_kernel, one warp and
+// a dependent round of shared-memory updates per 32 rows, took 131 us at 16384
+// rows).  Up to 24 warps own one contiguous run of rows each and a histogram row
+// of their own; a scan over (adapter, warp) gives every warp its first position
+// per adapter, and it then places its rows in order with match_any.  Tiles need
+// no packing: tile i is rows 128 i ..., its segments are the non-empty adapters
+// whose runs meet it, and segment number = tile + rank of the adapter among the
+// non-empty ones is strictly increasing along the sorted rows, so the other warps
+// write the tile list at the same time without any scan over tiles.
+// Batches of at most 128 rows keep token order: one tile, masks from match_any.
+// ----------------------------------------------------------------------------
+constexpr int ROUTE_SORT_WARPS = 24;
+constexpr int ROUTE_HIST_WORDS = 8192;
+
+__global__ void __launch_bounds__(ROUTE_THREADS)
+route_dense_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int hist_warps, int32_t* __restrict__ perm,
+                   int4* __restrict__ tiles, int4* __restrict__ seg_mask, int32_t* __restrict__ seg_adapter,
+                   int32_t* status, int32_t* __restrict__ zero_words, int zero_count) {
+  extern __shared__ int route_smem[];
+  int* hist = route_smem;                        // [hist_warps][num_adapters]: counts, then first positions
+  int* nz_start = hist + hist_warps * num_adapters;  // [num_adapters + 1] first sorted row of the non-empty adapters
+  int* nz_adapter = nz_start + num_adapters + 1; // [num_adapters]
+  int* total = nz_adapter + num_adapters;        // [num_adapters] rows per adapter, then the adapter's first sorted row
+  __shared__ int num_nonempty;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < hist_warps * num_adapters; i += ROUTE_THREADS) hist[i] = 0;
+  pdl_wait();
+  pdl_trigger();
+  if (zero_words != nullptr && tid < zero_count) zero_words[tid] = 0;
+  __syncthreads();
+
+  const int span = ((m + hist_warps - 1) / hist_warps + 31) / 32 * 32;
+  const int lo = min(m, warp * span), hi = warp < hist_warps ? min(m, lo + span) : lo;
+  int* mine = hist + warp * num_adapters;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  bool bad = false;
+  for (int base = lo; base < hi; base += 128) {
+    int a[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = base + 32 * j + lane;
+      a[j] = i < hi ? __ldg(ids + i) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (base + 32 * j >= hi) break;
+      const bool active = base + 32 * j + lane < hi;
+      if (active && (a[j] < 0 || a[j] >= num_adapters)) {
+        bad = true;
+        a[j] = min(max(a[j], 0), num_adapters - 1);
+      }
+      const unsigned peers = __match_any_sync(0xffffffffu, a[j]);
+      if (active && (peers & lt_mask) == 0) mine[a[j]] += __popc(peers);
+      __syncwarp();
+    }
+  }
+  if (bad) atomicCAS(status, 0, STATUS_BAD_ADAPTER_ID);
+  __syncthreads();
+  for (int a = tid; a < num_adapters; a += ROUTE_THREADS) {
+    int sum = 0;
+    for (int w = 0; w < hist_warps; ++w) {
+      const int c = hist[w * num_adapters + a];
+      hist[w * num_adapters + a] = sum;
+      sum += c;
+    }
+    total[a] = sum;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int rows = 0, nonempty = 0;
+    for (int base = 0; base < num_adapters; base += 32) {
+      const int a = base + lane;
+      const int c = a < num_adapters ? total[a] : 0;
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const unsigned have = __ballot_sync(0xffffffffu, c > 0);
+      if (c > 0) {
+        const int r = nonempty + __popc(have & lt_mask);
+        nz_start[r] = rows + incl - c;
+        nz_adapter[r] = a;
+      }
+      if (a < num_adapters) total[a] = rows + incl - c;
+      rows += __shfl_sync(0xffffffffu, incl, 31);
+      nonempty += __popc(have);
+    }
+    if (lane == 0) {
+      nz_start[nonempty] = m;
+      num_nonempty = nonempty;
+    }
+  }
+  __syncthreads();
+  const int nonempty = num_nonempty;
+
+  if (m <= SKYRL_TILE_ROWS) {  // token order: one tile, every adapter's rows wherever they are
+    for (int i = tid; i < m; i += ROUTE_THREADS) perm[i] = i;
+    int* words = reinterpret_cast<int*>(seg_mask);
+    for (int r = tid; r < nonempty; r += ROUTE_THREADS) {
+      seg_adapter[r] = nz_adapter[r];
+      seg_mask[r] = make_int4(0, 0, 0, 0);
+    }
+    if (tid == 0) tiles[0] = make_int4(0, m, nonempty, ~0);
+    __syncthreads();
+    if (warp < 4 && warp * 32 < m) {
+      const int i = warp * 32 + lane;
+      int a = i < m ? __ldg(ids + i) : -1;
+      if (i < m) a = min(max(a, 0), num_adapters - 1);
+      const unsigned peers = __match_any_sync(0xffffffffu, a);
+      if (i < m && (peers & lt_mask) == 0) {
+        int r = 0, above = nonempty - 1;  // rank of adapter a among the non-empty ones
+        while (r < above) {
+          const int mid = (r + above) >> 1;
+          if (nz_adapter[mid] < a) r = mid + 1; else above = mid;
+        }
+        words[4 * r + warp] = static_cast<int>(peers);
+      }
+    }
+    return;
+  }
+
+  for (int base = lo; base < hi; base += 128) {
+    int a[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = base + 32 * j + lane;
+      a[j] = i < hi ? min(max(__ldg(ids + i), 0), num_adapters - 1) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (base + 32 * j >= hi) break;
+      const int i = base + 32 * j + lane;
+      const unsigned peers = __match_any_sync(0xffffffffu, a[j]);
+      const int rank = __popc(peers & lt_mask);
+      const int at = i < hi ? mine[a[j]] : 0;
+      __syncwarp();
+      if (i < hi) {
+        perm[total[a[j]] + at + rank] = i;
+        if (rank == 0) mine[a[j]] = at + __popc(peers);
+      }
+      __syncwarp();
+    }
+  }
+  // the tile list: the warps without rows write it while the others scatter
+  const int first = hist_warps < ROUTE_THREADS / 32 ? hist_warps * 32 : 0;
+  const int count = (m + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS;
+  if (tid >= first) {
+    for (int t = tid - first; t < count; t += ROUTE_THREADS - first) {
+      const int r0 = t * SKYRL_TILE_ROWS, r1 = min(m, r0 + SKYRL_TILE_ROWS);
+      int r = 0, above = nonempty - 1;  // last non-empty adapter that starts at or before r0
+      while (r < above) {
+        const int mid = (r + above + 1) >> 1;
+        if (nz_start[mid] <= r0) r = mid; else above = mid - 1;
+      }
+      const int seg0 = t + r;
+      int segs = 0;
+      for (; r + segs < nonempty && nz_start[r + segs] < r1; ++segs) {
+        const int b = max(nz_start[r + segs], r0) - r0, e = min(nz_start[r + segs + 1], r1) - r0;
+        int w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int nb = min(max(b - 32 * q, 0), 32), ne = min(max(e - 32 * q, 0), 32);
+          const unsigned below_b = nb == 32 ? 0xffffffffu : (1u << nb) - 1u;
+          const unsigned below_e = ne == 32 ? 0xffffffffu : (1u << ne) - 1u;
+          w[q] = static_cast<int>(below_e & ~below_b);
+        }
+        seg_mask[seg0 + segs] = make_int4(w[0], w[1], w[2], w[3]);
+        seg_adapter[seg0 + segs] = nz_adapter[r + segs];
+      }
+      tiles[t] = make_int4(r0, r1 - r0, segs, ~seg0);
+    }
+  }
+}
+
+int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* seg_mask,
+                       int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count) {
+  if (ids == nullptr || m <= 0 || perm == nullptr || tiles == nullptr || seg_mask == nullptr || seg_adapter == nullptr ||
+      status == nullptr || !aligned16(tiles) || !aligned16(seg_mask))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: null or misaligned buffer");
+  if (num_adapters <= 0 || num_adapters > ROUTE_MAX_ADAPTERS)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: num_adapters must be in [1, %d], got %d", ROUTE_MAX_ADAPTERS,
+                num_adapters);
+  if (zero_count < 0 || zero_count > ROUTE_THREADS)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: at most %d words can be cleared", ROUTE_THREADS);
+  int warps = ROUTE_HIST_WORDS / num_adapters;
+  if (warps < 1) warps = 1;
+  if (warps > ROUTE_SORT_WARPS) warps = ROUTE_SORT_WARPS;
+  const int smem = (warps * num_adapters + 3 * num_adapters + 1) * static_cast<int>(sizeof(int));
+  static bool attr_set[MAX_DEVICES] = {};
+  cudaError_t e = ensure_dynamic_smem(route_dense_kernel, (ROUTE_HIST_WORDS + 3 * ROUTE_MAX_ADAPTERS + 1) * 4, attr_set);
+  if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "route attribute: %s", cudaGetErrorString(e));
+  e = launch_kernel(route_dense_kernel, dim3(1), dim3(ROUTE_THREADS), smem, stream, true, ids, m, num_adapters, warps, perm,
+                    reinterpret_cast<int4*>(tiles), reinterpret_cast<int4*>(seg_mask), seg_adapter, status, zero_words,
+                    zero_count);
+  if (e == cudaSuccess) e = cudaPeekAtLastError();
+  if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "route launch: %s", cudaGetErrorString(e));
+  return SKYRL_OK;
+}
+
+// ----------------------------------------------------------------------------
 // RMSNorm + per-token int8 quantisation.  One CTA per output row; the row is
 // staged in shared memory so HBM is read once.  Arithmetic follows the
 // reference exactly: fp32 mean of squares, (x * rinv) * (1 + delta) rounded to
@@ -163,16 +366,21 @@ int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int
 __global__ void __launch_bounds__(QUANT_THREADS)
 rms_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const __nv_bfloat16* __restrict__ delta,
                  float eps, const int32_t* __restrict__ row_map, int k, int8_t* __restrict__ xq,
-                 float* __restrict__ sx, __nv_bfloat16* __restrict__ xn) {
+                 float* __restrict__ sx, __nv_bfloat16* __restrict__ xn, float* __restrict__ zero_amax,
+                 int32_t* __restrict__ zero_words) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* row = reinterpret_cast<uint4*>(smem_raw);  // k / 8 vectors of 8 bf16
   __shared__ float red[QUANT_THREADS / 32];
 
+  pdl_wait();
+  pdl_trigger();
   const int out_row = blockIdx.x;
   const int64_t src_row = row_map != nullptr ? row_map[out_row] : out_row;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * x_row_stride);
   const int nvec = k >> 3;
   const bool norm = delta != nullptr;
+  if (threadIdx.x == 0 && zero_amax != nullptr) zero_amax[out_row] = 0.f;
+  if (zero_words != nullptr && out_row == 0 && threadIdx.x < ZERO_WORDS) zero_words[threadIdx.x] = 0;
 
   float ss = 0.f, amax = 0.f;
   for (int v = threadIdx.x; v < nvec; v += QUANT_THREADS) {
@@ -199,7 +407,8 @@ rms_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, cons
 }
 
 int launch_rms_quant(const void* x, int64_t x_row_stride, const void* rms_delta, float eps, const int32_t* row_map,
-                     int m, int k, void* xq, float* sx, void* xn, cudaStream_t stream) {
+                     int m, int k, void* xq, float* sx, void* xn, cudaStream_t stream, float* zero_amax,
+                     int32_t* zero_words) {
   if (x == nullptr || xq == nullptr || sx == nullptr || m <= 0 || k <= 0)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "rms_quant: null buffer or non-positive shape");
   if (k % 16 != 0) return fail(SKYRL_ERR_INVALID_ARGUMENT, "rms_quant: K must be a multiple of 16, got %d", k);
@@ -214,10 +423,10 @@ int launch_rms_quant(const void* x, int64_t x_row_stride, const void* rms_delta,
   static bool attr_set[MAX_DEVICES] = {};
   cudaError_t e = ensure_dynamic_smem(rms_quant_kernel, 200 * 1024, attr_set);
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "rms_quant attribute: %s", cudaGetErrorString(e));
-  rms_quant_kernel<<<m, QUANT_THREADS, smem, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), x_row_stride, static_cast<const __nv_bfloat16*>(rms_delta), eps, row_map,
-      k, static_cast<int8_t*>(xq), sx, static_cast<__nv_bfloat16*>(xn));
-  e = cudaPeekAtLastError();
+  e = launch_kernel(rms_quant_kernel, dim3(m), dim3(QUANT_THREADS), smem, stream, true,
+                    static_cast<const __nv_bfloat16*>(x), x_row_stride, static_cast<const __nv_bfloat16*>(rms_delta), eps,
+                    row_map, k, static_cast<int8_t*>(xq), sx, static_cast<__nv_bfloat16*>(xn), zero_amax, zero_words);
+  if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "rms_quant launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;
 }
@@ -229,6 +438,8 @@ int launch_rms_quant(const void* x, int64_t x_row_stride, const void* rms_delta,
 __global__ void __launch_bounds__(256)
 quant_stream_kernel(const uint4* __restrict__ x, const float* __restrict__ row_amax, int nvec, int64_t total_vecs,
                     uint2* __restrict__ xq, float* __restrict__ sx) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t v0 = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * 2;
   if (v0 >= total_vecs) return;
   const bool two = v0 + 1 < total_vecs;
@@ -264,9 +475,9 @@ int launch_quant_stream(const void* x, const float* row_amax, int m, int k, void
   const int64_t total = static_cast<int64_t>(m) * nvec;
   const int64_t ctas = (total + 511) / 512;
   if (ctas > 0x7fffffffll) return fail(SKYRL_ERR_UNSUPPORTED, "quant_stream: too many rows");
-  quant_stream_kernel<<<static_cast<unsigned>(ctas), 256, 0, stream>>>(static_cast<const uint4*>(x), row_amax, nvec, total,
-                                                                      static_cast<uint2*>(xq), sx);
-  cudaError_t e = cudaPeekAtLastError();
+  cudaError_t e = launch_kernel(quant_stream_kernel, dim3(static_cast<unsigned>(ctas)), dim3(256), 0, stream, true,
+                                static_cast<const uint4*>(x), row_amax, nvec, total, static_cast<uint2*>(xq), sx);
+  if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "quant_stream launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;
 }

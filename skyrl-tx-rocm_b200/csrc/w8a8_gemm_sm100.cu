@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
+#include "tiles.cuh"
 
 namespace skyrl {
 
@@ -48,7 +49,6 @@ constexpr int EPI_STAGE_BYTES = 32 * 128;     // the fp32 form holds 32 rows x 1
 // the single-tile kernel carves eight such tiles out of the top of the stage area
 constexpr int SINGLE_STAGE_AREA = STAGE_AREA_BYTES - 8 * EPI_STAGE_BYTES;
 constexpr int MAX_STAGES = 12;
-constexpr int Z_PLANE_BYTES = BM * LORA_ROW_BYTES;  // one bf16 plane of z for a tile: 128 rows x 128 bytes
 constexpr int LORA_INJECT_AFTER = 8;  // K blocks of the next tile issued before the previous tile's LoRA operands
 
 template <int BN>
@@ -59,15 +59,37 @@ struct GemmCfg {
   static constexpr int TMEM_COLS = 2 * BN;
 };
 
+// The LoRA operands of one M tile x N tile travel through slots of the TMA pipeline, at the width of the rank
+// (w = 32, 64 or 128 bytes per row for ranks up to 16, 32, 64, with the swizzle of that width).  They come in rounds:
+// the three z planes of the tile's rows, then the LoRA-B tiles of its segments (adapters), several to a slot; a round
+// never takes more slots than the pipeline has, so the slots of the planes can stay until its last MMA.
+struct LoraGeom {
+  int w;             // bytes per row of z and of a LoRA-B tile
+  int z_plane;       // bytes of one plane: 128 rows
+  int z_per_slot;    // planes per slot
+  int b_tile;        // bytes of one adapter's LoRA-B tile
+  int b_per_slot;    // adapters per slot
+  int b_per_round;   // adapters per round
+};
+static LoraGeom lora_geom(int rank, int b_rows, int stage_bytes, int stages) {
+  LoraGeom g;
+  g.w = rank <= 16 ? 32 : (rank <= 32 ? 64 : 128);
+  g.z_plane = BM * g.w;
+  g.z_per_slot = stage_bytes / g.z_plane < 3 ? stage_bytes / g.z_plane : 3;
+  g.b_tile = b_rows * g.w;
+  g.b_per_slot = stage_bytes / g.b_tile;
+  g.b_per_round = (stages - (3 + g.z_per_slot - 1) / g.z_per_slot) * g.b_per_slot;
+  return g;
+}
+
 struct GemmParams {
   CUtensorMap tm_xq;   // int8 [M, K], box 128 x 128
   CUtensorMap tm_w;    // int8 [K / 128, N, 128], box 128 x bn_eff x 1
-  CUtensorMap tm_z;    // bf16 [M, 6, 64], box 64 x 1 x 128 (one part of one adapter slot of one tile's rows)
-  CUtensorMap tm_b;    // bf16 [A, N, 64], box 64 x BN x 1
+  CUtensorMap tm_z;    // bf16 [M, 6, 64], box w / 2 x 1 x 128 (one part of one adapter slot of one tile's rows)
+  CUtensorMap tm_b;    // bf16 [A, N, rank slots], box w / 2 x BN x 1
   const float* sx;
   const float* sw;
-  const int4* tiles;
-  const int32_t* num_tiles;
+  TileSource src;      // the M tiles
   const int32_t* out_row_map;
   const __nv_bfloat16* residual;
   void* out;
@@ -76,6 +98,7 @@ struct GemmParams {
   int32_t* status;
   int m, n, k;
   int rank_blocks;  // ceil(rank / 16) MMAs per z plane
+  LoraGeom lora;    // how the LoRA operands of a tile travel through the pipeline slots
   int band;         // M tiles per raster band
   int bn_eff;       // columns per N tile actually used (multiple of 16, <= BN): MMA N, TMA box rows
   int num_stages;   // pipeline depth and byte pitch of one stage (A tile + bn_eff weight rows)
@@ -158,7 +181,8 @@ __device__ __forceinline__ int sched_claim(TileRing* ring, uint32_t it, int* cou
   const uint32_t slot = it & (SCHED_SLOTS - 1);
   ok = mbar_wait(&ring->empty[slot], ((it / SCHED_SLOTS) & 1u) ^ 1u, abort_flag, status, STATUS_TIMEOUT_PRODUCER);
   if (!ok) return -1;
-  int t = atomicAdd(counter, 1);
+  // without a counter: fixed stride (a launch of one wave, or one that shares the GPU with nothing)
+  int t = counter != nullptr ? atomicAdd(counter, 1) : static_cast<int>(blockIdx.x + it * gridDim.x);
   if (t >= total) t = -1;
   ring->tile[slot] = t;
   mbar_arrive(&ring->full[slot]);  // release: the tile number is visible to whoever observes the phase
@@ -175,7 +199,7 @@ __device__ __forceinline__ void sched_release(TileRing* ring, uint32_t it) {
 }
 // The last CTA of a launch puts the claim counter back to zero for the slot's next user.
 __device__ __forceinline__ void sched_finish(int* sched) {
-  if (atomicAdd(sched + 1, 1) == static_cast<int>(gridDim.x) - 1) {
+  if (sched != nullptr && atomicAdd(sched + 1, 1) == static_cast<int>(gridDim.x) - 1) {
     sched[0] = 0;
     sched[1] = 0;
     __threadfence();
@@ -189,9 +213,9 @@ struct IssuerProfile {
 };
 __device__ __forceinline__ bool timed_wait(bool on, long long& acc, uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                            int* status, int code) {
-  if (!on) return mbar_wait(bar, parity, abort_flag, status, code);
+  if (!on) return mbar_wait_warp(bar, parity, abort_flag, status, code);
   const long long t0 = clock64();
-  const bool ok = mbar_wait(bar, parity, abort_flag, status, code);
+  const bool ok = mbar_wait_warp(bar, parity, abort_flag, status, code);
   acc += clock64() - t0;
   return ok;
 }
@@ -221,6 +245,104 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int tm, int tn, int band)
 
 __device__ __forceinline__ float silu_f32(float t) { return __fdiv_rn(t, 1.0f + expf(-t)); }
 
+
+// ---- LoRA operands of one tile through the TMA pipeline (one CTA per tile; see LoraGeom) ----------------
+struct Pipe {
+  unsigned char* smem;
+  uint64_t* full;
+  uint64_t* empty;
+  int stages, bytes, stage;
+  uint32_t phase;
+  __device__ __forceinline__ void next() {
+    if (++stage == stages) {
+      stage = 0;
+      phase ^= 1u;
+    }
+  }
+  __device__ __forceinline__ unsigned char* at() const { return smem + stage * bytes; }
+};
+
+__device__ __forceinline__ bool lora_load(const GemmParams& p, Pipe& q, const int4& tile, int n0, volatile int* abort_flag) {
+  const LoraGeom& g = p.lora;
+  const int nseg = tile_segments(tile);
+  const bool dense = tile_is_dense(tile);
+  for (int j = 0; j < nseg;) {
+    const int slot = segment_slot(tile, j);
+    for (int pl = 0; pl < 3; pl += g.z_per_slot) {  // lo, mid, hi: the smallest plane is added first
+      if (!mbar_wait(&q.empty[q.stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
+      const int cnt = min(g.z_per_slot, 3 - pl);
+      mbar_expect_tx(&q.full[q.stage], cnt * g.z_plane);
+      for (int i = 0; i < cnt; ++i)
+        tma_load_3d(q.at() + i * g.z_plane, &p.tm_z, 0, 3 * slot + 2 - (pl + i), tile.x, &q.full[q.stage]);
+      q.next();
+    }
+    // a list of two slots keeps the second adapter's z elsewhere: every adapter is a round of its own
+    for (int left = dense ? min(nseg - j, g.b_per_round) : 1; left > 0;) {
+      const int cnt = min(g.b_per_slot, left);
+      if (!mbar_wait(&q.empty[q.stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
+      mbar_expect_tx(&q.full[q.stage], cnt * g.b_tile);
+      for (int i = 0; i < cnt; ++i)
+        tma_load_3d(q.at() + i * g.b_tile, &p.tm_b, 0, n0, segment_adapter(p.src, tile, j + i), &q.full[q.stage]);
+      q.next();
+      j += cnt;
+      left -= cnt;
+    }
+  }
+  return true;
+}
+
+// rank-r bf16 MMAs of one tile, accumulated onto the accumulator `d` the epilogue rewrote as fp32 (`ready` waits for
+// that rewrite, once the first operands are there); every segment touches the lanes of its own rows only.  Called by a
+// whole warp, which elects a thread for the instructions.
+template <typename Ready>
+__device__ __forceinline__ bool lora_issue(const GemmParams& p, Pipe& q, const int4& tile, uint32_t d, uint32_t idesc,
+                                           volatile int* abort_flag, Ready ready) {
+  const LoraGeom& g = p.lora;
+  const int nseg = tile_segments(tile);
+  const bool dense = tile_is_dense(tile);
+  for (int j = 0; j < nseg;) {
+    const int zstage0 = q.stage;
+    const int zslots = (3 + g.z_per_slot - 1) / g.z_per_slot;
+    for (int i = 0; i < zslots; ++i) {
+      if (!mbar_wait_warp(&q.full[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
+      q.next();
+    }
+    const bool first = j == 0;
+    bool started = false;
+    for (int left = dense ? min(nseg - j, g.b_per_round) : 1; left > 0;) {
+      const int cnt = min(g.b_per_slot, left);
+      if (!mbar_wait_warp(&q.full[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
+      if (first && !started && !ready()) return false;
+      started = true;
+      tc_fence_after_sync();
+      const uint32_t base = smem_u32(q.at());
+      for (int i = 0; i < cnt; ++i) {
+        const int4 mk = segment_mask(p.src, tile, j + i);
+        const int4 off = make_int4(~mk.x, ~mk.y, ~mk.z, ~mk.w);
+        const uint64_t bd = make_desc_width(base + i * g.b_tile, g.w);
+        if (elect_one()) {
+          for (int plane = 0; plane < 3; ++plane) {
+            int zs = zstage0 + plane / g.z_per_slot;
+            if (zs >= q.stages) zs -= q.stages;
+            const uint64_t zd = make_desc_width(smem_u32(q.smem + zs * q.bytes) + (plane % g.z_per_slot) * g.z_plane, g.w);
+            for (int kk = 0; kk < p.rank_blocks; ++kk) mma_bf16_lanes(d, zd + 2 * kk, bd + 2 * kk, idesc, 1u, off);
+          }
+        }
+        __syncwarp();
+      }
+      if (elect_one()) mma_commit(&q.empty[q.stage]);
+      __syncwarp();
+      q.next();
+      j += cnt;
+      left -= cnt;
+    }
+    if (elect_one()) {
+      for (int i = 0; i < zslots; ++i) mma_commit(&q.empty[(zstage0 + i) % q.stages]);
+    }
+    __syncwarp();
+  }
+  return true;
+}
 
 // ---- epilogue building blocks (one 32-column chunk of one TMEM lane quadrant) ------------------------
 // pass 1 of the LoRA path: int32 accumulator -> (f32(acc) * sx[m]) * sw[n], written back in place
@@ -564,7 +686,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  const int tm = *p.num_tiles;
+  const int tm = tile_count(p.src);
   const int bn_eff = p.bn_eff;
   const int tn = (p.n + bn_eff - 1) / bn_eff;
   const int ksplits = p.k_splits;
@@ -580,55 +702,27 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
   if (warp == 4) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
+      Pipe q = {smem, full_bar, empty_bar, nstages, stage_bytes, 0, 0u};
       bool ok = true, have_prev = false;
       bool dep_ready = false;  // the previous kernel of the stream has finished (programmatic launch)
       int held = 0, held_stage[MAX_STAGES], held_kb[MAX_STAGES];
-      int prev_row0 = 0, prev_n0 = 0, prev_adapter = 0, prev_second = 0;
-      // LoRA operands of one adapter slot of one tile: pipeline slot 1 = z parts lo and mid, pipeline
-      // slot 2 = z part hi and the adapter's B tile
-      auto lora_slots_of = [&](int row0, int n0, int adapter, int zslot) -> bool {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-        unsigned char* sa = smem + stage * stage_bytes;
-        mbar_expect_tx(&full_bar[stage], 2 * Z_PLANE_BYTES);
-        tma_load_3d(sa, &p.tm_z, 0, 3 * zslot + 2, row0, &full_bar[stage]);
-        tma_load_3d(sa + Z_PLANE_BYTES, &p.tm_z, 0, 3 * zslot + 1, row0, &full_bar[stage]);
-        if (++stage == nstages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-        sa = smem + stage * stage_bytes;
-        mbar_expect_tx(&full_bar[stage], Z_PLANE_BYTES + bn_eff * LORA_ROW_BYTES);
-        tma_load_3d(sa, &p.tm_z, 0, 3 * zslot, row0, &full_bar[stage]);
-        tma_load_3d(sa + Z_PLANE_BYTES, &p.tm_b, 0, n0, adapter, &full_bar[stage]);
-        if (++stage == nstages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        return true;
-      };
-      // a tile of two adapters (second != 0) brings both slots: z(slot 0) with the first adapter's B,
-      // z(slot 1) with the second's; each row is zero in the slot that is not its own
-      auto lora_slots = [&](int row0, int n0, int adapter, int second) -> bool {
-        if (!lora_slots_of(row0, n0, adapter, 0)) return false;
-        return second == 0 || lora_slots_of(row0, n0, (second & 0xffff) - 1, 1);
-      };
+      int4 prev_tile = make_int4(0, 0, 0, 0);
+      int prev_n0 = 0;
       for (uint32_t it = 0; ok; ++it) {
         const int t = sched_claim(ring, it, p.sched, total, abort_flag, p.status, ok);
         if (t < 0) break;
         const TileCoord c = tile_coord(t / ksplits, tm, tn, band);
-        const int4 tile = __ldg(p.tiles + c.m_idx);
+        const int4 tile = tile_at(p.src, c.m_idx);
         const int n0 = c.n_idx * bn_eff;
         const int kb0 = (t % ksplits) * p.kb_per_split;
         const int kb1 = min(kblocks, kb0 + p.kb_per_split);
         const int inject_at = min(LORA_INJECT_AFTER, kb1 - kb0);
         int issued = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER);
+          const int stage = q.stage;
+          ok = mbar_wait(&empty_bar[stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER);
           if (!ok) break;
-          unsigned char* sa = smem + stage * stage_bytes;
+          unsigned char* sa = q.at();
           mbar_expect_tx(&full_bar[stage], stage_tx);
           if (!dep_ready) {
             // The weights never depend on the kernel before this one, the activations do: until the
@@ -650,76 +744,51 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
             tma_load_2d(sa, &p.tm_xq, kb * BK, tile.x, &full_bar[stage]);
             tma_load_3d(sa + a_bytes, &p.tm_w, 0, n0, kb, &full_bar[stage]);
           }
-          if (++stage == nstages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          q.next();
           if (HAS_LORA && have_prev && ++issued == inject_at) {
-            ok = lora_slots(prev_row0, prev_n0, prev_adapter, prev_second);
+            ok = lora_load(p, q, prev_tile, prev_n0, abort_flag);
             if (!ok) break;
           }
         }
-        prev_row0 = tile.x;
+        prev_tile = tile;
         prev_n0 = n0;
-        prev_adapter = tile.z;
-        prev_second = tile.w;
         have_prev = true;
       }
-      if (HAS_LORA && have_prev && ok) lora_slots(prev_row0, prev_n0, prev_adapter, prev_second);
+      if (HAS_LORA && have_prev && ok) lora_load(p, q, prev_tile, prev_n0, abort_flag);
       if (ok && p.prefetch_bytes > 0) prefetch_share_to_l2(p);
     }
   } else if (warp == 5) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    // The whole warp walks the loop, one elected thread issues: operands that the compiler can keep in uniform
+    // registers make the issue of an MMA a third as long.
+    {
       const uint32_t idesc = make_idesc(IDESC_D_S32, IDESC_S8, IDESC_S8, BM, bn_eff);
       const uint32_t idesc_lora = make_idesc(IDESC_D_F32, IDESC_BF16, IDESC_BF16, BM, bn_eff);
-      int stage = 0;
-      uint32_t phase = 0, it = 0, lora_rounds = 0;
+      Pipe q = {smem, full_bar, empty_bar, nstages, stage_bytes, 0, 0u};
+      const uint32_t smem_base = smem_u32(smem);
+      uint32_t it = 0, lora_rounds = 0;
       bool ok = true, have_prev = false;
       uint32_t prev_s = 0;
-      int prev_second = 0;
+      int4 prev_tile = make_int4(0, 0, 0, 0);
       const bool prof = p.profile != 0 && blockIdx.x == 0;
       IssuerProfile pr;
       const long long prof_t0 = clock64();
-      // rank-r bf16 MMAs of one adapter slot of one tile, accumulated onto the accumulator the epilogue
-      // rewrote as fp32; `first` waits for that rewrite, `last` hands the accumulator back to the epilogue
-      auto lora_mma_of = [&](uint32_t acc_stage, bool first, bool last) -> bool {
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-        const int st1 = stage;
-        if (++stage == nstages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-        const int st2 = stage;
-        if (++stage == nstages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        if (first && !timed_wait(prof, pr.rewrite, conv_done, lora_rounds & 1u, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-        tc_fence_after_sync();
-        const uint32_t e1 = smem_u32(smem + st1 * stage_bytes), e2 = smem_u32(smem + st2 * stage_bytes);
-        const uint64_t bd = make_desc_sw128(e2 + Z_PLANE_BYTES);
-        const uint64_t zd[3] = {make_desc_sw128(e1), make_desc_sw128(e1 + Z_PLANE_BYTES), make_desc_sw128(e2)};
-        const uint32_t d = tmem_base + acc_stage * BN;
-        // smallest plane first, so the low-order terms are not absorbed early
-        for (int plane = 0; plane < 3; ++plane)
-          for (int kk = 0; kk < p.rank_blocks; ++kk) mma_bf16(d, zd[plane] + 2 * kk, bd + 2 * kk, idesc_lora, 1u);
-        mma_commit(&empty_bar[st1]);
-        mma_commit(&empty_bar[st2]);
-        if (last) {
-          mma_commit(lora_done);
-          ++lora_rounds;
-        }
+      // waits for the epilogue's rewrite of the accumulator, adds the LoRA term, hands the accumulator back
+      auto lora_mma = [&](uint32_t acc_stage, const int4& tile) -> bool {
+        const bool done = lora_issue(p, q, tile, tmem_base + acc_stage * BN, idesc_lora, abort_flag, [&]() {
+          return timed_wait(prof, pr.rewrite, conv_done, lora_rounds & 1u, abort_flag, p.status, STATUS_TIMEOUT_LORA);
+        });
+        if (!done) return false;
+        if (elect_one()) mma_commit(lora_done);
+        __syncwarp();
+        ++lora_rounds;
         return true;
-      };
-      auto lora_mma = [&](uint32_t acc_stage, int second) -> bool {
-        if (!lora_mma_of(acc_stage, true, second == 0)) return false;
-        return second == 0 || lora_mma_of(acc_stage, false, true);
       };
       for (; ok; ++it) {
         const int t = sched_read(ring, it, abort_flag, p.status, STATUS_TIMEOUT_MMA, ok);
-        if (ok) sched_release(ring, it);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane == 0) sched_release(ring, it);  // every lane has read the slot (warp-wide vote above)
         if (t < 0) break;
         const uint32_t s = it & 1u, aphase = (it >> 1) & 1u;
         ok = timed_wait(prof, pr.accumulator, &tmem_empty[s], aphase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_MMA);
@@ -729,36 +798,36 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
         const int kb0 = (t % ksplits) * p.kb_per_split;
         const int kb1 = min(kblocks, kb0 + p.kb_per_split);
         const int inject_at = min(LORA_INJECT_AFTER, kb1 - kb0);
-        const int second = HAS_LORA ? __ldg(p.tiles + tile_coord(t / ksplits, tm, tn, band).m_idx).w : 0;
+        const int4 tile = HAS_LORA ? tile_at(p.src, tile_coord(t / ksplits, tm, tn, band).m_idx) : make_int4(0, 0, 0, 0);
         int issued = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = timed_wait(prof, pr.operands, &full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_MMA);
+          ok = timed_wait(prof, pr.operands, &full_bar[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_MMA);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * stage_bytes);
-          const uint64_t adesc = make_desc_sw128(sa);
-          const uint64_t bdesc = make_desc_sw128(sa + a_bytes);
+          const uint32_t sa = smem_base + q.stage * stage_bytes;
+          if (elect_one()) {
+            const uint64_t adesc = make_desc_sw128(sa);
+            const uint64_t bdesc = make_desc_sw128(sa + a_bytes);
 #pragma unroll
-          for (int j = 0; j < BK / UMMA_K_I8; ++j) {
-            mma_i8(d, adesc + 2 * j, bdesc + 2 * j, idesc, (kb != kb0 || j != 0) ? 1u : 0u);
+            for (int j = 0; j < BK / UMMA_K_I8; ++j)
+              mma_i8(d, adesc + 2 * j, bdesc + 2 * j, idesc, (kb != kb0 || j != 0) ? 1u : 0u);
+            mma_commit(&empty_bar[q.stage]);
           }
-          mma_commit(&empty_bar[stage]);
-          if (++stage == nstages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          __syncwarp();
+          q.next();
           if (HAS_LORA && have_prev && ++issued == inject_at) {
-            ok = lora_mma(prev_s, prev_second);
+            ok = lora_mma(prev_s, prev_tile);
             if (!ok) break;
           }
         }
-        if (ok) mma_commit(&tmem_full[s]);
+        if (ok && elect_one()) mma_commit(&tmem_full[s]);
+        __syncwarp();
         prev_s = s;
-        prev_second = second;
+        prev_tile = tile;
         have_prev = true;
       }
-      if (HAS_LORA && have_prev && ok) lora_mma(prev_s, prev_second);
-      if (prof) store_profile(pr, p.status, clock64() - prof_t0);
+      if (HAS_LORA && have_prev && ok) lora_mma(prev_s, prev_tile);
+      if (prof && lane == 0) store_profile(pr, p.status, clock64() - prof_t0);
     }
   } else {
     // ------------------------------ epilogue warps 0-3, 6-9 --------------------
@@ -774,7 +843,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
     const int ew = warp < 4 ? warp : warp - 2;  // 0 ... 7 among the epilogue warps
     uint32_t it = 0, lora_it = 0;
     bool ok = true;
-    if (ROWS) pdl_wait();  // scales, z and the residual may come from the kernel just before this one
+    pdl_wait();  // scales, z and the residual may come from the kernel just before this one
     for (; ok; ++it) {
       const int t = sched_read(ring, it, abort_flag, p.status, STATUS_TIMEOUT_EPILOGUE, ok);
       ok = __all_sync(0xffffffffu, ok);
@@ -782,14 +851,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
       if (lane == 0) sched_release(ring, it);  // every lane has read the slot (warp-wide vote above)
       if (t < 0) break;
       const TileCoord c = tile_coord(t / ksplits, tm, tn, band);
-      const int4 tile = __ldg(p.tiles + c.m_idx);
+      const int4 tile = tile_at(p.src, c.m_idx);
       const int n0 = c.n_idx * bn_eff;
       const int n_end = min(p.n, n0 + bn_eff);  // first column this tile does not own
       const uint32_t s = it & 1u, aphase = (it >> 1) & 1u;
       const bool row_valid = r < tile.y;
       const int srow = tile.x + r;
       float sxr = 0.f;
-      if (row_valid) sxr = ROWS ? *(p.sx + srow) : __ldg(p.sx + srow);
+      if (row_valid) sxr = __ldcg(p.sx + srow);
       const int64_t orow = row_valid ? (p.out_row_map != nullptr ? __ldg(p.out_row_map + srow) : srow) : 0;
       if (rows_lora) {
         // the LoRA term of this tile, computed while the tensor cores still work on it
@@ -922,7 +991,9 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) w8a8_gemm_pair_kernel(const _
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  const int tm = *p.num_tiles;
+  pdl_wait();
+  pdl_trigger();
+  const int tm = tile_count(p.src);
   const int tp = (tm + 1) / 2;  // tile pairs
   const int tn = (p.n + PAIR_BN - 1) / PAIR_BN;
   const int total = tp * tn;
@@ -932,132 +1003,85 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) w8a8_gemm_pair_kernel(const _
   if (warp == 16) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
+      Pipe q = {smem, full_bar, empty_bar, PAIR_STAGES, PAIR_STAGE_BYTES, 0, 0u};
       bool ok = true;
-      auto lora_slots_of = [&](int row0, int n0, int adapter, int zslot) -> bool {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-        unsigned char* sa = smem + stage * PAIR_STAGE_BYTES;
-        mbar_expect_tx(&full_bar[stage], 2 * Z_PLANE_BYTES);
-        tma_load_3d(sa, &p.tm_z, 0, 3 * zslot + 2, row0, &full_bar[stage]);
-        tma_load_3d(sa + Z_PLANE_BYTES, &p.tm_z, 0, 3 * zslot + 1, row0, &full_bar[stage]);
-        if (++stage == PAIR_STAGES) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-        sa = smem + stage * PAIR_STAGE_BYTES;
-        mbar_expect_tx(&full_bar[stage], Z_PLANE_BYTES + PAIR_BN * LORA_ROW_BYTES);
-        tma_load_3d(sa, &p.tm_z, 0, 3 * zslot, row0, &full_bar[stage]);
-        tma_load_3d(sa + Z_PLANE_BYTES, &p.tm_b, 0, n0, adapter, &full_bar[stage]);
-        if (++stage == PAIR_STAGES) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        return true;
-      };
-      auto lora_slots = [&](const int4& tile, int n0) -> bool {  // both adapter slots of a two-adapter tile
-        if (!lora_slots_of(tile.x, n0, tile.z, 0)) return false;
-        return tile.w == 0 || lora_slots_of(tile.x, n0, (tile.w & 0xffff) - 1, 1);
-      };
       for (uint32_t it = 0; ok; ++it) {
         const int t = sched_claim(ring, it, p.sched, total, abort_flag, p.status, ok);
         if (t < 0) break;
         const TileCoord c = tile_coord(t, tp, tn, band);
-        const int4 tile_a = __ldg(p.tiles + 2 * c.m_idx);
+        const int4 tile_a = tile_at(p.src, 2 * c.m_idx);
         const bool has_b = 2 * c.m_idx + 1 < tm;
-        const int4 tile_b = has_b ? __ldg(p.tiles + 2 * c.m_idx + 1) : tile_a;
+        const int4 tile_b = has_b ? tile_at(p.src, 2 * c.m_idx + 1) : tile_a;
         const int n0 = c.n_idx * PAIR_BN;
         const uint32_t tx = (has_b ? 2 : 1) * BM * BK + PAIR_BN * BK;
         for (int kb = 0; kb < kblocks; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER);
+          const int stage = q.stage;
+          ok = mbar_wait(&empty_bar[stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER);
           if (!ok) break;
-          unsigned char* sa = smem + stage * PAIR_STAGE_BYTES;
+          unsigned char* sa = q.at();
           mbar_expect_tx(&full_bar[stage], tx);
           tma_load_2d(sa, &p.tm_xq, kb * BK, tile_a.x, &full_bar[stage]);
           if (has_b) tma_load_2d(sa + BM * BK, &p.tm_xq, kb * BK, tile_b.x, &full_bar[stage]);
           tma_load_3d(sa + PAIR_A_BYTES, &p.tm_w, 0, n0, kb, &full_bar[stage]);
-          if (++stage == PAIR_STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          q.next();
         }
         if (HAS_LORA && ok) {
-          ok = lora_slots(tile_a, n0);
-          if (ok && has_b) ok = lora_slots(tile_b, n0);
+          ok = lora_load(p, q, tile_a, n0, abort_flag);
+          if (ok && has_b) ok = lora_load(p, q, tile_b, n0, abort_flag);
         }
       }
     }
   } else if (warp == 17) {
-    // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    // ------------------------------ MMA issuer (whole warp, elected thread) ----
+    {
       const uint32_t idesc = make_idesc(IDESC_D_S32, IDESC_S8, IDESC_S8, BM, PAIR_BN);
       const uint32_t idesc_lora = make_idesc(IDESC_D_F32, IDESC_BF16, IDESC_BF16, BM, PAIR_BN);
-      int stage = 0;
-      uint32_t phase = 0, it = 0;
+      Pipe q = {smem, full_bar, empty_bar, PAIR_STAGES, PAIR_STAGE_BYTES, 0, 0u};
+      const uint32_t smem_base = smem_u32(smem);
+      uint32_t it = 0;
       bool ok = true;
-      auto lora_mma = [&](uint32_t d, bool wait_conv, uint32_t conv_parity) -> bool {
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-        const int st1 = stage;
-        if (++stage == PAIR_STAGES) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-        const int st2 = stage;
-        if (++stage == PAIR_STAGES) {
-          stage = 0;
-          phase ^= 1u;
-        }
-        if (wait_conv && !mbar_wait(conv_done, conv_parity, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-        tc_fence_after_sync();
-        const uint32_t e1 = smem_u32(smem + st1 * PAIR_STAGE_BYTES), e2 = smem_u32(smem + st2 * PAIR_STAGE_BYTES);
-        const uint64_t bd = make_desc_sw128(e2 + Z_PLANE_BYTES);
-        const uint64_t zd[3] = {make_desc_sw128(e1), make_desc_sw128(e1 + Z_PLANE_BYTES), make_desc_sw128(e2)};
-        for (int plane = 0; plane < 3; ++plane)
-          for (int kk = 0; kk < p.rank_blocks; ++kk) mma_bf16(d, zd[plane] + 2 * kk, bd + 2 * kk, idesc_lora, 1u);
-        mma_commit(&empty_bar[st1]);
-        mma_commit(&empty_bar[st2]);
-        return true;
-      };
       for (; ok; ++it) {
         const int t = sched_read(ring, it, abort_flag, p.status, STATUS_TIMEOUT_MMA, ok);
-        if (ok) sched_release(ring, it);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane == 0) sched_release(ring, it);
         if (t < 0) break;
         const TileCoord c = tile_coord(t, tp, tn, band);
         const bool has_b = 2 * c.m_idx + 1 < tm;
-        ok = mbar_wait(tmem_empty, (it & 1u) ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_MMA);
+        ok = mbar_wait_warp(tmem_empty, (it & 1u) ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_MMA);
         if (!ok) break;
         tc_fence_after_sync();
         for (int kb = 0; kb < kblocks; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_MMA);
+          ok = mbar_wait_warp(&full_bar[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_MMA);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * PAIR_STAGE_BYTES);
-          const uint64_t a0 = make_desc_sw128(sa), a1 = make_desc_sw128(sa + BM * BK);
-          const uint64_t bdesc = make_desc_sw128(sa + PAIR_A_BYTES);
+          const uint32_t sa = smem_base + q.stage * PAIR_STAGE_BYTES;
+          if (elect_one()) {
+            const uint64_t a0 = make_desc_sw128(sa), a1 = make_desc_sw128(sa + BM * BK);
+            const uint64_t bdesc = make_desc_sw128(sa + PAIR_A_BYTES);
 #pragma unroll
-          for (int j = 0; j < BK / UMMA_K_I8; ++j) {
-            const uint32_t accumulate = (kb != 0 || j != 0) ? 1u : 0u;
-            mma_i8(tmem_base, a0 + 2 * j, bdesc + 2 * j, idesc, accumulate);
-            if (has_b) mma_i8(tmem_base + PAIR_BN, a1 + 2 * j, bdesc + 2 * j, idesc, accumulate);
+            for (int j = 0; j < BK / UMMA_K_I8; ++j) {
+              const uint32_t accumulate = (kb != 0 || j != 0) ? 1u : 0u;
+              mma_i8(tmem_base, a0 + 2 * j, bdesc + 2 * j, idesc, accumulate);
+              if (has_b) mma_i8(tmem_base + PAIR_BN, a1 + 2 * j, bdesc + 2 * j, idesc, accumulate);
+            }
+            mma_commit(&empty_bar[q.stage]);
           }
-          mma_commit(&empty_bar[stage]);
-          if (++stage == PAIR_STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          __syncwarp();
+          q.next();
         }
         if (!ok) break;
-        mma_commit(tmem_full);
+        if (elect_one()) mma_commit(tmem_full);
+        __syncwarp();
         if (HAS_LORA) {
-          const int second_a = __ldg(p.tiles + 2 * c.m_idx).w;
-          const int second_b = has_b ? __ldg(p.tiles + 2 * c.m_idx + 1).w : 0;
-          ok = lora_mma(tmem_base, true, it & 1u);
-          if (ok && second_a != 0) ok = lora_mma(tmem_base, false, 0u);
-          if (ok && has_b) ok = lora_mma(tmem_base + PAIR_BN, false, 0u);
-          if (ok && second_b != 0) ok = lora_mma(tmem_base + PAIR_BN, false, 0u);
-          if (ok) mma_commit(lora_done);
+          ok = lora_issue(p, q, tile_at(p.src, 2 * c.m_idx), tmem_base, idesc_lora, abort_flag, [&]() {
+            return mbar_wait_warp(conv_done, it & 1u, abort_flag, p.status, STATUS_TIMEOUT_LORA);
+          });
+          if (ok && has_b)
+            ok = lora_issue(p, q, tile_at(p.src, 2 * c.m_idx + 1), tmem_base + PAIR_BN, idesc_lora, abort_flag,
+                            []() { return true; });
+          if (ok && elect_one()) mma_commit(lora_done);
+          __syncwarp();
         }
       }
     }
@@ -1078,7 +1102,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) w8a8_gemm_pair_kernel(const _
       const TileCoord c = tile_coord(t, tp, tn, band);
       const int tidx = 2 * c.m_idx + which;
       const bool present = tidx < tm;
-      const int4 tile = present ? __ldg(p.tiles + tidx) : make_int4(0, 0, 0, 0);
+      const int4 tile = present ? tile_at(p.src, tidx) : make_int4(0, 0, 0, 0);
       const int n0 = c.n_idx * PAIR_BN;
       const int n_end = min(p.n, n0 + PAIR_BN);
       const bool row_valid = r < tile.y;
@@ -1142,11 +1166,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) w8a8_gemm_pair_kernel(const _
 // Per unit of tensor-core work a CTA pulls a third fewer bytes from L2, which is what bounds the single-tile
 // kernel (bytes in flight per SM).  The two M tiles of a pair are neighbours in the tile list.
 //
-// LoRA: one MMA spans both tiles and has ONE B operand, while the two tiles may hold rows of up to four
-// adapters.  For every distinct adapter of the pair the leader issues the rank-r MMAs once, with each CTA
-// staging, at the same offset, the z planes of the slot that adapter has in ITS tile or, if it has none, a
-// box that lies outside the tensor and is therefore filled with zeros; every row receives exactly its own
-// adapter's term.
+// LoRA: one MMA spans both tiles and has ONE B operand, while the two tiles hold rows of several adapters.  The
+// leader issues the rank-r MMAs once for every distinct adapter of the pair, on the lanes of that adapter's rows.
 //
 // Static schedule (pair i takes tiles i, i + pairs, ...).  Barriers: TMA loads of both CTAs report to the
 // leader's full barrier; commits arrive on both CTAs' barriers; the epilogue warps of both CTAs release an
@@ -1162,32 +1183,30 @@ constexpr int PAIR2_THREADS = (PAIR2_EPI_WARPS + 2) * 32;
 constexpr int PAIR2_STAGE_AREA = STAGE_AREA_BYTES - PAIR2_EPI_WARPS * EPI_STAGE_BYTES;   // store-staging tiles on top
 constexpr int PAIR2_STAGES = PAIR2_STAGE_AREA / PAIR2_STAGE_BYTES;                        // 5
 
-struct PairAdapters {
-  int count;       // distinct adapters of the pair, <= 4
-  int adapter[4];
-  int slot[4];     // z slot of that adapter in THIS CTA's tile (0 / 1) or -1 (none: zero planes)
+// The distinct adapters of a pair of neighbouring tiles.  Tiles follow the adapter order, so the only adapter they can
+// share is the last of the first and the first of the second.
+struct PairSegments {
+  int4 t0, t1;
+  int n0, shared, count;
 };
-// `first` / `second` of the two tiles of a pair (second == 0: none); `mine` selects this CTA's tile
-__device__ __forceinline__ PairAdapters pair_adapters(const int4& t0, bool has1, const int4& t1, int mine) {
-  PairAdapters pa;
-  pa.count = 0;
-  const int cand[4] = {t0.z, t0.w != 0 ? (t0.w & 0xffff) - 1 : -1, has1 ? t1.z : -1, (has1 && t1.w != 0) ? (t1.w & 0xffff) - 1 : -1};
-  const int4& me = mine == 0 ? t0 : t1;
-  const bool have_me = mine == 0 || has1;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (cand[i] < 0) continue;
-    bool seen = false;
-    for (int j = 0; j < pa.count; ++j) seen = seen || pa.adapter[j] == cand[i];
-    if (seen) continue;
-    int slot = -1;
-    if (have_me && me.z == cand[i]) slot = 0;
-    else if (have_me && me.w != 0 && (me.w & 0xffff) - 1 == cand[i]) slot = 1;
-    pa.adapter[pa.count] = cand[i];
-    pa.slot[pa.count] = slot;
-    ++pa.count;
-  }
-  return pa;
+__device__ __forceinline__ PairSegments pair_segments(const TileSource& src, const int4& t0, bool has1, const int4& t1) {
+  PairSegments q;
+  q.t0 = t0;
+  q.t1 = t1;
+  q.n0 = tile_segments(t0);
+  const int n1 = has1 ? tile_segments(t1) : 0;
+  q.shared = n1 > 0 && segment_adapter(src, t0, q.n0 - 1) == segment_adapter(src, t1, 0) ? 1 : 0;
+  q.count = q.n0 + n1 - q.shared;
+  return q;
+}
+// index of pair segment g in the tile of CTA `rank`, or -1
+__device__ __forceinline__ int pair_segment_of(const PairSegments& q, int g, int rank) {
+  if (rank == 0) return g < q.n0 ? g : -1;
+  const int j = g - q.n0 + q.shared;
+  return j >= 0 ? j : -1;
+}
+__device__ __forceinline__ int pair_segment_adapter(const TileSource& src, const PairSegments& q, int g) {
+  return g < q.n0 ? segment_adapter(src, q.t0, g) : segment_adapter(src, q.t1, g - q.n0 + q.shared);
 }
 
 template <int EPI, bool HAS_LORA>
@@ -1244,7 +1263,9 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  const int tm = *p.num_tiles;
+  pdl_wait();
+  pdl_trigger();
+  const int tm = tile_count(p.src);
   const int tpairs = (tm + 1) / 2;
   const int tn = (p.n + PAIR2_BN - 1) / PAIR2_BN;
   const int total = tpairs * tn;
@@ -1268,36 +1289,49 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
           phase ^= 1u;
         }
       };
-      // LoRA operands of the pair's previous tile: per distinct adapter two pipeline slots
-      // (slot A: z parts lo and mid; slot B: z part hi and this CTA's half of the adapter's B tile)
+      // LoRA operands of the pair's previous tile: the z planes of this CTA's rows, and this CTA's half of the
+      // LoRA-B tile of every distinct adapter of the pair
       auto lora_slots = [&]() -> bool {
-        const PairAdapters pa = pair_adapters(prev0, prev_has1, prev1, static_cast<int>(rank));
-        const int4& me = rank == 0 ? prev0 : prev1;
-        for (int g = 0; g < pa.count; ++g) {
-          const int zrow = pa.slot[g] >= 0 ? me.x : oob_row;
-          const int zs = pa.slot[g] >= 0 ? pa.slot[g] : 0;
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-          unsigned char* sa = smem + stage * PAIR2_STAGE_BYTES;
-          uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * 2 * Z_PLANE_BYTES);
-          tma_load_3d_pair(sa, &p.tm_z, 0, 3 * zs + 2, zrow, fb);
-          tma_load_3d_pair(sa + Z_PLANE_BYTES, &p.tm_z, 0, 3 * zs + 1, zrow, fb);
-          next_stage();
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-          sa = smem + stage * PAIR2_STAGE_BYTES;
-          fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * (Z_PLANE_BYTES + 128 * LORA_ROW_BYTES));
-          tma_load_3d_pair(sa, &p.tm_z, 0, 3 * zs, zrow, fb);
-          tma_load_3d_pair(sa + Z_PLANE_BYTES, &p.tm_b, 0, prev_n0 + static_cast<int>(rank) * 128, pa.adapter[g], fb);
-          next_stage();
+        const LoraGeom& geom = p.lora;
+        const PairSegments ps = pair_segments(p.src, prev0, prev_has1, prev1);
+        const bool dense = tile_is_dense(prev0);
+        const int zrow = rank == 0 ? prev0.x : (prev_has1 ? prev1.x : oob_row);
+        for (int g = 0; g < ps.count;) {
+          // z slot of this adapter in this CTA's tile (lists of two slots; dense lists use the first); the lanes of a
+          // tile the adapter does not occur in are left untouched by the MMA, so what is loaded for them is irrelevant
+          const int mine = pair_segment_of(ps, g, static_cast<int>(rank));
+          const int zs = (!dense && mine > 0) ? mine : 0;
+          for (int pl = 0; pl < 3; pl += geom.z_per_slot) {
+            const int cnt = min(geom.z_per_slot, 3 - pl);
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
+            unsigned char* sa = smem + stage * PAIR2_STAGE_BYTES;
+            const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
+            if (leader) mbar_expect_tx(&full_bar[stage], 2 * cnt * geom.z_plane);
+            for (int i = 0; i < cnt; ++i)
+              tma_load_3d_pair(sa + i * geom.z_plane, &p.tm_z, 0, 3 * zs + 2 - (pl + i), zrow, fb);
+            next_stage();
+          }
+          for (int left = dense ? min(ps.count - g, geom.b_per_round) : 1; left > 0;) {
+            const int cnt = min(geom.b_per_slot, left);
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
+            unsigned char* sa = smem + stage * PAIR2_STAGE_BYTES;
+            const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
+            if (leader) mbar_expect_tx(&full_bar[stage], 2 * cnt * geom.b_tile);
+            for (int i = 0; i < cnt; ++i)
+              tma_load_3d_pair(sa + i * geom.b_tile, &p.tm_b, 0, prev_n0 + static_cast<int>(rank) * 128,
+                               pair_segment_adapter(p.src, ps, g + i), fb);
+            next_stage();
+            g += cnt;
+            left -= cnt;
+          }
         }
         return true;
       };
       for (int t = pair_id; t < total && ok; t += num_pairs) {
         const TileCoord c = tile_coord(t, tpairs, tn, band);
-        const int4 t0 = __ldg(p.tiles + 2 * c.m_idx);
+        const int4 t0 = tile_at(p.src, 2 * c.m_idx);
         const bool has1 = 2 * c.m_idx + 1 < tm;
-        const int4 t1 = has1 ? __ldg(p.tiles + 2 * c.m_idx + 1) : make_int4(oob_row, 0, 0, 0);
+        const int4 t1 = has1 ? tile_at(p.src, 2 * c.m_idx + 1) : make_int4(oob_row, 0, 0, 0);
         const int row0 = rank == 0 ? t0.x : (has1 ? t1.x : oob_row);
         const int n0 = c.n_idx * PAIR2_BN;
         const int inject_at = min(LORA_INJECT_AFTER, kblocks);
@@ -1325,15 +1359,16 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
       if (HAS_LORA && have_prev && ok) lora_slots();
     }
   } else if (warp == PAIR2_EPI_WARPS + 1) {
-    // ------------------------------ MMA issuer (the leader only) ---------------------------
-    if (lane == 0 && leader) {
+    // ------------------------------ MMA issuer (the leader's warp, elected thread) ---------
+    if (leader) {
       const uint32_t idesc = make_idesc(IDESC_D_S32, IDESC_S8, IDESC_S8, 2 * BM, PAIR2_BN);
       const uint32_t idesc_lora = make_idesc(IDESC_D_F32, IDESC_BF16, IDESC_BF16, 2 * BM, PAIR2_BN);
+      const uint32_t smem_base = smem_u32(smem);
       int stage = 0;
       uint32_t phase = 0, it = 0, lora_rounds = 0;
       bool ok = true, have_prev = false;
       uint32_t prev_s = 0;
-      int prev_groups = 0;
+      PairSegments prev_ps = {};
       const bool prof = p.profile != 0 && blockIdx.x == 0;
       IssuerProfile pr;
       const long long prof_t0 = clock64();
@@ -1343,26 +1378,54 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
           phase ^= 1u;
         }
       };
-      auto lora_mma = [&](uint32_t acc_stage, int groups) -> bool {
-        for (int g = 0; g < groups; ++g) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-          const int st1 = stage;
-          next_stage();
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-          const int st2 = stage;
-          next_stage();
+      auto lora_mma = [&](uint32_t acc_stage, const PairSegments& ps) -> bool {
+        const LoraGeom& geom = p.lora;
+        const bool dense = tile_is_dense(ps.t0);
+        const uint32_t d = tmem_base + acc_stage * PAIR2_BN;
+        const int zslots = (3 + geom.z_per_slot - 1) / geom.z_per_slot;
+        for (int g = 0; g < ps.count;) {
+          const int zstage0 = stage;
+          for (int i = 0; i < zslots; ++i) {
+            if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
+            next_stage();
+          }
           if (g == 0 && !timed_wait(prof, pr.rewrite, conv_done, lora_rounds & 1u, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-          tc_fence_after_sync();
-          const uint32_t e1 = smem_u32(smem + st1 * PAIR2_STAGE_BYTES), e2 = smem_u32(smem + st2 * PAIR2_STAGE_BYTES);
-          const uint64_t bd = make_desc_sw128(e2 + Z_PLANE_BYTES);
-          const uint64_t zd[3] = {make_desc_sw128(e1), make_desc_sw128(e1 + Z_PLANE_BYTES), make_desc_sw128(e2)};
-          const uint32_t d = tmem_base + acc_stage * PAIR2_BN;
-          for (int plane = 0; plane < 3; ++plane)   // smallest plane first
-            for (int kk = 0; kk < p.rank_blocks; ++kk) mma_bf16_pair(d, zd[plane] + 2 * kk, bd + 2 * kk, idesc_lora, 1u);
-          mma_commit_pair(&empty_bar[st1]);
-          mma_commit_pair(&empty_bar[st2]);
+          for (int left = dense ? min(ps.count - g, geom.b_per_round) : 1; left > 0;) {
+            const int cnt = min(geom.b_per_slot, left);
+            if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
+            tc_fence_after_sync();
+            const uint32_t base = smem_base + stage * PAIR2_STAGE_BYTES;
+            for (int i = 0; i < cnt; ++i) {
+              const int j0 = pair_segment_of(ps, g + i, 0), j1 = pair_segment_of(ps, g + i, 1);
+              const int4 none = make_int4(0, 0, 0, 0);
+              const int4 m0 = j0 >= 0 ? segment_mask(p.src, ps.t0, j0) : none;
+              const int4 m1 = j1 >= 0 && ps.t1.y > 0 ? segment_mask(p.src, ps.t1, j1) : none;
+              const int4 off0 = make_int4(~m0.x, ~m0.y, ~m0.z, ~m0.w), off1 = make_int4(~m1.x, ~m1.y, ~m1.z, ~m1.w);
+              const uint64_t bd = make_desc_width(base + i * geom.b_tile, geom.w);
+              if (elect_one()) {
+                for (int plane = 0; plane < 3; ++plane) {  // smallest plane first
+                  int zs = zstage0 + plane / geom.z_per_slot;
+                  if (zs >= PAIR2_STAGES) zs -= PAIR2_STAGES;
+                  const uint64_t zd = make_desc_width(smem_base + zs * PAIR2_STAGE_BYTES + (plane % geom.z_per_slot) * geom.z_plane, geom.w);
+                  for (int kk = 0; kk < p.rank_blocks; ++kk)
+                    mma_bf16_pair_lanes(d, zd + 2 * kk, bd + 2 * kk, idesc_lora, 1u, off0, off1);
+                }
+              }
+              __syncwarp();
+            }
+            if (elect_one()) mma_commit_pair(&empty_bar[stage]);
+            __syncwarp();
+            next_stage();
+            g += cnt;
+            left -= cnt;
+          }
+          if (elect_one()) {
+            for (int i = 0; i < zslots; ++i) mma_commit_pair(&empty_bar[(zstage0 + i) % PAIR2_STAGES]);
+          }
+          __syncwarp();
         }
-        mma_commit_pair(lora_done);
+        if (elect_one()) mma_commit_pair(lora_done);
+        __syncwarp();
         ++lora_rounds;
         return true;
       };
@@ -1372,13 +1435,13 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d = tmem_base + s * PAIR2_BN;
-        int groups = 0;
+        PairSegments ps = {};
         if (HAS_LORA) {
           const TileCoord c = tile_coord(t, tpairs, tn, band);
-          const int4 t0 = __ldg(p.tiles + 2 * c.m_idx);
+          const int4 t0 = tile_at(p.src, 2 * c.m_idx);
           const bool has1 = 2 * c.m_idx + 1 < tm;
-          const int4 t1 = has1 ? __ldg(p.tiles + 2 * c.m_idx + 1) : make_int4(0, 0, 0, 0);
-          groups = pair_adapters(t0, has1, t1, 0).count;
+          const int4 t1 = has1 ? tile_at(p.src, 2 * c.m_idx + 1) : make_int4(0, 0, 0, 0);
+          ps = pair_segments(p.src, t0, has1, t1);
         }
         const int inject_at = min(LORA_INJECT_AFTER, kblocks);
         int issued = 0;
@@ -1386,26 +1449,30 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
           ok = timed_wait(prof, pr.operands, &full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_MMA);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * PAIR2_STAGE_BYTES);
-          const uint64_t adesc = make_desc_sw128(sa);
-          const uint64_t bdesc = make_desc_sw128(sa + BM * BK);
+          const uint32_t sa = smem_base + stage * PAIR2_STAGE_BYTES;
+          if (elect_one()) {
+            const uint64_t adesc = make_desc_sw128(sa);
+            const uint64_t bdesc = make_desc_sw128(sa + BM * BK);
 #pragma unroll
-          for (int j = 0; j < BK / UMMA_K_I8; ++j)
-            mma_i8_pair(d, adesc + 2 * j, bdesc + 2 * j, idesc, (kb != 0 || j != 0) ? 1u : 0u);
-          mma_commit_pair(&empty_bar[stage]);
+            for (int j = 0; j < BK / UMMA_K_I8; ++j)
+              mma_i8_pair(d, adesc + 2 * j, bdesc + 2 * j, idesc, (kb != 0 || j != 0) ? 1u : 0u);
+            mma_commit_pair(&empty_bar[stage]);
+          }
+          __syncwarp();
           next_stage();
           if (HAS_LORA && have_prev && ++issued == inject_at) {
-            ok = lora_mma(prev_s, prev_groups);
+            ok = lora_mma(prev_s, prev_ps);
             if (!ok) break;
           }
         }
-        if (ok) mma_commit_pair(&tmem_full[s]);
+        if (ok && elect_one()) mma_commit_pair(&tmem_full[s]);
+        __syncwarp();
         prev_s = s;
-        prev_groups = groups;
+        prev_ps = ps;
         have_prev = true;
       }
-      if (HAS_LORA && have_prev && ok) lora_mma(prev_s, prev_groups);
-      if (prof) store_profile(pr, p.status, clock64() - prof_t0);
+      if (HAS_LORA && have_prev && ok) lora_mma(prev_s, prev_ps);
+      if (prof && lane == 0) store_profile(pr, p.status, clock64() - prof_t0);
     }
   } else {
     // ------------------------------ epilogue warps 0-15 (both CTAs, own tile) ---------------
@@ -1420,7 +1487,7 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
       const TileCoord c = tile_coord(t, tpairs, tn, band);
       const int tidx = 2 * c.m_idx + static_cast<int>(rank);
       const bool present = tidx < tm;
-      const int4 tile = present ? __ldg(p.tiles + tidx) : make_int4(0, 0, 0, 0);
+      const int4 tile = present ? tile_at(p.src, tidx) : make_int4(0, 0, 0, 0);
       const int n0 = c.n_idx * PAIR2_BN;
       const int n_end = min(p.n, n0 + PAIR2_BN);
       const uint32_t s = it & 1u, aphase = (it >> 1) & 1u;
@@ -1476,67 +1543,67 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
 }
 
 template <int EPI, bool HAS_LORA>
-static int launch_pair2_variant(const GemmParams& p, int grid, cudaStream_t stream) {
+static int launch_pair2_variant(const GemmParams& p, int grid, cudaStream_t stream, bool programmatic) {
   using Cfg = GemmCfg<PAIR2_BN>;
   auto kernel = w8a8_gemm_pair2_kernel<EPI, HAS_LORA>;
   static bool attr_set[MAX_DEVICES] = {};
   cudaError_t e = ensure_dynamic_smem(kernel, Cfg::SMEM_BYTES, attr_set);
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "gemm attribute: %s", cudaGetErrorString(e));
-  kernel<<<grid, PAIR2_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
-  e = cudaPeekAtLastError();
+  e = launch_kernel(kernel, dim3(grid), dim3(PAIR2_THREADS), Cfg::SMEM_BYTES, stream, programmatic, p);
+  if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "gemm launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;
 }
 
-static int launch_pair2(const GemmParams& p, int epi, bool lora, int grid, cudaStream_t stream) {
+static int launch_pair2(const GemmParams& p, int epi, bool lora, int grid, cudaStream_t stream, bool programmatic) {
   switch (epi) {
     case SKYRL_EPI_LINEAR:
-      return lora ? launch_pair2_variant<SKYRL_EPI_LINEAR, true>(p, grid, stream)
-                  : launch_pair2_variant<SKYRL_EPI_LINEAR, false>(p, grid, stream);
+      return lora ? launch_pair2_variant<SKYRL_EPI_LINEAR, true>(p, grid, stream, programmatic)
+                  : launch_pair2_variant<SKYRL_EPI_LINEAR, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_SWIGLU:
-      return lora ? launch_pair2_variant<SKYRL_EPI_SWIGLU, true>(p, grid, stream)
-                  : launch_pair2_variant<SKYRL_EPI_SWIGLU, false>(p, grid, stream);
+      return lora ? launch_pair2_variant<SKYRL_EPI_SWIGLU, true>(p, grid, stream, programmatic)
+                  : launch_pair2_variant<SKYRL_EPI_SWIGLU, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_RESIDUAL:
-      return lora ? launch_pair2_variant<SKYRL_EPI_RESIDUAL, true>(p, grid, stream)
-                  : launch_pair2_variant<SKYRL_EPI_RESIDUAL, false>(p, grid, stream);
+      return lora ? launch_pair2_variant<SKYRL_EPI_RESIDUAL, true>(p, grid, stream, programmatic)
+                  : launch_pair2_variant<SKYRL_EPI_RESIDUAL, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_PARTIAL_F32:
-      return lora ? launch_pair2_variant<SKYRL_EPI_PARTIAL_F32, true>(p, grid, stream)
-                  : launch_pair2_variant<SKYRL_EPI_PARTIAL_F32, false>(p, grid, stream);
+      return lora ? launch_pair2_variant<SKYRL_EPI_PARTIAL_F32, true>(p, grid, stream, programmatic)
+                  : launch_pair2_variant<SKYRL_EPI_PARTIAL_F32, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_ACC_I32:
-      return launch_pair2_variant<SKYRL_EPI_ACC_I32, false>(p, grid, stream);
+      return launch_pair2_variant<SKYRL_EPI_ACC_I32, false>(p, grid, stream, programmatic);
     default:
       return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: unknown epilogue %d", epi);
   }
 }
 
 template <int EPI, bool HAS_LORA>
-static int launch_pair_variant(const GemmParams& p, int grid, cudaStream_t stream) {
+static int launch_pair_variant(const GemmParams& p, int grid, cudaStream_t stream, bool programmatic) {
   auto kernel = w8a8_gemm_pair_kernel<EPI, HAS_LORA>;
   static bool attr_set[MAX_DEVICES] = {};
   cudaError_t e = ensure_dynamic_smem(kernel, PAIR_SMEM_BYTES, attr_set);
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "gemm attribute: %s", cudaGetErrorString(e));
-  kernel<<<grid, PAIR_THREADS, PAIR_SMEM_BYTES, stream>>>(p);
-  e = cudaPeekAtLastError();
+  e = launch_kernel(kernel, dim3(grid), dim3(PAIR_THREADS), PAIR_SMEM_BYTES, stream, programmatic, p);
+  if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "gemm launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;
 }
 
-static int launch_pair(const GemmParams& p, int epi, bool lora, int grid, cudaStream_t stream) {
+static int launch_pair(const GemmParams& p, int epi, bool lora, int grid, cudaStream_t stream, bool programmatic) {
   switch (epi) {
     case SKYRL_EPI_LINEAR:
-      return lora ? launch_pair_variant<SKYRL_EPI_LINEAR, true>(p, grid, stream)
-                  : launch_pair_variant<SKYRL_EPI_LINEAR, false>(p, grid, stream);
+      return lora ? launch_pair_variant<SKYRL_EPI_LINEAR, true>(p, grid, stream, programmatic)
+                  : launch_pair_variant<SKYRL_EPI_LINEAR, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_SWIGLU:
-      return lora ? launch_pair_variant<SKYRL_EPI_SWIGLU, true>(p, grid, stream)
-                  : launch_pair_variant<SKYRL_EPI_SWIGLU, false>(p, grid, stream);
+      return lora ? launch_pair_variant<SKYRL_EPI_SWIGLU, true>(p, grid, stream, programmatic)
+                  : launch_pair_variant<SKYRL_EPI_SWIGLU, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_RESIDUAL:
-      return lora ? launch_pair_variant<SKYRL_EPI_RESIDUAL, true>(p, grid, stream)
-                  : launch_pair_variant<SKYRL_EPI_RESIDUAL, false>(p, grid, stream);
+      return lora ? launch_pair_variant<SKYRL_EPI_RESIDUAL, true>(p, grid, stream, programmatic)
+                  : launch_pair_variant<SKYRL_EPI_RESIDUAL, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_PARTIAL_F32:
-      return lora ? launch_pair_variant<SKYRL_EPI_PARTIAL_F32, true>(p, grid, stream)
-                  : launch_pair_variant<SKYRL_EPI_PARTIAL_F32, false>(p, grid, stream);
+      return lora ? launch_pair_variant<SKYRL_EPI_PARTIAL_F32, true>(p, grid, stream, programmatic)
+                  : launch_pair_variant<SKYRL_EPI_PARTIAL_F32, false>(p, grid, stream, programmatic);
     case SKYRL_EPI_ACC_I32:
-      return launch_pair_variant<SKYRL_EPI_ACC_I32, false>(p, grid, stream);
+      return launch_pair_variant<SKYRL_EPI_ACC_I32, false>(p, grid, stream, programmatic);
     default:
       return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: unknown epilogue %d", epi);
   }
@@ -1646,7 +1713,7 @@ GemmPlan plan_gemm(int m, int n, int k, int epilogue, int max_slabs) {
   return pl;
 }
 
-int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic) {
+int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic, const TileSource* src) {
   if (a.struct_size != sizeof(SkyrlW8A8GemmArgs))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: struct_size %u does not match ABI v%d (%zu)", a.struct_size,
                 SKYRL_W8A8_ABI_VERSION, sizeof(SkyrlW8A8GemmArgs));
@@ -1654,9 +1721,9 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   if (a.k % 16 != 0) return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: K must be a multiple of 16, got %d", a.k);
   if (a.n % 16 != 0) return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: N must be a multiple of 16, got %d", a.n);
   if (a.xq == nullptr || a.sx == nullptr || a.wq == nullptr || a.sw == nullptr || a.out == nullptr ||
-      a.tiles == nullptr || a.num_tiles == nullptr || a.status == nullptr)
+      (src == nullptr && (a.tiles == nullptr || a.num_tiles == nullptr)) || a.status == nullptr)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: null buffer");
-  if (!aligned16(a.xq) || !aligned16(a.wq) || !aligned16(a.sw) || !aligned16(a.out) || !aligned16(a.tiles))
+  if (!aligned16(a.xq) || !aligned16(a.wq) || !aligned16(a.sw) || !aligned16(a.out) || !aligned16(src != nullptr ? static_cast<const void*>(src->tiles) : a.tiles))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: buffers must be 16-byte aligned");
   if (a.rank < 0 || a.rank > SKYRL_LORA_RANK_PAD)
     return fail(SKYRL_ERR_UNSUPPORTED, "gemm: LoRA rank must be in [0, %d], got %d", SKYRL_LORA_RANK_PAD, a.rank);
@@ -1685,7 +1752,9 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: output stride must be >= the row length and a multiple of 8");
   if (a.out == a.xq || a.out == a.wq || a.out == a.z_parts)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: output aliases an input");
-  if (a.max_tiles <= 0) return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: max_tiles must be positive");
+  if (src == nullptr && a.max_tiles <= 0) return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: max_tiles must be positive");
+  const int list_tiles = src != nullptr ? src->count : a.max_tiles;  // exact for the internal lists, else a capacity
+  if (list_tiles <= 0) return SKYRL_OK;
 
   const int sms = sm_count();
   if (sms <= 0) return fail(SKYRL_ERR_LAUNCH, "gemm: no CUDA device");
@@ -1725,12 +1794,18 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
                            static_cast<uint64_t>(a.n) * BK, BK, w_box_rows)))
     return rc;
   if (lora) {
+    // the dense table [A, n, rank rounded up to 8] where there is one: a quarter of the 64-slot table's bytes at rank 16
+    const bool dense_b = a.lora_b_rows != nullptr;
+    const void* b_table = dense_b ? a.lora_b_rows : a.lora_b_packed;
+    const int b_slots = dense_b ? a.lora_b_rows_rank : SKYRL_LORA_RANK_PAD;
+    if (!aligned16(b_table) || b_slots < a.rank || b_slots % 8 != 0)
+      return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: LoRA-B table misaligned or of the wrong rank");
+    const uint32_t half = (a.rank <= 16 ? 32 : (a.rank <= 32 ? 64 : 128)) / 2;
     if ((rc = encode_tmap_3d(&p.tm_z, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.z_parts, SKYRL_LORA_RANK_PAD, SKYRL_Z_PARTS,
-                             a.m, LORA_ROW_BYTES, SKYRL_Z_PARTS * LORA_ROW_BYTES, SKYRL_LORA_RANK_PAD, 1, BM)))
+                             a.m, LORA_ROW_BYTES, SKYRL_Z_PARTS * LORA_ROW_BYTES, half, 1, BM)))
       return rc;
-    if ((rc = encode_tmap_3d(&p.tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.lora_b_packed, SKYRL_LORA_RANK_PAD, a.n,
-                             a.num_adapters, LORA_ROW_BYTES, static_cast<uint64_t>(a.n) * LORA_ROW_BYTES,
-                             SKYRL_LORA_RANK_PAD, w_box_rows)))
+    if ((rc = encode_tmap_3d(&p.tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, b_table, b_slots, a.n, a.num_adapters,
+                             static_cast<uint64_t>(b_slots) * 2, static_cast<uint64_t>(a.n) * b_slots * 2, half, w_box_rows)))
       return rc;
   } else {
     p.tm_z = p.tm_xq;
@@ -1738,8 +1813,7 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   }
   p.sx = a.sx;
   p.sw = a.sw;
-  p.tiles = reinterpret_cast<const int4*>(a.tiles);
-  p.num_tiles = a.num_tiles;
+  p.src = src != nullptr ? *src : TileSource{reinterpret_cast<const int4*>(a.tiles), nullptr, nullptr, a.num_tiles, 0, 0, a.m};
   p.out_row_map = a.out_row_map;
   p.residual = static_cast<const __nv_bfloat16*>(a.residual);
   p.out = a.out;
@@ -1758,7 +1832,6 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   // The whole stage area is pipeline depth: the main loop is bound by bytes in flight per SM.
   p.a_rows = (!lora && a.m <= 64) ? 64 : BM;
   p.stage_bytes = p.a_rows * BK + (bn_eff * BK + 1023) / 1024 * 1024;
-  if (lora && p.stage_bytes < 2 * Z_PLANE_BYTES) p.stage_bytes = 2 * Z_PLANE_BYTES;  // a slot also carries two z planes
   p.num_stages = SINGLE_STAGE_AREA / p.stage_bytes;
   p.z_rows = nullptr;
   p.row_ids = nullptr;
@@ -1810,8 +1883,13 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   }
   p.direct_stores = 0;
   if (p.num_stages > MAX_STAGES) p.num_stages = MAX_STAGES;
-  p.sched = a.sched != nullptr ? a.sched : next_sched_counter();
-  if (p.sched == nullptr) return fail(SKYRL_ERR_LAUNCH, "gemm: scheduler counters unavailable");
+  p.lora = LoraGeom{};
+  if (lora)
+    p.lora = lora_geom(a.rank, pair2 ? 128 : bn_eff, pair2 ? PAIR2_STAGE_BYTES : (paired ? PAIR_STAGE_BYTES : p.stage_bytes),
+                       pair2 ? PAIR2_STAGES : (paired ? PAIR_STAGES : p.num_stages));
+  // an internal launch without scheduler words takes its tiles with a fixed stride
+  p.sched = a.sched != nullptr ? a.sched : (src != nullptr ? nullptr : next_sched_counter());
+  if (p.sched == nullptr && src == nullptr) return fail(SKYRL_ERR_LAUNCH, "gemm: scheduler counters unavailable");
   p.prefetch = nullptr;
   p.prefetch_bytes = 0;
   if (a.prefetch != nullptr && a.prefetch_bytes > 0) {
@@ -1823,19 +1901,19 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   p.k_splits = k_splits;
   p.kb_per_split = kb_per_split;
   p.slab_stride = static_cast<int64_t>(a.m) * a.out_row_stride;
-  const int64_t max_total = static_cast<int64_t>(a.max_tiles) * ((a.n + bn_eff - 1) / bn_eff) * k_splits;
+  const int64_t max_total = static_cast<int64_t>(list_tiles) * ((a.n + bn_eff - 1) / bn_eff) * k_splits;
   int grid = static_cast<int>(max_total < sms ? max_total : sms);
   if (a.cta_limit > 0 && grid > a.cta_limit) grid = a.cta_limit;  // leave SMs to a concurrent collective
   if (pair2) {
-    const int64_t pair_total = static_cast<int64_t>((a.max_tiles + 1) / 2) * ((a.n + 255) / 256);
+    const int64_t pair_total = static_cast<int64_t>((list_tiles + 1) / 2) * ((a.n + 255) / 256);
     const int pairs = static_cast<int>(pair_total < sms / 2 ? pair_total : sms / 2);
-    return launch_pair2(p, a.epilogue, lora, 2 * pairs, stream);
+    return launch_pair2(p, a.epilogue, lora, 2 * pairs, stream, programmatic);
   }
   if (paired) {
-    const int64_t pair_total = static_cast<int64_t>((a.max_tiles + 1) / 2) * ((a.n + 255) / 256);
+    const int64_t pair_total = static_cast<int64_t>((list_tiles + 1) / 2) * ((a.n + 255) / 256);
     int pgrid = static_cast<int>(pair_total < sms ? pair_total : sms);
     if (a.cta_limit > 0 && pgrid > a.cta_limit) pgrid = a.cta_limit;
-    return launch_pair(p, a.epilogue, lora, pgrid, stream);
+    return launch_pair(p, a.epilogue, lora, pgrid, stream, programmatic);
   }
   if (rows)
     return bn == 256 ? launch_rows_bn<256>(p, a.epilogue, grid, stream, programmatic)
