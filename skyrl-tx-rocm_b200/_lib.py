@@ -129,6 +129,8 @@ SYMBOLS = {
     "skyrl_w8a8_gemm_k_splits": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "skyrl_w8a8_linear_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "skyrl_w8a8_lora_forward_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
+    "skyrl_w8a8_grouped_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "skyrl_w8a8_lora_forward_grouped_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_int32, C.c_void_p]),
     "skyrl_w8a8_lora_forward_noalloc_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "skyrl_rms_gate_up_w8a8_lora_swiglu_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "skyrl_down_w8a8_lora_residual_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),

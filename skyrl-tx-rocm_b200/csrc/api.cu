@@ -497,6 +497,96 @@ extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, sk
   return run_projection(q, stream);
 }
 
+// ---- group-wise scales ---------------------------------------------------------
+namespace skyrl {
+
+struct GroupedWs {
+  RouteWs route;
+  int8_t* xq;
+  float* sx;           // [groups, m]
+  uint16_t* xn;
+  uint16_t* z_parts;
+  size_t bytes;
+};
+
+static GroupedWs carve_grouped(void* ws, int m, int k, int num_adapters, int group) {
+  Carver c(ws);
+  GroupedWs w;
+  w.route = carve_route(c, m, num_adapters);
+  w.xq = c.take<int8_t>(static_cast<size_t>(m) * k);
+  w.sx = c.take<float>(static_cast<size_t>(m) * (k / group));
+  w.xn = c.take<uint16_t>(static_cast<size_t>(m) * k);
+  w.z_parts = c.take<uint16_t>(SKYRL_Z_PARTS * static_cast<size_t>(m) * SKYRL_LORA_RANK_PAD);
+  w.bytes = c.total();
+  return w;
+}
+
+}  // namespace skyrl
+
+extern "C" size_t skyrl_w8a8_grouped_workspace_bytes(int32_t m, int32_t n, int32_t k, int32_t num_adapters,
+                                                      int32_t group_size) {
+  if (m <= 0 || n <= 0 || k <= 0 || group_size <= 0) return 0;
+  return carve_grouped(nullptr, m, k, num_adapters, group_size).bytes;
+}
+
+extern "C" int skyrl_w8a8_lora_forward_grouped_sm100_v1(const SkyrlW8A8LinearArgs* a, int32_t group_size,
+                                                         skyrl_stream_t stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (a == nullptr) return fail(SKYRL_ERR_INVALID_ARGUMENT, "grouped linear: args is null");
+  if (a->struct_size != sizeof(SkyrlW8A8LinearArgs))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "grouped linear: struct_size %u does not match ABI v%d (%zu)", a->struct_size,
+                SKYRL_W8A8_ABI_VERSION, sizeof(SkyrlW8A8LinearArgs));
+  if (a->m <= 0 || a->n <= 0 || a->k <= 0) return fail(SKYRL_ERR_INVALID_ARGUMENT, "grouped linear: non-positive shape");
+  if (group_size <= 0 || group_size % 32 != 0 || a->k % group_size != 0)
+    return fail(SKYRL_ERR_UNSUPPORTED, "grouped linear: the group must be a multiple of 32 that divides K, got %d of %d", group_size, a->k);
+  if (a->x == nullptr || a->wq == nullptr || a->sw == nullptr || a->out == nullptr || a->status == nullptr)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "grouped linear: null buffer");
+  if (a->epilogue != SKYRL_EPI_LINEAR || a->rms_delta != nullptr || a->residual != nullptr)
+    return fail(SKYRL_ERR_UNSUPPORTED, "grouped linear: plain linear epilogue only");
+  if (a->rank < 0 || a->rank > SKYRL_LORA_RANK_PAD)
+    return fail(SKYRL_ERR_UNSUPPORTED, "grouped linear: LoRA rank must be in [0, %d], got %d", SKYRL_LORA_RANK_PAD, a->rank);
+  const bool lora = a->rank > 0;
+  if (lora && (a->lora_a_packed == nullptr || a->lora_b_packed == nullptr || a->lora_scaling == nullptr || a->num_adapters <= 0))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "grouped linear: LoRA tables missing");
+  const int na = a->num_adapters > 0 ? a->num_adapters : 1;
+  const GroupedWs w = carve_grouped(a->workspace, a->m, a->k, na, group_size);
+  int rc = check_ws(a->workspace, a->workspace_bytes, w.bytes, "grouped linear");
+  if (rc) return rc;
+  // adapters in sorted order above one tile of rows, by masks over token order within one
+  const bool routed = lora && a->adapter_ids != nullptr;
+  if (routed && (rc = launch_route_dense(a->adapter_ids, a->m, na, w.route.perm, w.route.tiles, w.route.seg_mask,
+                                         w.route.seg_adapter, a->status, stream, nullptr, 0)))
+    return rc;
+  const int32_t* perm = routed && a->m > SKYRL_TILE_ROWS ? w.route.perm : nullptr;
+  const bool copy = lora && (perm != nullptr || a->x_row_stride != a->k);
+  if ((rc = launch_group_quant(a->x, a->x_row_stride, perm, a->m, a->k, group_size, w.xq, w.sx, copy ? w.xn : nullptr, stream)))
+    return rc;
+  const TileSource src = tile_source(w.route, routed, 0, a->m);
+  if (lora && (rc = launch_lora_a_proj(copy ? static_cast<const void*>(w.xn) : a->x, a->m, a->k, a->lora_a_packed,
+                                       a->lora_scaling, na, a->rank, src, src.count, w.z_parts, a->status, stream)))
+    return rc;
+  GroupedGemmLaunch g = {};
+  g.m = a->m;
+  g.n = a->n;
+  g.k = a->k;
+  g.group = group_size;
+  g.rank = a->rank;
+  g.num_adapters = na;
+  g.src = src;
+  g.xq = w.xq;
+  g.sx = w.sx;
+  g.wq = a->wq;
+  g.sw = a->sw;
+  g.z_parts = w.z_parts;
+  g.b_table = a->lora_b_rows != nullptr ? a->lora_b_rows : a->lora_b_packed;
+  g.b_slots = a->lora_b_rows != nullptr ? a->lora_b_rows_rank : SKYRL_LORA_RANK_PAD;
+  g.out_row_map = perm;
+  g.out = a->out;
+  g.out_stride = a->out_row_stride;
+  g.status = a->status;
+  return launch_grouped_gemm(g, stream);
+}
+
 // One exported target per fused variant: thin wrappers that check what the variant needs and fix the epilogue.
 extern "C" int skyrl_rms_gate_up_w8a8_lora_swiglu_sm100_v1(const SkyrlW8A8LinearArgs* a, skyrl_stream_t stream) {
   if (a == nullptr) return fail(SKYRL_ERR_INVALID_ARGUMENT, "rms_gate_up_swiglu: args is null");

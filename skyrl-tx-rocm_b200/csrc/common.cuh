@@ -101,6 +101,25 @@ int launch_finalize_rows(int epilogue, const int32_t* acc, int slabs, const floa
                          const int32_t* ids, int num_adapters, const void* b_table, int64_t b_adapter_stride,
                          int b_row_stride, int rank, int m, int n, const void* residual, int64_t res_stride, void* out,
                          int64_t out_stride, int32_t* status, cudaStream_t stream, bool programmatic = false);
+// Linear on group-wise scales (grouped_gemm_sm100.cu): a scale per row and group, a weight scale per group and column.
+int launch_group_quant(const void* x, int64_t x_row_stride, const int32_t* row_map, int m, int k, int group, void* xq,
+                       float* sx, void* xn, cudaStream_t stream);
+struct GroupedGemmLaunch {
+  int m, n, k, group, rank, num_adapters;
+  TileSource src;
+  const void* xq;
+  const float* sx;      // [k / group, m]
+  const void* wq;
+  const float* sw;      // [k / group, n]
+  const void* z_parts;
+  const void* b_table;  // bf16 [A, n, b_slots]
+  int b_slots;
+  const int32_t* out_row_map;
+  void* out;
+  int64_t out_stride;
+  int32_t* status;
+};
+int launch_grouped_gemm(const GroupedGemmLaunch& a, cudaStream_t stream);
 int launch_tp_finalize(const float* reduced, const int32_t* perm, const void* residual, void* out, int hidden,
                        int row_begin, int row_count, cudaStream_t stream, bool out_sorted = false);
 int launch_tp_finalize_slabs(const float* const* slabs, int num_slabs, const int32_t* perm, const void* residual,

@@ -31,14 +31,12 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_parts.cuh"
 #include "ptx_sm100.cuh"
 #include "tiles.cuh"
 
 namespace skyrl {
 
-constexpr int BM = 128;       // rows per tile == TMEM lanes
-constexpr int BK = 128;       // int8 elements (bytes) of K per pipeline stage: one 128-byte swizzled row
-constexpr int UMMA_K_I8 = 32; // K of one kind::i8 instruction
 constexpr int GEMM_THREADS = 320;  // warps 0-3 and 6-9 epilogue, warp 4 TMA producer, warp 5 MMA issuer
 constexpr int EPI_THREADS = 256;
 constexpr int LORA_ROW_BYTES = SKYRL_LORA_RANK_PAD * 2;  // 128-byte rows of z and packed B
@@ -58,29 +56,6 @@ struct GemmCfg {
   static constexpr int SMEM_BYTES = BAR_OFF + NUM_BARS * 8 + 16 + 128 + 1024;  // + tmem ptr/abort, tile ring, alignment slack
   static constexpr int TMEM_COLS = 2 * BN;
 };
-
-// The LoRA operands of one M tile x N tile travel through slots of the TMA pipeline, at the width of the rank
-// (w = 32, 64 or 128 bytes per row for ranks up to 16, 32, 64, with the swizzle of that width).  They come in rounds:
-// the three z planes of the tile's rows, then the LoRA-B tiles of its segments (adapters), several to a slot; a round
-// never takes more slots than the pipeline has, so the slots of the planes can stay until its last MMA.
-struct LoraGeom {
-  int w;             // bytes per row of z and of a LoRA-B tile
-  int z_plane;       // bytes of one plane: 128 rows
-  int z_per_slot;    // planes per slot
-  int b_tile;        // bytes of one adapter's LoRA-B tile
-  int b_per_slot;    // adapters per slot
-  int b_per_round;   // adapters per round
-};
-static LoraGeom lora_geom(int rank, int b_rows, int stage_bytes, int stages) {
-  LoraGeom g;
-  g.w = rank <= 16 ? 32 : (rank <= 32 ? 64 : 128);
-  g.z_plane = BM * g.w;
-  g.z_per_slot = stage_bytes / g.z_plane < 3 ? stage_bytes / g.z_plane : 3;
-  g.b_tile = b_rows * g.w;
-  g.b_per_slot = stage_bytes / g.b_tile;
-  g.b_per_round = (stages - (3 + g.z_per_slot - 1) / g.z_per_slot) * g.b_per_slot;
-  return g;
-}
 
 struct GemmParams {
   CUtensorMap tm_xq;   // int8 [M, K], box 128 x 128
@@ -245,104 +220,6 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int tm, int tn, int band)
 
 __device__ __forceinline__ float silu_f32(float t) { return __fdiv_rn(t, 1.0f + expf(-t)); }
 
-
-// ---- LoRA operands of one tile through the TMA pipeline (one CTA per tile; see LoraGeom) ----------------
-struct Pipe {
-  unsigned char* smem;
-  uint64_t* full;
-  uint64_t* empty;
-  int stages, bytes, stage;
-  uint32_t phase;
-  __device__ __forceinline__ void next() {
-    if (++stage == stages) {
-      stage = 0;
-      phase ^= 1u;
-    }
-  }
-  __device__ __forceinline__ unsigned char* at() const { return smem + stage * bytes; }
-};
-
-__device__ __forceinline__ bool lora_load(const GemmParams& p, Pipe& q, const int4& tile, int n0, volatile int* abort_flag) {
-  const LoraGeom& g = p.lora;
-  const int nseg = tile_segments(tile);
-  const bool dense = tile_is_dense(tile);
-  for (int j = 0; j < nseg;) {
-    const int slot = segment_slot(tile, j);
-    for (int pl = 0; pl < 3; pl += g.z_per_slot) {  // lo, mid, hi: the smallest plane is added first
-      if (!mbar_wait(&q.empty[q.stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-      const int cnt = min(g.z_per_slot, 3 - pl);
-      mbar_expect_tx(&q.full[q.stage], cnt * g.z_plane);
-      for (int i = 0; i < cnt; ++i)
-        tma_load_3d(q.at() + i * g.z_plane, &p.tm_z, 0, 3 * slot + 2 - (pl + i), tile.x, &q.full[q.stage]);
-      q.next();
-    }
-    // a list of two slots keeps the second adapter's z elsewhere: every adapter is a round of its own
-    for (int left = dense ? min(nseg - j, g.b_per_round) : 1; left > 0;) {
-      const int cnt = min(g.b_per_slot, left);
-      if (!mbar_wait(&q.empty[q.stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
-      mbar_expect_tx(&q.full[q.stage], cnt * g.b_tile);
-      for (int i = 0; i < cnt; ++i)
-        tma_load_3d(q.at() + i * g.b_tile, &p.tm_b, 0, n0, segment_adapter(p.src, tile, j + i), &q.full[q.stage]);
-      q.next();
-      j += cnt;
-      left -= cnt;
-    }
-  }
-  return true;
-}
-
-// rank-r bf16 MMAs of one tile, accumulated onto the accumulator `d` the epilogue rewrote as fp32 (`ready` waits for
-// that rewrite, once the first operands are there); every segment touches the lanes of its own rows only.  Called by a
-// whole warp, which elects a thread for the instructions.
-template <typename Ready>
-__device__ __forceinline__ bool lora_issue(const GemmParams& p, Pipe& q, const int4& tile, uint32_t d, uint32_t idesc,
-                                           volatile int* abort_flag, Ready ready) {
-  const LoraGeom& g = p.lora;
-  const int nseg = tile_segments(tile);
-  const bool dense = tile_is_dense(tile);
-  for (int j = 0; j < nseg;) {
-    const int zstage0 = q.stage;
-    const int zslots = (3 + g.z_per_slot - 1) / g.z_per_slot;
-    for (int i = 0; i < zslots; ++i) {
-      if (!mbar_wait_warp(&q.full[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-      q.next();
-    }
-    const bool first = j == 0;
-    bool started = false;
-    for (int left = dense ? min(nseg - j, g.b_per_round) : 1; left > 0;) {
-      const int cnt = min(g.b_per_slot, left);
-      if (!mbar_wait_warp(&q.full[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
-      if (first && !started && !ready()) return false;
-      started = true;
-      tc_fence_after_sync();
-      const uint32_t base = smem_u32(q.at());
-      for (int i = 0; i < cnt; ++i) {
-        const int4 mk = segment_mask(p.src, tile, j + i);
-        const int4 off = make_int4(~mk.x, ~mk.y, ~mk.z, ~mk.w);
-        const uint64_t bd = make_desc_width(base + i * g.b_tile, g.w);
-        if (elect_one()) {
-          for (int plane = 0; plane < 3; ++plane) {
-            int zs = zstage0 + plane / g.z_per_slot;
-            if (zs >= q.stages) zs -= q.stages;
-            const uint64_t zd = make_desc_width(smem_u32(q.smem + zs * q.bytes) + (plane % g.z_per_slot) * g.z_plane, g.w);
-            for (int kk = 0; kk < p.rank_blocks; ++kk) mma_bf16_lanes(d, zd + 2 * kk, bd + 2 * kk, idesc, 1u, off);
-          }
-        }
-        __syncwarp();
-      }
-      if (elect_one()) mma_commit(&q.empty[q.stage]);
-      __syncwarp();
-      q.next();
-      j += cnt;
-      left -= cnt;
-    }
-    if (elect_one()) {
-      for (int i = 0; i < zslots; ++i) mma_commit(&q.empty[(zstage0 + i) % q.stages]);
-    }
-    __syncwarp();
-  }
-  return true;
-}
 
 // ---- epilogue building blocks (one 32-column chunk of one TMEM lane quadrant) ------------------------
 // pass 1 of the LoRA path: int32 accumulator -> (f32(acc) * sx[m]) * sw[n], written back in place

@@ -429,9 +429,10 @@ def _lora_of(weight: PackedW8Weight, lora_a, lora_b, lora_scaling) -> PackedLoRA
 
 
 def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids):
-    """Compatibility path for group_size < K: one single-group GEMM per K group into fp32 slabs, then the
-    ordered group sum, the LoRA term (accumulated by the last group's GEMM) and the single bf16 cast
-    (quantized_lora.py:242-254, 298-304).  Correct for every group size; not tuned."""
+    """group_size < K (quantized_lora.py:242-254, 298-304).  Groups of whole 32-wide MMA steps run in one kernel that
+    scales every group's int32 accumulator as it leaves tensor memory; other group sizes take one single-group GEMM
+    per K group into fp32 slabs, then the ordered group sum, the LoRA term (accumulated by the last group's GEMM) and
+    the single bf16 cast: correct for every group size, not tuned."""
     lib = _lib.load()
     m, k, npad, g_size = x2.shape[0], weight.in_features, weight.padded_out_features, weight.group_size
     groups = k // g_size
@@ -439,6 +440,27 @@ def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids
     dev = x2.device
     na = lora.num_adapters if lora is not None else 1
     st = _status_word(dev)
+    if g_size % 32 == 0:
+        out = torch.empty((m, npad), dtype=torch.bfloat16, device=dev)
+        nbytes = lib.skyrl_w8a8_grouped_workspace_bytes(m, npad, k, na, g_size)
+        ws = _workspace(dev, nbytes)
+        a = _lib.LinearArgs()
+        a.struct_size = C.sizeof(_lib.LinearArgs)
+        a.epilogue = EPI_LINEAR
+        a.m, a.n, a.k = m, npad, k
+        a.rank, a.num_adapters = (lora.rank if lora is not None else 0), na
+        a.x, a.x_row_stride = x2.data_ptr(), x2.stride(0)
+        a.wq, a.sw = weight.wq.data_ptr(), weight.sw.data_ptr()
+        if lora is not None:
+            a.lora_a_packed, a.lora_b_packed = lora.a.data_ptr(), lora.b.data_ptr()
+            a.lora_scaling = lora.scaling.data_ptr()
+            if lora.b_rows is not None:
+                a.lora_b_rows, a.lora_b_rows_rank = lora.b_rows.data_ptr(), lora.b_rows.shape[2]
+        a.adapter_ids = ids.data_ptr() if ids is not None else None
+        a.out, a.out_row_stride = out.data_ptr(), npad
+        a.workspace, a.workspace_bytes, a.status = ws.data_ptr(), nbytes, st.data_ptr()
+        _lib.check(lib.skyrl_w8a8_lora_forward_grouped_sm100_v1(C.byref(a), g_size, _stream()), "w8a8_lora_forward_grouped")
+        return out
     perm, tiles, num = prepare_routing(ids, m, na)
     row_map = perm if ids is not None else None
     max_tiles = tiles.shape[0]

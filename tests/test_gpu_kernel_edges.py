@@ -1,0 +1,81 @@
+"""Kernel variants at the sizes where they can go wrong: tile edges, remainders, both ends of their ranges.
+
+Bars: integer work and the frozen base are bit-exact against the oracle.  With the LoRA term the order of the fp32
+sums of length K and r is not pinned: they differ by at most a few 2^-24 of the terms' size, so a bf16 result (2^-9 of
+its value per half step) lands on the other side of a rounding boundary for at most about 2^-24 * 32 / 2^-9 = 1e-3 of the
+elements; 2e-3 of them may differ, by one bf16 step of their own or, where terms cancel, by less than 2e-2.
+"""
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import w8a8_oracle as O  # noqa: E402
+from test_gpu_parity import device_weight, make_case, to_dev, to_np  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def S():
+    import skyrl_tx_rocm_b200 as S
+
+    return S
+
+
+def assert_one_step(got, want, what):
+    g32, w32 = got.astype(np.float32), want.astype(np.float32)
+    assert got.shape == want.shape and np.all(np.isfinite(g32)), what
+    assert O.relative_l2(g32, w32) < 1e-3, what
+    bound = np.maximum(2e-2, np.abs(w32) * 2.0 ** -7)
+    assert np.all(np.abs(g32 - w32) <= bound), f"{what}: {np.abs(g32 - w32).max()}"
+    frac = float((O.bf16_ulp_distance(got, want) > 0).mean())
+    assert frac <= 2e-3, f"{what}: {frac:.2e} of the elements differ"
+
+
+@pytest.mark.parametrize("m,k,n,g,rank,na", [
+    (1, 64, 32, 64, 8, 1),          # one row, one group, half a K block
+    (127, 384, 96, 96, 16, 40),     # groups that straddle K blocks; more adapters than a pass of the projection takes
+    (128, 512, 200, 32, 4, 2),      # groups of a single MMA step
+    (129, 1024, 4128, 64, 32, 5),   # a tile of one row; 128-wide column tiles with a remainder
+    (300, 768, 160, 256, 64, 33),   # groups of two K blocks, rank 64 over many adapters
+    (260, 512, 64, 512, 16, 3),     # one group over K
+])
+def test_grouped_scales_in_one_kernel(S, m, k, n, g, rank, na):
+    x, w, a, b, s, ids = make_case(31 + m, m, k, n, rank, na, w_std=0.05)
+    q = O.quantize_frozen_weight(w, group_size=g)
+    pw = S.PackedW8Weight(*_packed_grouped(S, q, k, n, g))
+    frozen = S.w8a8_frozen_linear(to_dev(x), pw, enabled=True)
+    np.testing.assert_array_equal(to_np(frozen).view(np.uint16), O.quantized_lora_linear(x, q).view(np.uint16))
+    lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=k, padded_out_features=pw.padded_out_features)
+    y = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids), enabled=True)
+    S.check_status()
+    assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), what=f"group {g}")
+
+
+def _packed_grouped(S, q, k, n, g):
+    """Packed form with group_size kept even where one group covers K (pack_weight would treat it as per-channel)."""
+    npad = (n + 31) // 32 * 32
+    codes = np.zeros((k, npad), dtype=np.int8)
+    codes[:, :n] = q.codes
+    p = S.pack_weight(S.GroupQuantizedWeight(to_dev(codes), to_dev(np.ones((1, npad), dtype=np.float32)), k, k, 8, k))
+    sw = torch.zeros((k // g, npad), dtype=torch.float32, device="cuda")
+    sw[:, :n] = torch.from_numpy(np.asarray(q.scales, dtype=np.float32))
+    return p.wq, sw, k, n, g
+
+
+@pytest.mark.parametrize("m,k,n,rank,na", [
+    (129, 512, 96, 16, 129),        # a tile with an adapter per row, and a tile of one row
+    (256, 1040, 320, 64, 32),       # rank 64: one adapter per pipeline slot, several rounds; K remainder
+    (385, 2048, 1056, 33, 20),      # rank between two widths
+    (1000, 256, 64, 8, 300),        # adapters that never occur
+])
+def test_tiles_of_many_adapters(S, m, k, n, rank, na):
+    x, w, a, b, s, ids = make_case(57 + m, m, k, n, rank, na, w_std=0.05)
+    q, pw = device_weight(S, w)
+    lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=pw.in_features,
+                       padded_out_features=pw.padded_out_features)
+    y = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids), enabled=True)
+    S.check_status()
+    assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), what=f"{na} adapters")
