@@ -100,6 +100,20 @@ class MlpArgs(C.Structure):
     ]
 
 
+class TrainArgs(C.Structure):
+    _fields_ = [
+        ("struct_size", C.c_uint32), ("m", C.c_int32), ("n", C.c_int32), ("k", C.c_int32), ("n_logical", C.c_int32),
+        ("rank", C.c_int32), ("num_adapters", C.c_int32), ("flags", C.c_uint32),
+        ("x", C.c_void_p), ("x_row_stride", C.c_int64), ("dy", C.c_void_p), ("dy_row_stride", C.c_int64),
+        ("wq", C.c_void_p), ("sw", C.c_void_p), ("lora_a", C.c_void_p), ("lora_b", C.c_void_p),
+        ("lora_scaling", C.c_void_p), ("adapter_ids", C.c_void_p), ("bwd_a", C.c_void_p), ("bwd_b", C.c_void_p),
+        ("bwd_a_rows", C.c_int32), ("bwd_a_cols", C.c_int32), ("bwd_b_slots", C.c_int32), ("reserved", C.c_int32),
+        ("y", C.c_void_p), ("dx", C.c_void_p), ("da", C.c_void_p), ("db", C.c_void_p),
+        ("saved", C.c_void_p), ("saved_bytes", C.c_size_t), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
+        ("status", C.c_void_p),
+    ]
+
+
 class TpExchangeArgs(C.Structure):
     _fields_ = [
         ("struct_size", C.c_uint32), ("tp", C.c_int32), ("row_begin", C.c_int32), ("row_count", C.c_int32),
@@ -131,6 +145,10 @@ SYMBOLS = {
     "skyrl_w8a8_lora_forward_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "skyrl_w8a8_grouped_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "skyrl_w8a8_lora_forward_grouped_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_int32, C.c_void_p]),
+    "skyrl_w8a8_train_saved_bytes": (C.c_size_t, [C.c_int32, C.c_int32]),
+    "skyrl_w8a8_train_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "skyrl_w8a8_train_forward_sm100_v1": (C.c_int, [C.POINTER(TrainArgs), C.c_void_p]),
+    "skyrl_w8a8_train_backward_sm100_v1": (C.c_int, [C.POINTER(TrainArgs), C.c_void_p]),
     "skyrl_w8a8_lora_forward_noalloc_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "skyrl_rms_gate_up_w8a8_lora_swiglu_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "skyrl_down_w8a8_lora_residual_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),

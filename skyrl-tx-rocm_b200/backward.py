@@ -8,14 +8,17 @@ skyrl/tx/kernels/quantized_lora.py:337-394):
     dx = dy @ deq(W)^T + R @ A^T          (dominant: an [M, N] x [N, K] contraction)
     dA = x^T @ R,   dB = s * (x @ A)^T @ dy,   ds = sum(dy * ((x @ A) @ B))
 
-Here the dominant contraction runs on the same tcgen05 int8 kernels as the forward: the weight's
+Here the dominant contraction runs on the same tcgen05 int8 path as the forward: the weight's
 per-output-channel scale moves to the cotangent, g = dy * sw, each row of g is split into two int8 planes
-(`skyrl_w8a8_grad_quant_sm100_v1`), and the GEMM runs once per plane over a TRANSPOSED packed copy of the
-codes (unit weight scales) into fp32 slabs.  dx therefore equals the fp32 product to about 2^-15 relative
-(two planes) — far inside bf16's own rounding — at the cost of one bf16 GEMM, and `R @ A^T` rides the LoRA
-slice of the last plane's launch exactly as `s (x A) B` does in the forward.  The rank-r reductions dA, dB and
-ds are two orders of magnitude smaller and use library matmuls over the adapter-sorted rows (bf16 tensor-core
-products with fp32 results; the small fp32 factors are split into two bf16 terms).
+(`skyrl_w8a8_grad_quant_sm100_v1`), and one GEMM over a TRANSPOSED packed copy of the codes multiplies both planes
+with every weight tile it loads.  dx therefore equals the fp32 product to about 2^-15 relative (two planes), far
+inside bf16's own rounding, at the cost of one bf16 GEMM, and `R @ A^T` rides the same launch as `s (x A) B` does in
+the forward.  dA and dB contract x and dy with the two LoRA projections (the forward's, which it keeps, and the
+cotangent's, which dx needs anyway) in one launch over the adapters' row ranges.
+
+A training step takes the LoRA tables in the reference's layout, [A, K, r] and [A, r, N]: they change at every
+optimizer step, so the forward lays them out for its kernels in one launch and the backward, whose operator is the
+transposed one, reads them as they are.
 
 `W8A8LoRALinearFunction` ties forward and backward together for `torch.autograd`, the counterpart of the
 reference's `quantized_lora_linear.defvjp(...)` (quantized_lora.py:397).
@@ -29,7 +32,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib, ops
-from .ops import EPI_PARTIAL_F32, LORA_RANK_PAD, Z_PARTS, PackedLoRA, PackedW8Weight
+from .ops import EPI_LINEAR, LORA_RANK_PAD, Z_PARTS, PackedLoRA, PackedW8Weight
 
 
 @dataclass(frozen=True)
@@ -83,17 +86,31 @@ def w8a8_lora_linear_input_grad(dy: torch.Tensor, weight_bwd: PackedW8Backward, 
     na = lora_bwd.num_adapters if lora_bwd is not None else 1
     ids = ops._check_ids(adapter_ids, m, lora_bwd)
     st = ops._status_word(dev)
+    if planes == 2:
+        a = _train_args(m, npad, k, n_logical, lora_bwd.rank if lora_bwd is not None else 0, na, st)
+        a.dy, a.dy_row_stride = dy2.data_ptr(), dy2.stride(0)
+        a.wq, a.sw = wt.wq.data_ptr(), weight_bwd.col_scale.data_ptr()
+        if lora_bwd is not None:
+            table = lora_bwd.b_rows if lora_bwd.b_rows is not None else lora_bwd.b
+            a.lora_scaling = lora_bwd.scaling.data_ptr()
+            a.bwd_a, a.bwd_a_rows, a.bwd_a_cols = lora_bwd.a.data_ptr(), lora_bwd.a.shape[1], lora_bwd.a.shape[2]
+            a.bwd_b, a.bwd_b_slots = table.data_ptr(), table.shape[2]
+        a.adapter_ids = ids.data_ptr() if ids is not None else None
+        dx = torch.empty((m, k), dtype=torch.bfloat16, device=dev)
+        a.dx = dx.data_ptr()
+        _with_workspace(a, dev, True)
+        _lib.check(lib.skyrl_w8a8_train_backward_sm100_v1(C.byref(a), ops._stream()), "train_backward (input gradient)")
+        return dx.reshape(*dy.shape[:-1], k)
+    # one plane: the int8 step of the cotangent stays visible in dx; same kernels as the forward
     perm, tiles, num = ops.prepare_routing(ids, m, na)
     row_map = perm if ids is not None else None
     max_tiles = tiles.shape[0]
 
-    q = torch.empty((planes, m, npad), dtype=torch.int8, device=dev)
-    s = torch.empty((planes, m), dtype=torch.float32, device=dev)
-    second = planes == 2
+    q = torch.empty((m, npad), dtype=torch.int8, device=dev)
+    s = torch.empty((m,), dtype=torch.float32, device=dev)
     _lib.check(lib.skyrl_w8a8_grad_quant_sm100_v1(
-        ops._ptr(dy2), dy2.stride(0), ops._ptr(weight_bwd.col_scale), ops._ptr(row_map), m, npad, ops._ptr(q[0]),
-        ops._ptr(s[0]), ops._ptr(q[1]) if second else None, ops._ptr(s[1]) if second else None, ops._stream()),
-        "grad_quant")
+        ops._ptr(dy2), dy2.stride(0), ops._ptr(weight_bwd.col_scale), ops._ptr(row_map), m, npad, ops._ptr(q), ops._ptr(s),
+        None, None, ops._stream()), "grad_quant")
 
     z_parts = None
     if lora_bwd is not None:
@@ -106,28 +123,38 @@ def w8a8_lora_linear_input_grad(dy: torch.Tensor, weight_bwd: PackedW8Backward, 
                                                   na, lora_bwd.rank, ops._ptr(tiles), ops._ptr(num), max_tiles,
                                                   ops._ptr(z_parts), ops._ptr(st), ops._stream()), "lora_a_proj (backward)")
 
-    slabs = torch.empty((planes, m, k), dtype=torch.float32, device=dev)
-    for p in range(planes):
-        a = _lib.GemmArgs()
-        a.struct_size = C.sizeof(_lib.GemmArgs)
-        a.epilogue = EPI_PARTIAL_F32
-        a.m, a.n, a.k = m, k, npad
-        a.xq, a.sx, a.sw = q[p].data_ptr(), s[p].data_ptr(), wt.sw.data_ptr()
-        a.wq = wt.wq.data_ptr()
-        last = p == planes - 1
-        a.rank = lora_bwd.rank if (lora_bwd is not None and last) else 0
-        a.num_adapters = na
-        a.max_tiles = max_tiles
-        if a.rank:
-            a.z_parts, a.lora_b_packed = z_parts.data_ptr(), lora_bwd.b.data_ptr()
-        a.tiles, a.num_tiles = tiles.data_ptr(), num.data_ptr()
-        a.out, a.out_row_stride = slabs[p].data_ptr(), k
-        a.status = st.data_ptr()
-        _lib.check(lib.skyrl_w8a8_gemm_sm100_v1(C.byref(a), ops._stream()), "w8a8_gemm (input gradient)")
     dx = torch.empty((m, k), dtype=torch.bfloat16, device=dev)
-    _lib.check(lib.skyrl_group_sum_cast_sm100_v1(ops._ptr(slabs), planes, m, k, ops._ptr(row_map), ops._ptr(dx), k,
-                                                 ops._stream()), "group_sum_cast (input gradient)")
+    a = _lib.GemmArgs()
+    a.struct_size = C.sizeof(_lib.GemmArgs)
+    a.epilogue = EPI_LINEAR
+    a.m, a.n, a.k = m, k, npad
+    a.xq, a.sx, a.sw = q.data_ptr(), s.data_ptr(), wt.sw.data_ptr()
+    a.wq = wt.wq.data_ptr()
+    a.rank = lora_bwd.rank if lora_bwd is not None else 0
+    a.num_adapters = na
+    a.max_tiles = max_tiles
+    if a.rank:
+        a.z_parts, a.lora_b_packed = z_parts.data_ptr(), lora_bwd.b.data_ptr()
+    a.tiles, a.num_tiles = tiles.data_ptr(), num.data_ptr()
+    a.out_row_map = row_map.data_ptr() if row_map is not None else None
+    a.out, a.out_row_stride = dx.data_ptr(), k
+    a.status = st.data_ptr()
+    _lib.check(lib.skyrl_w8a8_gemm_sm100_v1(C.byref(a), ops._stream()), "w8a8_gemm (input gradient)")
     return dx.reshape(*dy.shape[:-1], k)
+
+
+def _train_args(m: int, n: int, k: int, n_logical: int, rank: int, adapters: int, status: torch.Tensor):
+    a = _lib.TrainArgs()
+    a.struct_size = C.sizeof(_lib.TrainArgs)
+    a.m, a.n, a.k, a.n_logical, a.rank, a.num_adapters = m, n, k, n_logical, rank, adapters
+    a.status = status.data_ptr()
+    return a
+
+
+def _with_workspace(a, device, backward: bool) -> None:
+    nbytes = _lib.load().skyrl_w8a8_train_workspace_bytes(a.m, a.n, a.k, a.rank, a.num_adapters, backward)
+    ws = ops._workspace(device, nbytes)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
 
 
 def _mm_f32(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
@@ -203,21 +230,99 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, lora_a, lora_b, lora_scaling, weight, weight_bwd, adapter_ids):
-        ctx.save_for_backward(x, lora_a, lora_b, lora_scaling, adapter_ids if adapter_ids is not None else torch.empty(0))
+        w = ops._weight_of(weight)
+        if w.group_size:
+            raise ops.SkyrlKernelError("the backward path takes per-output-channel scales (one group over K)")
+        k, npad, n = w.in_features, w.padded_out_features, w.out_features
+        x2 = ops._pad_cols(ops._check_x(x, weight_bwd.in_features), k)
+        m, dev = x2.shape[0], x2.device
+        a3, b3, scaling = _tables(lora_a, lora_b, lora_scaling, k, n)
+        na, _, rank = a3.shape
+        if adapter_ids is None and na != 1:
+            raise ValueError("adapter_ids is required when the LoRA tables hold more than one adapter")
+        ids = ops._check_ids(adapter_ids, m, None)
+        lib = _lib.load()
+        saved = torch.empty(lib.skyrl_w8a8_train_saved_bytes(m, na) + 1024, dtype=torch.uint8, device=dev)
+        y = torch.empty((m, npad), dtype=torch.bfloat16, device=dev)
+        a = _train_args(m, npad, k, n, rank, na, ops._status_word(dev))
+        a.x, a.x_row_stride = x2.data_ptr(), x2.stride(0)
+        a.wq, a.sw = w.wq.data_ptr(), w.sw.data_ptr()
+        a.lora_a, a.lora_b, a.lora_scaling = a3.data_ptr(), b3.data_ptr(), scaling.data_ptr()
+        a.adapter_ids = ids.data_ptr() if ids is not None else None
+        a.y = y.data_ptr()
+        _with_saved(a, saved)
+        _with_workspace(a, dev, False)
+        _lib.check(lib.skyrl_w8a8_train_forward_sm100_v1(C.byref(a), ops._stream()), "train_forward")
+        ctx.save_for_backward(x, lora_a, lora_b, lora_scaling, ids, saved)
         ctx.weight_bwd = weight_bwd
-        ctx.has_ids = adapter_ids is not None
-        return ops.w8a8_lora_linear(x, weight, lora_a, lora_b, lora_scaling, adapter_ids, enabled=True)
+        return y[:, :n].reshape(*x.shape[:-1], n)
 
     @staticmethod
     def backward(ctx, dy):
-        x, lora_a, lora_b, lora_scaling, ids = ctx.saved_tensors
-        ids = ids if ctx.has_ids else None
-        dy = dy.contiguous()
-        lora_bwd = pack_lora_backward(lora_a.detach(), lora_b.detach(), lora_scaling.detach(), ctx.weight_bwd)
-        dx = w8a8_lora_linear_input_grad(dy, ctx.weight_bwd, lora_bwd, ids, enabled=True) if ctx.needs_input_grad[0] else None
-        d_a, d_b, d_s = lora_parameter_grads(x.detach(), dy, lora_a.detach(), lora_b.detach(), lora_scaling.detach(), ids)
-        return (dx, d_a.to(lora_a.dtype), d_b.to(lora_b.dtype), d_s.reshape(lora_scaling.shape).to(lora_scaling.dtype),
+        x, lora_a, lora_b, lora_scaling, ids, saved = ctx.saved_tensors
+        wb = ctx.weight_bwd
+        k, n, npad = wb.in_features, wb.out_features, wb.wq_t.in_features
+        x2 = ops._pad_cols(x.reshape(-1, x.shape[-1]), k)
+        dy2 = ops._pad_cols(ops._check_x(dy, n), npad)
+        m, dev = dy2.shape[0], dy2.device
+        a3, b3, scaling = _tables(lora_a, lora_b, lora_scaling, k, n)
+        na, _, rank = a3.shape
+        # the transposed operator's tables are B and A themselves, padded where a row is no multiple of 16 bytes
+        table_b = a3 if rank % 8 == 0 else torch.nn.functional.pad(a3, (0, -rank % 8))
+        table_a = b3 if n % 8 == 0 else torch.nn.functional.pad(b3, (0, -n % 8))
+        d_a = torch.empty((na, k, rank), dtype=torch.bfloat16, device=dev)
+        d_b = torch.empty((na, rank, n), dtype=torch.bfloat16, device=dev)
+        dx = torch.empty((m, k), dtype=torch.bfloat16, device=dev) if ctx.needs_input_grad[0] else None
+        a = _train_args(m, npad, k, n, rank, na, ops._status_word(dev))
+        a.x, a.x_row_stride = x2.data_ptr(), x2.stride(0)
+        a.dy, a.dy_row_stride = dy2.data_ptr(), dy2.stride(0)
+        a.wq, a.sw = wb.wq_t.wq.data_ptr(), wb.col_scale.data_ptr()
+        a.lora_scaling = scaling.data_ptr()
+        a.adapter_ids = ids.data_ptr() if ids is not None else None
+        a.bwd_a, a.bwd_a_rows, a.bwd_a_cols = table_a.data_ptr(), rank, table_a.shape[2]
+        a.bwd_b, a.bwd_b_slots = table_b.data_ptr(), table_b.shape[2]
+        a.dx = dx.data_ptr() if dx is not None else None
+        a.da, a.db = d_a.data_ptr(), d_b.data_ptr()
+        _with_saved(a, saved)
+        _with_workspace(a, dev, True)
+        _lib.check(_lib.load().skyrl_w8a8_train_backward_sm100_v1(C.byref(a), ops._stream()), "train_backward")
+        d_s = None
+        if ctx.needs_input_grad[3]:   # rarely wanted (alpha / r is a constant): library matmuls
+            d_s = lora_parameter_grads(x.detach(), dy.contiguous(), lora_a.detach(), lora_b.detach(), lora_scaling.detach(), ids)[2]
+            d_s = d_s.reshape(lora_scaling.shape).to(lora_scaling.dtype)
+        return (dx.reshape(x.shape) if dx is not None else None, d_a.reshape(lora_a.shape), d_b.reshape(lora_b.shape), d_s,
                 None, None, None)
+
+
+def _tables(lora_a, lora_b, lora_scaling, k: int, n: int):
+    """LoRA tables in the reference's layout (one adapter as matrices, or a stack) as contiguous [A, K, r], [A, r, N], [A]."""
+    ops._require_cuda(lora_a, "lora_a")
+    ops._require_cuda(lora_b, "lora_b")
+    if lora_a.dtype != torch.bfloat16 or lora_b.dtype != torch.bfloat16:
+        raise TypeError("LoRA A and B must both be BF16")
+    if lora_a.ndim == 2 and lora_b.ndim == 2:
+        lora_a, lora_b = lora_a[None], lora_b[None]
+    if lora_a.ndim != 3 or lora_b.ndim != 3:
+        raise ValueError("lora_a and lora_b must both be rank-two or both rank-three")
+    na, ka, r = lora_a.shape
+    if lora_b.shape[:2] != (na, r):
+        raise ValueError(f"incompatible LoRA shapes: A={tuple(lora_a.shape)}, B={tuple(lora_b.shape)}")
+    if ka != k or lora_b.shape[2] != n:
+        raise ValueError(f"LoRA tables of {ka} and {lora_b.shape[2]} features do not match the weight's {k} and {n}")
+    if r > ops.MAX_LORA_RANK:
+        raise ValueError(f"LoRA rank must not exceed {ops.MAX_LORA_RANK}, got {r}")
+    scaling = lora_scaling.detach().reshape(-1)
+    if scaling.dtype != torch.float32 or not scaling.is_cuda:
+        scaling = scaling.to(device=lora_a.device, dtype=torch.float32)
+    if scaling.numel() != na:
+        raise ValueError(f"lora_scaling must have {na} entries, got {scaling.numel()}")
+    return lora_a.detach().contiguous(), lora_b.detach().contiguous(), scaling.contiguous()
+
+
+def _with_saved(a, saved: torch.Tensor) -> None:
+    base = saved.data_ptr()
+    off = -base % 1024
+    a.saved, a.saved_bytes = base + off, saved.numel() - off
 
 
 def w8a8_lora_linear_trainable(x, weight, weight_bwd: PackedW8Backward, lora_a, lora_b, lora_scaling, adapter_ids=None):

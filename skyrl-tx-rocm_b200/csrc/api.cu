@@ -587,6 +587,215 @@ extern "C" int skyrl_w8a8_lora_forward_grouped_sm100_v1(const SkyrlW8A8LinearArg
   return launch_grouped_gemm(g, stream);
 }
 
+// ---- training step -----------------------------------------------------------------
+namespace skyrl {
+
+struct TrainSaved {
+  RouteWs route;
+  int32_t* adapter_start;  // [A + 1]
+  uint16_t* z_parts;       // s (x A) of the sorted rows
+  size_t bytes;
+};
+static TrainSaved carve_train_saved(void* base, int m, int num_adapters) {
+  Carver c(base);
+  TrainSaved s;
+  s.route = carve_route(c, m, num_adapters);
+  s.adapter_start = c.take<int32_t>(num_adapters + 1);
+  s.z_parts = c.take<uint16_t>(SKYRL_Z_PARTS * static_cast<size_t>(m) * SKYRL_LORA_RANK_PAD);
+  s.bytes = c.total();
+  return s;
+}
+
+struct TrainWs {
+  int32_t* sched;
+  int8_t* xq;        // forward
+  float* sx;
+  uint16_t* rows;    // gathered rows of x (forward) or dy (backward)
+  uint16_t* at;      // forward: tables in kernel layout
+  uint16_t* bt;
+  int8_t* q;         // backward: two planes
+  float* s;
+  uint16_t* zb;
+  TrainSaved own;    // backward without `saved`
+  size_t bytes;
+};
+static TrainWs carve_train(void* ws, int m, int n, int k, int rank, int num_adapters, bool backward) {
+  Carver c(ws);
+  TrainWs w = {};
+  const size_t mm = static_cast<size_t>(m);
+  w.sched = c.take<int32_t>(SCHED_WORDS);
+  if (!backward) {
+    w.xq = c.take<int8_t>(mm * k);
+    w.sx = c.take<float>(mm);
+    w.rows = c.take<uint16_t>(mm * k);
+    w.at = c.take<uint16_t>(static_cast<size_t>(num_adapters) * rank * k);
+    w.bt = c.take<uint16_t>(static_cast<size_t>(num_adapters) * n * ((rank + 7) / 8 * 8));
+  } else {
+    w.q = c.take<int8_t>(2 * mm * n);
+    w.s = c.take<float>(2 * mm);
+    w.rows = c.take<uint16_t>(mm * n);
+    w.zb = c.take<uint16_t>(SKYRL_Z_PARTS * mm * SKYRL_LORA_RANK_PAD);
+    c.off = align_up(c.off, 1024);
+    w.own = carve_train_saved(c.base != nullptr ? c.base + c.off : nullptr, m, num_adapters);
+    c.off += w.own.bytes;
+  }
+  w.bytes = c.total();
+  return w;
+}
+
+static int check_train(const SkyrlW8A8TrainArgs* a, const char* who) {
+  if (a == nullptr) return fail(SKYRL_ERR_INVALID_ARGUMENT, "%s: args is null", who);
+  if (a->struct_size != sizeof(SkyrlW8A8TrainArgs))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "%s: struct_size %u does not match ABI v%d (%zu)", who, a->struct_size,
+                SKYRL_W8A8_ABI_VERSION, sizeof(SkyrlW8A8TrainArgs));
+  if (a->m <= 0 || a->n <= 0 || a->k <= 0 || a->n % 32 != 0 || a->k % 16 != 0 || a->n_logical <= 0 || a->n_logical > a->n)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "%s: bad shape", who);
+  if (a->wq == nullptr || a->sw == nullptr || a->status == nullptr)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "%s: null buffer", who);
+  if (a->rank < 0 || a->rank > SKYRL_LORA_RANK_PAD)
+    return fail(SKYRL_ERR_UNSUPPORTED, "%s: LoRA rank must be in [0, %d], got %d", who, SKYRL_LORA_RANK_PAD, a->rank);
+  return SKYRL_OK;
+}
+
+}  // namespace skyrl
+
+extern "C" size_t skyrl_w8a8_train_saved_bytes(int32_t m, int32_t num_adapters) {
+  if (m <= 0) return 0;
+  return carve_train_saved(nullptr, m, num_adapters > 0 ? num_adapters : 1).bytes;
+}
+
+extern "C" size_t skyrl_w8a8_train_workspace_bytes(int32_t m, int32_t n, int32_t k, int32_t rank, int32_t num_adapters,
+                                                    int32_t backward) {
+  if (m <= 0 || n <= 0 || k <= 0 || rank < 0) return 0;
+  return carve_train(nullptr, m, n, k, rank, num_adapters > 0 ? num_adapters : 1, backward != 0).bytes;
+}
+
+extern "C" int skyrl_w8a8_train_forward_sm100_v1(const SkyrlW8A8TrainArgs* a, skyrl_stream_t stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  int rc = check_train(a, "train_forward");
+  if (rc) return rc;
+  if (a->x == nullptr || a->y == nullptr || a->rank <= 0 || a->lora_a == nullptr || a->lora_b == nullptr ||
+      a->lora_scaling == nullptr || a->num_adapters <= 0)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "train_forward: null buffer or LoRA tables missing");
+  const int na = a->num_adapters;
+  const TrainSaved sv = carve_train_saved(a->saved, a->m, na);
+  const TrainWs w = carve_train(a->workspace, a->m, a->n, a->k, a->rank, na, false);
+  if ((rc = check_ws(a->saved, a->saved_bytes, sv.bytes, "train_forward (saved)"))) return rc;
+  if ((rc = check_ws(a->workspace, a->workspace_bytes, w.bytes, "train_forward"))) return rc;
+  const bool routed = a->adapter_ids != nullptr;
+  if ((rc = launch_train_tables(a->lora_a, a->lora_b, na, a->k, a->n_logical, a->n, a->rank, w.at, w.bt, stream))) return rc;
+  if (routed && (rc = launch_route_dense(a->adapter_ids, a->m, na, sv.route.perm, sv.route.tiles, sv.route.seg_mask,
+                                         sv.route.seg_adapter, a->status, stream, nullptr, 0, true, sv.adapter_start)))
+    return rc;
+  const int32_t* perm = routed ? sv.route.perm : nullptr;
+  const bool copy = routed || a->x_row_stride != a->k;
+  if ((rc = launch_rms_quant(a->x, a->x_row_stride, nullptr, 0.f, perm, a->m, a->k, w.xq, w.sx, copy ? w.rows : nullptr,
+                             stream, nullptr, w.sched)))
+    return rc;
+  const TileSource src = tile_source(sv.route, routed, 0, a->m);
+  if ((rc = launch_lora_a_proj(copy ? static_cast<const void*>(w.rows) : a->x, a->m, a->k, w.at, a->lora_scaling, na,
+                               a->rank, src, src.count, sv.z_parts, a->status, stream, 0, -1, nullptr, 0, -1, a->rank)))
+    return rc;
+  SkyrlW8A8GemmArgs g = {};
+  g.struct_size = sizeof(g);
+  g.epilogue = SKYRL_EPI_LINEAR;
+  g.m = a->m;
+  g.n = a->n;
+  g.k = a->k;
+  g.rank = a->rank;
+  g.num_adapters = na;
+  g.xq = w.xq;
+  g.sx = w.sx;
+  g.wq = a->wq;
+  g.sw = a->sw;
+  g.z_parts = sv.z_parts;
+  g.lora_b_packed = w.bt;
+  g.lora_b_rows = w.bt;
+  g.lora_b_rows_rank = (a->rank + 7) / 8 * 8;
+  g.out_row_map = perm;
+  g.out = a->y;
+  g.out_row_stride = a->n;
+  g.status = a->status;
+  g.sched = w.sched;
+  return launch_gemm(g, stream, true, &src);
+}
+
+extern "C" int skyrl_w8a8_train_backward_sm100_v1(const SkyrlW8A8TrainArgs* a, skyrl_stream_t stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  int rc = check_train(a, "train_backward");
+  if (rc) return rc;
+  const bool grads = a->saved != nullptr;
+  const bool lora = a->rank > 0;
+  if (a->dy == nullptr || (a->dx == nullptr && !grads) ||
+      (grads && (a->x == nullptr || a->da == nullptr || a->db == nullptr || !lora)))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "train_backward: null buffer");
+  if (lora && (a->bwd_a == nullptr || a->bwd_b == nullptr || a->lora_scaling == nullptr || a->num_adapters <= 0))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "train_backward: LoRA tables missing");
+  const int na = a->num_adapters > 0 ? a->num_adapters : 1;
+  const TrainWs w = carve_train(a->workspace, a->m, a->n, a->k, a->rank, na, true);
+  if ((rc = check_ws(a->workspace, a->workspace_bytes, w.bytes, "train_backward"))) return rc;
+  TrainSaved sv = w.own;
+  const bool routed = lora && a->adapter_ids != nullptr;
+  if (grads) {
+    sv = carve_train_saved(a->saved, a->m, na);
+    if ((rc = check_ws(a->saved, a->saved_bytes, sv.bytes, "train_backward (saved)"))) return rc;
+  } else if (routed && (rc = launch_route_dense(a->adapter_ids, a->m, na, sv.route.perm, sv.route.tiles, sv.route.seg_mask,
+                                                sv.route.seg_adapter, a->status, stream, nullptr, 0, true, sv.adapter_start))) {
+    return rc;
+  }
+  const int32_t* perm = routed ? sv.route.perm : nullptr;
+  const TileSource src = tile_source(sv.route, routed, 0, a->m);
+  const bool copy = lora && (routed || a->dy_row_stride != a->n);
+  const size_t plane = static_cast<size_t>(a->m) * a->n;
+  if ((rc = launch_grad_quant(a->dy, a->dy_row_stride, a->sw, perm, a->m, a->n, w.q, w.s, w.q + plane, w.s + a->m, stream,
+                              copy ? w.rows : nullptr)))
+    return rc;
+  if (lora && (rc = launch_lora_a_proj(copy ? static_cast<const void*>(w.rows) : a->dy, a->m, a->n, a->bwd_a, a->lora_scaling,
+                                       na, a->rank, src, src.count, w.zb, a->status, stream, 0, -1, nullptr, 0, -1,
+                                       a->bwd_a_rows, a->bwd_a_cols)))
+    return rc;
+  if (a->dx != nullptr) {
+    PlanesGemmLaunch g = {};
+    g.m = a->m;
+    g.n = a->k;
+    g.k = a->n;
+    g.rank = a->rank;
+    g.num_adapters = na;
+    g.src = src;
+    g.q = w.q;
+    g.s = w.s;
+    g.wq = a->wq;
+    g.z_parts = w.zb;
+    g.b_table = a->bwd_b;
+    g.b_slots = a->bwd_b_slots;
+    g.out_row_map = perm;
+    g.out = a->dx;
+    g.out_stride = a->k;
+    g.status = a->status;
+    if ((rc = launch_planes_gemm(g, stream))) return rc;
+  }
+  if (!grads) return SKYRL_OK;
+  LoraGradLaunch q = {};
+  q.m = a->m;
+  q.k = a->k;
+  q.n = a->n;
+  q.n_logical = a->n_logical;
+  q.adapters = na;
+  q.rank = a->rank;
+  q.x = a->x;
+  q.x_stride = a->x_row_stride;
+  q.dy = a->dy;
+  q.dy_stride = a->dy_row_stride;
+  q.z = sv.z_parts;
+  q.zb = w.zb;
+  q.perm = perm;
+  q.adapter_start = routed ? sv.adapter_start : nullptr;
+  q.da = a->da;
+  q.db = a->db;
+  q.status = a->status;
+  return launch_lora_grad(q, stream);
+}
+
 // One exported target per fused variant: thin wrappers that check what the variant needs and fix the epilogue.
 extern "C" int skyrl_rms_gate_up_w8a8_lora_swiglu_sm100_v1(const SkyrlW8A8LinearArgs* a, skyrl_stream_t stream) {
   if (a == nullptr) return fail(SKYRL_ERR_INVALID_ARGUMENT, "rms_gate_up_swiglu: args is null");

@@ -44,6 +44,26 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   cfg.numAttrs = programmatic ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+// The same with a cluster of `cluster` CTAs along x, always programmatic (the kernels wait before they read).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_cluster_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                         int cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 // The opt-in to more than 48 KB of dynamic shared memory is an attribute of the function PER DEVICE
 // (a single process may drive several GPUs, as an XLA host does): `done` is the caller's
 // function-local `static bool[MAX_DEVICES]`, indexed by the current device.  A benign race only
@@ -68,9 +88,11 @@ int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int
                  int max_tiles, int32_t* status, cudaStream_t stream, int chunk_rows = 0, int chunk_cap = 0,
                  int32_t* zero_words = nullptr, int zero_count = 0);
 int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* seg_mask,
-                       int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count);
+                       int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count,
+                       bool always_sort = false, int32_t* adapter_start = nullptr);
+// `always_sort`: sorted rows also within one tile; `adapter_start` int32 [adapters + 1]: first sorted row of each adapter
 int launch_grad_quant(const void* dy, int64_t dy_row_stride, const float* col_scale, const int32_t* row_map, int m, int n,
-                      void* q1, float* s1, void* q2, float* s2, cudaStream_t stream);
+                      void* q1, float* s1, void* q2, float* s2, cudaStream_t stream, void* rows = nullptr);  // rows: gathered dy
 constexpr int ZERO_WORDS = 8;  // scheduler words of a workspace: {claimed, finished} of up to four GEMM launches
 int launch_rms_quant(const void* x, int64_t x_row_stride, const void* rms_delta, float eps, const int32_t* row_map,
                      int m, int k, void* xq, float* sx, void* xn, cudaStream_t stream, float* zero_amax = nullptr,
@@ -80,7 +102,8 @@ int launch_quant_stream(const void* x, const float* row_amax, int m, int k, void
 int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const float* scaling, int num_adapters,
                        int rank, const TileSource& src, int max_tiles, void* z_parts, int32_t* status,
                        cudaStream_t stream, int row_lo = 0, int row_hi = -1, void* const* extra_dests = nullptr,
-                       int extra_count = 0, int list_row0 = -1);  // extra copies of the rows written
+                       int extra_count = 0, int list_row0 = -1,  // extra copies of the rows written
+                       int table_rows = SKYRL_LORA_RANK_PAD, int table_k = 0);  // rows and columns of a table (0: k)
 // Tile width and K split the GEMM launcher chooses for a shape (deterministic per device).
 struct GemmPlan {
   int bn_eff;
@@ -120,6 +143,40 @@ struct GroupedGemmLaunch {
   int32_t* status;
 };
 int launch_grouped_gemm(const GroupedGemmLaunch& a, cudaStream_t stream);
+// Input gradient over both int8 planes of the cotangent (planes_gemm_sm100.cu).
+struct PlanesGemmLaunch {
+  int m, n, k, rank, num_adapters;
+  TileSource src;
+  const void* q;        // int8 [2, m, k]
+  const float* s;       // [2, m]
+  const void* wq;
+  const void* z_parts;
+  const void* b_table;  // bf16 [A, n, b_slots]
+  int b_slots;
+  const int32_t* out_row_map;
+  void* out;
+  int64_t out_stride;
+  int32_t* status;
+};
+int launch_planes_gemm(const PlanesGemmLaunch& a, cudaStream_t stream);
+// Gradients of the LoRA tables, and the layouts of new tables (lora_grad_sm100.cu).
+struct LoraGradLaunch {
+  int m, k, n, n_logical, adapters, rank;
+  const void* x;
+  int64_t x_stride;
+  const void* dy;
+  int64_t dy_stride;
+  const void* z;        // parts of s (x A), sorted rows
+  const void* zb;       // parts of s (dy B^T), sorted rows
+  const int32_t* perm;
+  const int32_t* adapter_start;
+  void* da;             // bf16 [A, k, rank]
+  void* db;             // bf16 [A, rank, n_logical]
+  int32_t* status;
+};
+int launch_lora_grad(const LoraGradLaunch& a, cudaStream_t stream);
+int launch_train_tables(const void* a, const void* b, int adapters, int k, int n, int n_pad, int rank, void* at, void* bt,
+                        cudaStream_t stream);
 int launch_tp_finalize(const float* reduced, const int32_t* perm, const void* residual, void* out, int hidden,
                        int row_begin, int row_count, cudaStream_t stream, bool out_sorted = false);
 int launch_tp_finalize_slabs(const float* const* slabs, int num_slabs, const int32_t* perm, const void* residual,

@@ -19,11 +19,13 @@ namespace {
 __global__ void __launch_bounds__(QUANT_THREADS)
 grad_quant_kernel(const __nv_bfloat16* __restrict__ dy, int64_t dy_row_stride, const float* __restrict__ col_scale,
                   const int32_t* __restrict__ row_map, int n, int8_t* __restrict__ q1, float* __restrict__ s1,
-                  int8_t* __restrict__ q2, float* __restrict__ s2) {
+                  int8_t* __restrict__ q2, float* __restrict__ s2, uint4* __restrict__ rows) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float4* g = reinterpret_cast<float4*>(smem_raw);  // n / 4 vectors
   __shared__ float red[QUANT_THREADS / 32];
 
+  pdl_wait();
+  pdl_trigger();
   const int out_row = blockIdx.x;
   const int64_t src_row = row_map != nullptr ? row_map[out_row] : out_row;
   const uint4* src = reinterpret_cast<const uint4*>(dy + src_row * dy_row_stride);
@@ -33,6 +35,7 @@ grad_quant_kernel(const __nv_bfloat16* __restrict__ dy, int64_t dy_row_stride, c
   float amax = 0.f;
   for (int v = threadIdx.x; v < nvec; v += QUANT_THREADS) {
     const uint4 u = __ldg(src + v);
+    if (rows != nullptr) rows[static_cast<int64_t>(out_row) * nvec + v] = u;  // for the LoRA projection of the sorted rows
     const float4 c0 = __ldg(cs + 2 * v), c1 = __ldg(cs + 2 * v + 1);
     float4 a, b;
     a.x = __fmul_rn(bf16_lo(u.x), c0.x);
@@ -92,7 +95,7 @@ grad_quant_kernel(const __nv_bfloat16* __restrict__ dy, int64_t dy_row_stride, c
 }  // namespace
 
 int launch_grad_quant(const void* dy, int64_t dy_row_stride, const float* col_scale, const int32_t* row_map, int m, int n,
-                      void* q1, float* s1, void* q2, float* s2, cudaStream_t stream) {
+                      void* q1, float* s1, void* q2, float* s2, cudaStream_t stream, void* rows) {
   if (dy == nullptr || col_scale == nullptr || q1 == nullptr || s1 == nullptr || m <= 0 || n <= 0)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "grad_quant: null buffer or non-positive shape");
   if ((q2 == nullptr) != (s2 == nullptr))
@@ -107,10 +110,10 @@ int launch_grad_quant(const void* dy, int64_t dy_row_stride, const float* col_sc
   static bool attr_set[MAX_DEVICES] = {};
   cudaError_t e = ensure_dynamic_smem(grad_quant_kernel, 200 * 1024, attr_set);
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "grad_quant attribute: %s", cudaGetErrorString(e));
-  grad_quant_kernel<<<m, QUANT_THREADS, smem, stream>>>(static_cast<const __nv_bfloat16*>(dy), dy_row_stride, col_scale,
-                                                        row_map, n, static_cast<int8_t*>(q1), s1,
-                                                        static_cast<int8_t*>(q2), s2);
-  e = cudaPeekAtLastError();
+  e = launch_kernel(grad_quant_kernel, dim3(m), dim3(QUANT_THREADS), smem, stream, true,
+                    static_cast<const __nv_bfloat16*>(dy), dy_row_stride, col_scale, row_map, n, static_cast<int8_t*>(q1), s1,
+                    static_cast<int8_t*>(q2), s2, static_cast<uint4*>(rows));
+  if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "grad_quant launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;
 }

@@ -383,7 +383,7 @@ static int proj_cluster(int m, int slices) {
 int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const float* scaling, int num_adapters,
                        int rank, const TileSource& src, int max_tiles, void* z_parts, int32_t* status,
                        cudaStream_t stream, int row_lo, int row_hi, void* const* extra_dests, int extra_count,
-                       int list_row0) {
+                       int list_row0, int table_rows, int table_k) {
   if (x == nullptr || a_packed == nullptr || scaling == nullptr || z_parts == nullptr || status == nullptr)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "lora_a_proj: null buffer");
   if (m <= 0 || k <= 0 || num_adapters <= 0 || max_tiles <= 0)
@@ -400,9 +400,13 @@ int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const 
   if ((rc = encode_tmap_2d(&p.tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, k, m, static_cast<uint64_t>(k) * 2,
                            PROJ_HALF, PROJ_BM)))
     return rc;
-  if ((rc = encode_tmap_3d(&p.tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a_packed, k, SKYRL_LORA_RANK_PAD,
-                           num_adapters, static_cast<uint64_t>(k) * 2,
-                           static_cast<uint64_t>(k) * 2 * SKYRL_LORA_RANK_PAD, PROJ_HALF, p.rank16)))
+  // table rows past the last, and columns past K where x is padded, read as zeros
+  if (table_k <= 0) table_k = k;
+  if (table_rows < rank || table_k % 8 != 0 || table_k > k)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "lora_a_proj: table of %d rows and %d columns", table_rows, table_k);
+  if ((rc = encode_tmap_3d(&p.tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a_packed, table_k, table_rows, num_adapters,
+                           static_cast<uint64_t>(table_k) * 2, static_cast<uint64_t>(table_k) * 2 * table_rows, PROJ_HALF,
+                           p.rank16)))
     return rc;
   p.scaling = scaling;
   p.src = src;
@@ -436,21 +440,7 @@ int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const 
   if (grid <= 0) return SKYRL_OK;
   p.slices = proj_slices(k);
   const int cluster = proj_cluster(m, p.slices);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid * cluster);
-  cfg.blockDim = dim3(PROJ_THREADS);
-  cfg.dynamicSmemBytes = PROJ_SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  e = cudaLaunchKernelEx(&cfg, lora_a_proj_kernel, static_cast<const ProjParams&>(p));
+  e = launch_cluster_kernel(lora_a_proj_kernel, dim3(grid * cluster), dim3(PROJ_THREADS), PROJ_SMEM_BYTES, stream, cluster, p);
   if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "lora_a_proj launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;

@@ -172,7 +172,8 @@ constexpr int ROUTE_HIST_WORDS = 8192;
 __global__ void __launch_bounds__(ROUTE_THREADS)
 route_dense_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int hist_warps, int32_t* __restrict__ perm,
                    int4* __restrict__ tiles, int4* __restrict__ seg_mask, int32_t* __restrict__ seg_adapter,
-                   int32_t* status, int32_t* __restrict__ zero_words, int zero_count) {
+                   int32_t* status, int32_t* __restrict__ zero_words, int zero_count, int always_sort,
+                   int32_t* __restrict__ adapter_start) {
   extern __shared__ int route_smem[];
   int* hist = route_smem;                        // [hist_warps][num_adapters]: counts, then first positions
   int* nz_start = hist + hist_warps * num_adapters;  // [num_adapters + 1] first sorted row of the non-empty adapters
@@ -251,8 +252,10 @@ route_dense_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int
   }
   __syncthreads();
   const int nonempty = num_nonempty;
+  if (adapter_start != nullptr)
+    for (int a = tid; a <= num_adapters; a += ROUTE_THREADS) adapter_start[a] = a < num_adapters ? total[a] : m;
 
-  if (m <= SKYRL_TILE_ROWS) {  // token order: one tile, every adapter's rows wherever they are
+  if (m <= SKYRL_TILE_ROWS && !always_sort) {  // token order: one tile, every adapter's rows wherever they are
     for (int i = tid; i < m; i += ROUTE_THREADS) perm[i] = i;
     int* words = reinterpret_cast<int*>(seg_mask);
     for (int r = tid; r < nonempty; r += ROUTE_THREADS) {
@@ -332,7 +335,8 @@ route_dense_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int
 }
 
 int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* seg_mask,
-                       int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count) {
+                       int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count,
+                       bool always_sort, int32_t* adapter_start) {
   if (ids == nullptr || m <= 0 || perm == nullptr || tiles == nullptr || seg_mask == nullptr || seg_adapter == nullptr ||
       status == nullptr || !aligned16(tiles) || !aligned16(seg_mask))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: null or misaligned buffer");
@@ -350,7 +354,7 @@ int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* per
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "route attribute: %s", cudaGetErrorString(e));
   e = launch_kernel(route_dense_kernel, dim3(1), dim3(ROUTE_THREADS), smem, stream, true, ids, m, num_adapters, warps, perm,
                     reinterpret_cast<int4*>(tiles), reinterpret_cast<int4*>(seg_mask), seg_adapter, status, zero_words,
-                    zero_count);
+                    zero_count, always_sort ? 1 : 0, adapter_start);
   if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "route launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;

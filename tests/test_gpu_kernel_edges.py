@@ -79,3 +79,32 @@ def test_tiles_of_many_adapters(S, m, k, n, rank, na):
     y = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids), enabled=True)
     S.check_status()
     assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), what=f"{na} adapters")
+
+
+@pytest.mark.parametrize("m,k,n,rank,na", [
+    (1, 64, 40, 8, 1),              # one row; N padded to 64
+    (64, 160, 96, 16, 5),           # within one tile, sorted all the same; one stage of rows
+    (129, 1024, 3072, 64, 2),       # clusters over the rows; a row range that ends one row into a stage
+    (700, 256, 1120, 12, 9),        # a rank that is no multiple of 8: padded tables, scalar stores; adapters that never occur
+    (300, 384, 100, 40, 3),         # rank 40 (three 16-wide column groups in a 64-wide plane), N no multiple of 8
+])
+def test_training_step_against_the_oracle(S, m, k, n, rank, na):
+    from skyrl_tx_rocm_b200 import backward as B
+
+    x, w, a, b, s, ids = make_case(91 + m, m, k, n, rank, na, w_std=0.05)
+    if na == 9:
+        ids = np.where(ids % 3 == 0, 0, ids).astype(np.int32)
+    dy = (np.random.default_rng(m).standard_normal((m, n)) * 0.3).astype(np.float32).astype(x.dtype)
+    q, pw = device_weight(S, w)
+    xd, ad, bd = to_dev(x).requires_grad_(), to_dev(a).requires_grad_(), to_dev(b).requires_grad_()
+    y = B.w8a8_lora_linear_trainable(xd, pw, B.pack_weight_backward(pw), ad, bd, to_dev(s), to_dev(ids))
+    y.backward(to_dev(dy))
+    S.check_status()
+    assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), "y")
+    dx, da, db, _ = O.quantized_lora_linear_vjp(x, q, a, b, s, dy, ids)
+    # bf16 results of fp32 sums: one rounding, 2^-9 relative at most, 2^-9 / sqrt(3) in the 2-norm
+    assert O.relative_l2(to_np(xd.grad), dx) < 4e-3
+    assert O.relative_l2(to_np(ad.grad), da) < 2.0 ** -9
+    assert O.relative_l2(to_np(bd.grad), db) < 2.0 ** -9
+    empty = [i for i in range(na) if not (ids == i).any()]
+    assert not to_np(ad.grad)[empty].astype(np.float32).any() and not to_np(bd.grad)[empty].astype(np.float32).any()
