@@ -51,11 +51,34 @@ struct Pipe {
   __device__ __forceinline__ unsigned char* at() const { return smem + stage * bytes; }
 };
 
+// A tile of many adapters (16 in each of two tiles for 256 rows over 32) would pay one round trip to memory per
+// segment if its adapter and its row mask were read where they are used, between the waits: 17 segments added about 10 us
+// to a tile's tail.  They are read ahead instead: eight adapters at a time by the producing thread, one segment's mask
+// per lane by the issuing warp.
+struct SegmentAdapters {
+  int held[8];
+  int first = -8;
+  template <typename Fetch>
+  __device__ __forceinline__ int at(int j, int nseg, Fetch fetch) {
+    if (j >= first + 8) {
+      first = j & ~7;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) held[i] = first + i < nseg ? fetch(first + i) : 0;
+    }
+    return held[j & 7];
+  }
+};
+__device__ __forceinline__ int4 shfl_int4(const int4& v, int lane) {
+  return make_int4(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
+                   __shfl_sync(0xffffffffu, v.z, lane), __shfl_sync(0xffffffffu, v.w, lane));
+}
+
 template <typename P>
 __device__ __forceinline__ bool lora_load(const P& p, Pipe& q, const int4& tile, int n0, volatile int* abort_flag) {
   const LoraGeom& g = p.lora;
   const int nseg = tile_segments(tile);
   const bool dense = tile_is_dense(tile);
+  SegmentAdapters adapters;
   for (int j = 0; j < nseg;) {
     const int slot = segment_slot(tile, j);
     for (int pl = 0; pl < 3; pl += g.z_per_slot) {  // lo, mid, hi: the smallest plane is added first
@@ -72,7 +95,8 @@ __device__ __forceinline__ bool lora_load(const P& p, Pipe& q, const int4& tile,
       if (!mbar_wait(&q.empty[q.stage], q.phase ^ 1u, abort_flag, p.status, STATUS_TIMEOUT_PRODUCER)) return false;
       mbar_expect_tx(&q.full[q.stage], cnt * g.b_tile);
       for (int i = 0; i < cnt; ++i)
-        tma_load_3d(q.at() + i * g.b_tile, &p.tm_b, 0, n0, segment_adapter(p.src, tile, j + i), &q.full[q.stage]);
+        tma_load_3d(q.at() + i * g.b_tile, &p.tm_b, 0, n0,
+                    adapters.at(j + i, nseg, [&](int s) { return segment_adapter(p.src, tile, s); }), &q.full[q.stage]);
       q.next();
       j += cnt;
       left -= cnt;
@@ -91,6 +115,9 @@ __device__ __forceinline__ bool lora_issue(const P& p, Pipe& q, const int4& tile
   const LoraGeom& g = p.lora;
   const int nseg = tile_segments(tile);
   const bool dense = tile_is_dense(tile);
+  const int lane = static_cast<int>(threadIdx.x & 31u);
+  int4 lane_mask = make_int4(0, 0, 0, 0);  // of segment (j & ~31) + lane
+  int masks_from = -32;
   for (int j = 0; j < nseg;) {
     const int zstage0 = q.stage;
     const int zslots = (3 + g.z_per_slot - 1) / g.z_per_slot;
@@ -108,7 +135,11 @@ __device__ __forceinline__ bool lora_issue(const P& p, Pipe& q, const int4& tile
       tc_fence_after_sync();
       const uint32_t base = smem_u32(q.at());
       for (int i = 0; i < cnt; ++i) {
-        const int4 mk = segment_mask(p.src, tile, j + i);
+        if (j + i >= masks_from + 32) {
+          masks_from = (j + i) & ~31;
+          lane_mask = segment_mask(p.src, tile, min(masks_from + lane, nseg - 1));
+        }
+        const int4 mk = shfl_int4(lane_mask, (j + i) & 31);
         const int4 off = make_int4(~mk.x, ~mk.y, ~mk.z, ~mk.w);
         const uint64_t bd = make_desc_width(base + i * g.b_tile, g.w);
         if (elect_one()) {

@@ -18,8 +18,8 @@
 //
 // A tile of several adapters takes their tables side by side: one MMA of width adapters * rank per K step computes
 // every row against every adapter of the group and the epilogue picks the row's own columns; groups beyond 128 table
-// rows make another pass over the tile with the other rows' lanes disabled.  The whole warp walks the issuing loop
-// and elects a thread for the instruction alone: operands computed by one divergent thread cost the issue 144 cycles
+// rows make another pass over the tile with the other rows' lanes disabled, on a cluster of its own (blockIdx.y) where
+// the GPU has room for it.  The whole warp walks the issuing loop and elects a thread for the instruction alone: operands computed by one divergent thread cost the issue 144 cycles
 // per MMA instead of 47.
 //
 // Reference arithmetic: `x.astype(f32) @ lora_a.astype(f32)`
@@ -117,6 +117,10 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) lora_a_proj_kernel(const __gr
   if (tile_index >= tile_count(p.src)) return;  // uniform for the cluster
   const int4 tile = tile_at(p.src, tile_index);
   if (tile.x >= p.row_hi || tile.x + tile.y <= p.row_lo) return;  // outside the row window, also uniform
+  const int nseg = tile_segments(tile);
+  const int group = min(nseg, PROJ_TABLE_ROWS / p.rank16);  // adapters per pass, at most eight
+  const int seg_begin = static_cast<int>(blockIdx.y) * group, seg_step = static_cast<int>(gridDim.y) * group;
+  if (seg_begin >= nseg) return;  // fewer adapters in this tile than the launch provided for, also uniform
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < PROJ_MAX_STAGES; ++s) {
@@ -139,8 +143,6 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) lora_a_proj_kernel(const __gr
 
   const int kblocks = (p.k + PROJ_BK - 1) / PROJ_BK;
   const int own = p.slices / csize, slice0 = crank * own;  // this CTA's K slices; slices <= kblocks, so none is empty
-  const int nseg = tile_segments(tile);
-  const int group = min(nseg, PROJ_TABLE_ROWS / p.rank16);  // adapters per pass, at most eight
   int slice_cols = 16;                                      // tensor-memory columns of a slice
   while (slice_cols < group * p.rank16) slice_cols <<= 1;
   const int per_phase = min(own, PROJ_TMEM_COLS / slice_cols);  // slices accumulated before the epilogue drains them
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) lora_a_proj_kernel(const __gr
       for (int ph = 0; ph < phases && ok; ++ph) {
         const int kb0 = kblocks * (slice0 + ph * per_phase) / p.slices;
         const int kb1 = kblocks * (slice0 + min(own, (ph + 1) * per_phase)) / p.slices;
-        for (int j0 = 0; j0 < nseg && ok; j0 += group) {
+        for (int j0 = seg_begin; j0 < nseg && ok; j0 += seg_step) {
           const int cnt = min(group, nseg - j0);
           int adapter[8];
 #pragma unroll
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) lora_a_proj_kernel(const __gr
         tc_fence_after_sync();
       }
       const int sl0 = ph * per_phase, sl1 = min(own, sl0 + per_phase);
-      for (int j0 = 0; j0 < nseg && ok; j0 += group) {
+      for (int j0 = seg_begin; j0 < nseg && ok; j0 += seg_step) {
         const int cnt = min(group, nseg - j0);
         const uint32_t idesc = make_idesc(IDESC_D_F32, IDESC_BF16, IDESC_BF16, PROJ_BM, cnt * p.rank16);
         int4 off = make_int4(0, 0, 0, 0);
@@ -246,13 +248,15 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) lora_a_proj_kernel(const __gr
     const int r = warp * 32 + lane;
     // this row's segment: which columns of its pass, which adapter, which z slot
     int seg = 0;
+#pragma unroll 8
     for (int j = 0; j < nseg; ++j) {
       const int4 mk = segment_mask(p.src, tile, j);
       const int word = warp == 0 ? mk.x : (warp == 1 ? mk.y : (warp == 2 ? mk.z : mk.w));
       if ((word >> lane) & 1) seg = j;
     }
     const int64_t row = tile.x + r;
-    const bool row_valid = r < tile.y && row >= p.row_lo && row < p.row_hi;
+    const bool row_valid = r < tile.y && row >= p.row_lo && row < p.row_hi &&
+                           (seg / group) % static_cast<int>(gridDim.y) == static_cast<int>(blockIdx.y);
     const bool dense = tile_is_dense(tile);
     const int slot = segment_slot(tile, seg);
     const float s = __ldg(p.scaling + segment_adapter(p.src, tile, seg));
@@ -440,7 +444,15 @@ int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const 
   if (grid <= 0) return SKYRL_OK;
   p.slices = proj_slices(k);
   const int cluster = proj_cluster(m, p.slices);
-  e = launch_cluster_kernel(lora_a_proj_kernel, dim3(grid * cluster), dim3(PROJ_THREADS), PROJ_SMEM_BYTES, stream, cluster, p);
+  // A tile of more adapters than one pass takes: its passes on clusters of their own where the GPU has room for them (two
+  // tiles of 32 adapters of rank 16 left 132 SMs idle and took three passes in a row: 36 us at K = 12288).
+  int passes = 1;
+  if (src.tiles != nullptr && src.num_tiles == nullptr) {
+    const int most = num_adapters < PROJ_BM ? num_adapters : PROJ_BM, per_pass = PROJ_TABLE_ROWS / p.rank16;
+    const int want = (most + per_pass - 1) / per_pass, room = sm_count() / (grid * cluster);
+    passes = want < room ? want : (room > 1 ? room : 1);
+  }
+  e = launch_cluster_kernel(lora_a_proj_kernel, dim3(grid * cluster, passes), dim3(PROJ_THREADS), PROJ_SMEM_BYTES, stream, cluster, p);
   if (e == cudaSuccess) e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "lora_a_proj launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;

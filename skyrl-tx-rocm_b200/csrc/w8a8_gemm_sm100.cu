@@ -1035,7 +1035,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) w8a8_gemm_pair_kernel(const _
 }
 
 // ---------------------------------------------------------------------------------------------------
-// CTA-pair variant (tcgen05 cta_group::2) for large problems with a short K loop.  Two CTAs of a cluster
+// CTA-pair variant (tcgen05 cta_group::2).  Two CTAs of a cluster
 // compute a 256-row x 256-column output tile: each stages ITS 128-row activation tile and ITS 128 output
 // channels of the weight tile (32 KB per K stage and CTA instead of 48 KB), the leader issues one 256-row MMA
 // per K step that reads both CTAs' shared memory, and each CTA receives its 128 rows of the accumulator in
@@ -1140,8 +1140,6 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  pdl_wait();
-  pdl_trigger();
   const int tm = tile_count(p.src);
   const int tpairs = (tm + 1) / 2;
   const int tn = (p.n + PAIR2_BN - 1) / PAIR2_BN;
@@ -1160,6 +1158,8 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
       int4 prev0 = make_int4(0, 0, 0, 0), prev1 = prev0;
       bool prev_has1 = false;
       int prev_n0 = 0;
+      bool dep_ready = false;  // as in the single-tile kernel: the weights of the first stages before the wait
+      int held = 0, held_stage[PAIR2_STAGES], held_kb[PAIR2_STAGES];
       auto next_stage = [&]() {
         if (++stage == PAIR2_STAGES) {
           stage = 0;
@@ -1173,6 +1173,7 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
         const PairSegments ps = pair_segments(p.src, prev0, prev_has1, prev1);
         const bool dense = tile_is_dense(prev0);
         const int zrow = rank == 0 ? prev0.x : (prev_has1 ? prev1.x : oob_row);
+        SegmentAdapters adapters;
         for (int g = 0; g < ps.count;) {
           // z slot of this adapter in this CTA's tile (lists of two slots; dense lists use the first); the lanes of a
           // tile the adapter does not occur in are left untouched by the MMA, so what is loaded for them is irrelevant
@@ -1196,7 +1197,7 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
             if (leader) mbar_expect_tx(&full_bar[stage], 2 * cnt * geom.b_tile);
             for (int i = 0; i < cnt; ++i)
               tma_load_3d_pair(sa + i * geom.b_tile, &p.tm_b, 0, prev_n0 + static_cast<int>(rank) * 128,
-                               pair_segment_adapter(p.src, ps, g + i), fb);
+                               adapters.at(g + i, ps.count, [&](int s) { return pair_segment_adapter(p.src, ps, s); }), fb);
             next_stage();
             g += cnt;
             left -= cnt;
@@ -1219,8 +1220,22 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
           unsigned char* sa = smem + stage * PAIR2_STAGE_BYTES;
           const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
           if (leader) mbar_expect_tx(&full_bar[stage], 2 * PAIR2_STAGE_BYTES);
-          tma_load_2d_pair(sa, &p.tm_xq, kb * BK, row0, fb);
           tma_load_3d_pair(sa + BM * BK, &p.tm_w, 0, n0 + static_cast<int>(rank) * 128, kb, fb);
+          if (dep_ready) {
+            tma_load_2d_pair(sa, &p.tm_xq, kb * BK, row0, fb);
+          } else {
+            held_stage[held] = stage;
+            held_kb[held] = kb;
+            ++held;
+            if (held == PAIR2_STAGES || kb + 1 == kblocks) {
+              pdl_wait();
+              pdl_trigger();
+              dep_ready = true;
+              for (int hq = 0; hq < held; ++hq)
+                tma_load_2d_pair(smem + held_stage[hq] * PAIR2_STAGE_BYTES, &p.tm_xq, held_kb[hq] * BK, row0,
+                                 map_to_cta(smem_u32(&full_bar[held_stage[hq]]), 0));
+            }
+          }
           next_stage();
           if (HAS_LORA && have_prev && ++issued == inject_at) {
             ok = lora_slots();
@@ -1260,6 +1275,8 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
         const bool dense = tile_is_dense(ps.t0);
         const uint32_t d = tmem_base + acc_stage * PAIR2_BN;
         const int zslots = (3 + geom.z_per_slot - 1) / geom.z_per_slot;
+        int4 lane_off0 = make_int4(0, 0, 0, 0), lane_off1 = lane_off0;  // of segment (g & ~31) + lane
+        int masks_from = -32;
         for (int g = 0; g < ps.count;) {
           const int zstage0 = stage;
           for (int i = 0; i < zslots; ++i) {
@@ -1273,11 +1290,17 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
             tc_fence_after_sync();
             const uint32_t base = smem_base + stage * PAIR2_STAGE_BYTES;
             for (int i = 0; i < cnt; ++i) {
-              const int j0 = pair_segment_of(ps, g + i, 0), j1 = pair_segment_of(ps, g + i, 1);
-              const int4 none = make_int4(0, 0, 0, 0);
-              const int4 m0 = j0 >= 0 ? segment_mask(p.src, ps.t0, j0) : none;
-              const int4 m1 = j1 >= 0 && ps.t1.y > 0 ? segment_mask(p.src, ps.t1, j1) : none;
-              const int4 off0 = make_int4(~m0.x, ~m0.y, ~m0.z, ~m0.w), off1 = make_int4(~m1.x, ~m1.y, ~m1.z, ~m1.w);
+              if (g + i >= masks_from + 32) {
+                masks_from = (g + i) & ~31;
+                const int gl = min(masks_from + lane, ps.count - 1);
+                const int j0 = pair_segment_of(ps, gl, 0), j1 = pair_segment_of(ps, gl, 1);
+                const int4 none = make_int4(0, 0, 0, 0);
+                const int4 m0 = j0 >= 0 ? segment_mask(p.src, ps.t0, j0) : none;
+                const int4 m1 = j1 >= 0 && ps.t1.y > 0 ? segment_mask(p.src, ps.t1, j1) : none;
+                lane_off0 = make_int4(~m0.x, ~m0.y, ~m0.z, ~m0.w);
+                lane_off1 = make_int4(~m1.x, ~m1.y, ~m1.z, ~m1.w);
+              }
+              const int4 off0 = shfl_int4(lane_off0, (g + i) & 31), off1 = shfl_int4(lane_off1, (g + i) & 31);
               const uint64_t bd = make_desc_width(base + i * geom.b_tile, geom.w);
               if (elect_one()) {
                 for (int plane = 0; plane < 3; ++plane) {  // smallest plane first
@@ -1360,6 +1383,7 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
     const uint32_t conv_remote = map_to_cta(smem_u32(conv_done), 0);
     uint32_t it = 0, lora_it = 0;
     bool ok = true;
+    pdl_wait();  // scales and the residual may come from the kernel just before this one
     for (int t = pair_id; t < total && ok; t += num_pairs, ++it) {
       const TileCoord c = tile_coord(t, tpairs, tn, band);
       const int tidx = 2 * c.m_idx + static_cast<int>(rank);
@@ -1590,6 +1614,18 @@ GemmPlan plan_gemm(int m, int n, int k, int epilogue, int max_slabs) {
   return pl;
 }
 
+// Cycles per SM of the two forms (see launch_gemm): waves x (K loop + LoRA MMAs, three planes per adapter of the tile).
+static bool pair_is_faster(int mt, int n, int kblocks, int bn, int sms, int rank, int adapters) {
+  const int tn = (n + bn - 1) / bn, tn_pair = (n + PAIR2_BN - 1) / PAIR2_BN;
+  const double lora = rank > 0 ? 3.0 * ((rank + 15) / 16) : 0.0;
+  const double cuts = adapters > 1 ? static_cast<double>(adapters - 1) / mt : 0.0;  // adapter boundaries per M tile
+  const int64_t waves = (static_cast<int64_t>(mt) * tn + sms - 1) / sms;
+  const int64_t waves_pair = (static_cast<int64_t>((mt + 1) / 2) * tn_pair + sms / 2 - 1) / (sms / 2);
+  const double single = waves * ((202 + 1.58 * bn) * kblocks + lora * 75 * (1 + cuts));
+  const double pair = waves_pair * (527.0 * kblocks + lora * 128 * (1 + 2 * cuts));
+  return pair < single;
+}
+
 int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic, const TileSource* src) {
   if (a.struct_size != sizeof(SkyrlW8A8GemmArgs))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: struct_size %u does not match ABI v%d (%zu)", a.struct_size,
@@ -1640,26 +1676,29 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   int bn_eff = pl.bn_eff;
   if (rows && a.m > 64 && bn_eff > 128) bn_eff = 128;  // the l tile (rows x columns fp32) must leave room for the pipeline
   const int k_splits = pl.k_splits, kb_per_split = pl.kb_per_split;
-  const int bn = bn_eff > 128 ? 256 : 128;
-  // Kernel variant for large problems (all give the same bits).
-  //   long K loop (>= 64 blocks of 128): a CTA pair per 256 x 256 tile (tcgen05 cta_group::2): each CTA stages its
-  //     128 rows and half of the weight tile, a third fewer bytes per unit of tensor-core work, two accumulator
-  //     stages, sixteen epilogue warps.  Measured on B200: down projection of the Qwen3-32B-shaped block (K = 25600)
-  //     1.57 ms against 1.61 ms for the two-tiles-per-CTA kernel, the Qwen3-8B-shaped one (K = 12288) 0.555 against
-  //     0.607 ms.  With a CTA cap (a concurrent stream wants SMs) the two-tile kernel, whose tile claims are dynamic.
-  //   shorter K loop: one 128 x 256 tile per CTA.  There the MMA-issuing thread is blocked on the tensor pipe ~89 %
-  //     of the time whatever the variant (SKYRL_GEMM_VARIANT_PROFILE), the CTA pair brings nothing (K = 5120:
-  //     3.61 ms against 3.50 ms), and the single tile keeps dynamic tile claims.
-  // Neither pair form with a row scatter (their epilogues' tile order is static / their stores are 16 bytes per
-  // row from registers, which NVLink carries poorly).
-  const bool big = !rows && bn_eff == 256 && k_splits == 1 && a.scatter_rows == 0 &&
-                   static_cast<int64_t>(mt_est) * ((a.n + 255) / 256) >= 4 * sms;
-  bool pair2 = big && kblocks_of(a.k) >= 64 && a.cta_limit <= 0;
-  bool paired = big && kblocks_of(a.k) >= 64 && !pair2;
+  // Kernel variant (all give the same bits).
+  //   CTA pair, 256 x 256 (tcgen05 cta_group::2): each CTA stages its 128 rows and half of the weight tile.  A K block
+  //     costs the pair 527 cycles (the MMAs themselves are 512), the single-tile kernel 607 at 256 columns and
+  //     about 202 + 1.58 columns below: what enters and leaves shared memory bounds it.  Measured on B200, whole calls:
+  //     2048 x 4096 -> 6144 85.6 -> 82.9 us; 3000 x 2048 -> 12288 SwiGLU 153 -> 143; 4096 x 12288 -> 4096 250 -> 237;
+  //     8192 x 4096 -> 24576 SwiGLU 722 -> 687; 16384 x 5120 -> 51200 SwiGLU, rank 64 3582 -> 3405.
+  //   Single tile where that takes fewer or cheaper waves (1500 x 2048 -> 2048: 29.1 us on 192 columns, pair 30.9), or
+  //     where many adapters meet a tile: every adapter of a pair costs MMAs over all 256 rows (256 x 4096 -> 24576
+  //     with 32 adapters: 81 us, pair 94).
+  // With a CTA cap (a concurrent stream wants SMs) no pair: its tile schedule is static; a long K loop then takes the
+  // two-tiles-per-CTA kernel, whose claims are dynamic.  Neither with a row scatter (static tile order / 16-byte
+  // stores from registers, which NVLink carries poorly).
+  const bool wide = !rows && k_splits == 1 && a.scatter_rows == 0 && a.n >= 256;
+  const bool big = wide && bn_eff == 256 && static_cast<int64_t>(mt_est) * ((a.n + 255) / 256) >= 4 * sms;
+  bool pair2 = wide && a.cta_limit <= 0 && mt_est >= 2 && a.epilogue != SKYRL_EPI_ACC_I32 &&
+               pair_is_faster(mt_est, a.n, kblocks_of(a.k), bn_eff, sms, lora ? a.rank : 0, a.num_adapters);
+  bool paired = big && kblocks_of(a.k) >= 64 && a.cta_limit > 0;
   const int forced = a.variant & 3;
   if (forced == SKYRL_GEMM_VARIANT_SINGLE) paired = pair2 = false;
   if (forced == SKYRL_GEMM_VARIANT_TWO_TILES) paired = big, pair2 = false;
   if (forced == SKYRL_GEMM_VARIANT_CTA_PAIR) pair2 = big && a.cta_limit <= 0, paired = paired && !pair2;
+  if (pair2) bn_eff = PAIR2_BN;
+  const int bn = bn_eff > 128 ? 256 : 128;
   const int w_box_rows = pair2 ? 128 : bn_eff;   // a CTA of a pair stages half of the weight (and LoRA-B) tile
 
   GemmParams p;

@@ -108,3 +108,24 @@ def test_training_step_against_the_oracle(S, m, k, n, rank, na):
     assert O.relative_l2(to_np(bd.grad), db) < 2.0 ** -9
     empty = [i for i in range(na) if not (ids == i).any()]
     assert not to_np(ad.grad)[empty].astype(np.float32).any() and not to_np(bd.grad)[empty].astype(np.float32).any()
+
+
+@pytest.mark.parametrize("m,k,n,rank,na", [
+    (900, 256, 4160, 0, 1),         # fewer K blocks than pipeline stages; a tile of four rows, a column tile of 64
+    (773, 2048, 4608, 8, 1),        # an odd number of M tiles: the last pair has one
+    (897, 4096, 4128, 16, 3),       # a tile of one row; adapters that change inside a pair
+])
+def test_cta_pairs_below_four_waves(S, m, k, n, rank, na):
+    x, w, a, b, s, ids = make_case(77 + m, m, k, n, max(rank, 1), na, w_std=0.05)
+    q, pw = device_weight(S, w)
+    if rank == 0:
+        y = S.w8a8_frozen_linear(to_dev(x), pw, enabled=True)
+        np.testing.assert_array_equal(to_np(y).view(np.uint16), O.quantized_lora_linear(x, q).view(np.uint16))
+        return
+    lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=pw.in_features,
+                       padded_out_features=pw.padded_out_features)
+    y = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids) if na > 1 else None, enabled=True)
+    one = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids) if na > 1 else None, enabled=True, gemm_variant=1)
+    S.check_status()
+    assert torch.equal(y, one)
+    assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), what=f"{m} rows")
