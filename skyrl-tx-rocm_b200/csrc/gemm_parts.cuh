@@ -105,6 +105,21 @@ __device__ __forceinline__ bool lora_load(const P& p, Pipe& q, const int4& tile,
   return true;
 }
 
+// Descriptors of the three z planes of a round whose first slot is `stage`.  Computed once: with a division per plane in
+// front of every MMA an adapter cost the issuing warp 1400 cycles.
+__device__ __forceinline__ void lora_plane_descs(const LoraGeom& g, uint32_t smem_base, int stage_bytes, int stages, int stage,
+                                                 uint64_t (&zd)[3]) {
+  int in_slot = 0;
+#pragma unroll
+  for (int plane = 0; plane < 3; ++plane) {
+    zd[plane] = make_desc_width(smem_base + stage * stage_bytes + in_slot * g.z_plane, g.w);
+    if (++in_slot == g.z_per_slot) {
+      in_slot = 0;
+      stage = stage + 1 == stages ? 0 : stage + 1;
+    }
+  }
+}
+
 // rank-r bf16 MMAs of one tile, accumulated onto the accumulator `d` the epilogue rewrote as fp32 (`ready` waits for
 // that rewrite, once the first operands are there); every segment touches the lanes of its own rows only.  FRESH: `d` are
 // columns of the LoRA term's own, whose first contribution overwrites.  Called by a whole warp, which elects a thread for
@@ -125,6 +140,8 @@ __device__ __forceinline__ bool lora_issue(const P& p, Pipe& q, const int4& tile
       if (!mbar_wait_warp(&q.full[q.stage], q.phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
       q.next();
     }
+    uint64_t zd[3];
+    lora_plane_descs(g, smem_u32(q.smem), q.bytes, q.stages, zstage0, zd);
     const bool first = j == 0;
     bool started = false;
     for (int left = dense ? min(nseg - j, g.b_per_round) : 1; left > 0;) {
@@ -133,7 +150,7 @@ __device__ __forceinline__ bool lora_issue(const P& p, Pipe& q, const int4& tile
       if (first && !started && !ready()) return false;
       started = true;
       tc_fence_after_sync();
-      const uint32_t base = smem_u32(q.at());
+      uint64_t bd = make_desc_width(smem_u32(q.at()), g.w);
       for (int i = 0; i < cnt; ++i) {
         if (j + i >= masks_from + 32) {
           masks_from = (j + i) & ~31;
@@ -141,16 +158,14 @@ __device__ __forceinline__ bool lora_issue(const P& p, Pipe& q, const int4& tile
         }
         const int4 mk = shfl_int4(lane_mask, (j + i) & 31);
         const int4 off = make_int4(~mk.x, ~mk.y, ~mk.z, ~mk.w);
-        const uint64_t bd = make_desc_width(base + i * g.b_tile, g.w);
         if (elect_one()) {
-          for (int plane = 0; plane < 3; ++plane) {
-            int zs = zstage0 + plane / g.z_per_slot;
-            if (zs >= q.stages) zs -= q.stages;
-            const uint64_t zd = make_desc_width(smem_u32(q.smem + zs * q.bytes) + (plane % g.z_per_slot) * g.z_plane, g.w);
-            for (int kk = 0; kk < p.rank_blocks; ++kk) mma_bf16_lanes(d, zd + 2 * kk, bd + 2 * kk, idesc, FRESH && plane == 0 && kk == 0 ? 0u : 1u, off);
-          }
+#pragma unroll
+          for (int plane = 0; plane < 3; ++plane)
+            for (int kk = 0; kk < p.rank_blocks; ++kk)
+              mma_bf16_lanes(d, zd[plane] + 2 * kk, bd + 2 * kk, idesc, FRESH && plane == 0 && kk == 0 ? 0u : 1u, off);
         }
         __syncwarp();
+        bd += g.b_tile >> 4;  // the descriptor's address field counts 16 bytes
       }
       if (elect_one()) mma_commit(&q.empty[q.stage]);
       __syncwarp();

@@ -1283,12 +1283,14 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
             if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
             next_stage();
           }
+          uint64_t zd[3];
+          lora_plane_descs(geom, smem_base, PAIR2_STAGE_BYTES, PAIR2_STAGES, zstage0, zd);
           if (g == 0 && !timed_wait(prof, pr.rewrite, conv_done, lora_rounds & 1u, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
           for (int left = dense ? min(ps.count - g, geom.b_per_round) : 1; left > 0;) {
             const int cnt = min(geom.b_per_slot, left);
             if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_LORA)) return false;
             tc_fence_after_sync();
-            const uint32_t base = smem_base + stage * PAIR2_STAGE_BYTES;
+            uint64_t bd = make_desc_width(smem_base + stage * PAIR2_STAGE_BYTES, geom.w);
             for (int i = 0; i < cnt; ++i) {
               if (g + i >= masks_from + 32) {
                 masks_from = (g + i) & ~31;
@@ -1301,17 +1303,14 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
                 lane_off1 = make_int4(~m1.x, ~m1.y, ~m1.z, ~m1.w);
               }
               const int4 off0 = shfl_int4(lane_off0, (g + i) & 31), off1 = shfl_int4(lane_off1, (g + i) & 31);
-              const uint64_t bd = make_desc_width(base + i * geom.b_tile, geom.w);
               if (elect_one()) {
-                for (int plane = 0; plane < 3; ++plane) {  // smallest plane first
-                  int zs = zstage0 + plane / geom.z_per_slot;
-                  if (zs >= PAIR2_STAGES) zs -= PAIR2_STAGES;
-                  const uint64_t zd = make_desc_width(smem_base + zs * PAIR2_STAGE_BYTES + (plane % geom.z_per_slot) * geom.z_plane, geom.w);
+#pragma unroll
+                for (int plane = 0; plane < 3; ++plane)  // smallest plane first
                   for (int kk = 0; kk < p.rank_blocks; ++kk)
-                    mma_bf16_pair_lanes(d, zd + 2 * kk, bd + 2 * kk, idesc_lora, 1u, off0, off1);
-                }
+                    mma_bf16_pair_lanes(d, zd[plane] + 2 * kk, bd + 2 * kk, idesc_lora, 1u, off0, off1);
               }
               __syncwarp();
+              bd += geom.b_tile >> 4;
             }
             if (elect_one()) mma_commit_pair(&empty_bar[stage]);
             __syncwarp();
