@@ -144,6 +144,8 @@ SYMBOLS = {
     "skyrl_w8a8_linear_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "skyrl_w8a8_lora_forward_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "skyrl_w8a8_grouped_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "skyrl_w8a8_lora_forward_split_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_int32, C.POINTER(C.c_int32),
+                                               C.POINTER(C.c_void_p), C.c_void_p]),
     "skyrl_w8a8_lora_forward_grouped_sm100_v1": (C.c_int, [C.POINTER(LinearArgs), C.c_int32, C.c_void_p]),
     "skyrl_w8a8_train_saved_bytes": (C.c_size_t, [C.c_int32, C.c_int32]),
     "skyrl_w8a8_train_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),

@@ -257,6 +257,7 @@ struct Projection {
   int32_t* acc;
   TileSource src;
   int epilogue;
+  ColumnSplit split;      // linear epilogue: output columns dealt to several matrices (count 0: `out`)
   const int32_t* out_row_map;
   const void* residual;
   int64_t residual_stride;
@@ -359,7 +360,7 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
     if (rc) return rc;
     return launch_finalize_rows(q.epilogue, q.acc, slabs, q.sx, q.sw, z_rows, q.ids, q.na,
                                 dense ? q.b_rows : q.b_packed, static_cast<int64_t>(q.n) * brow, brow, q.rank, q.m, q.n,
-                                q.residual, q.residual_stride, q.out, q.out_stride, q.status, stream, chain);
+                                q.residual, q.residual_stride, q.out, q.out_stride, q.status, stream, chain, q.split);
   }
   {
     if (!q.skip_quant && (rc = run_quant_stage(q, stream))) return rc;
@@ -406,7 +407,8 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
   if (q.ev_begin != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_begin), stream);
   // launched programmatically behind this call's own quantiser stage: what it reads before its wait (the tile list)
   // then comes from at least two kernels back
-  rc = launch_gemm(g, stream, !q.skip_quant && q.ev_begin == nullptr && q.ev_end == nullptr, &q.src);
+  rc = launch_gemm(g, stream, !q.skip_quant && q.ev_begin == nullptr && q.ev_end == nullptr, &q.src,
+                   q.split.count > 0 ? &q.split : nullptr);
   if (q.ev_end != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_end), stream);
   return rc;
 }
@@ -428,7 +430,7 @@ extern "C" size_t skyrl_w8a8_mlp_workspace_bytes(int32_t m, int32_t hidden, int3
   return carve_mlp(nullptr, m, hidden, inter, num_adapters).bytes;
 }
 
-extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, skyrl_stream_t stream_) {
+static int linear_forward(const SkyrlW8A8LinearArgs* a, const ColumnSplit& split, skyrl_stream_t stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (a == nullptr) return fail(SKYRL_ERR_INVALID_ARGUMENT, "linear: args is null");
   if (a->struct_size != sizeof(SkyrlW8A8LinearArgs))
@@ -484,6 +486,7 @@ extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, sk
   q.b_rows_rank = a->lora_b_rows_rank;
   q.src = tile_source(w.route, routed, 0, a->m);
   q.epilogue = a->epilogue;
+  q.split = split;
   q.out_row_map = routed ? w.route.perm : nullptr;
   q.residual = a->residual;
   q.residual_stride = a->residual_row_stride;
@@ -495,6 +498,30 @@ extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, sk
   q.ev_begin = a->timing_events[0];
   q.ev_end = a->timing_events[1];
   return run_projection(q, stream);
+}
+
+extern "C" int skyrl_w8a8_lora_forward_sm100_v1(const SkyrlW8A8LinearArgs* a, skyrl_stream_t stream) {
+  return linear_forward(a, ColumnSplit{}, stream);
+}
+
+extern "C" int skyrl_w8a8_lora_forward_split_sm100_v1(const SkyrlW8A8LinearArgs* a, int32_t parts, const int32_t* part_cols,
+                                                      void* const* outs, skyrl_stream_t stream) {
+  if (a == nullptr || part_cols == nullptr || outs == nullptr || parts < 1 || parts > 4)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "split linear: one to four parts");
+  if (a->struct_size != sizeof(SkyrlW8A8LinearArgs))
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "split linear: struct_size %u does not match", a->struct_size);
+  ColumnSplit s = {};
+  s.count = parts;
+  for (int i = 0; i < parts; ++i) {
+    if (part_cols[i] <= 0 || part_cols[i] % 32 != 0 || part_cols[i] > (1 << 24) || outs[i] == nullptr || !aligned16(outs[i]))
+      return fail(SKYRL_ERR_INVALID_ARGUMENT, "split linear: part %d needs a multiple of 32 columns and a 16-byte aligned output", i);
+    s.off[i + 1] = s.off[i] + part_cols[i];
+    s.base[i] = outs[i];
+  }
+  s.group = s.off[parts];
+  if (a->epilogue != SKYRL_EPI_LINEAR || a->rank <= 0 || (a->flags & SKYRL_LINEAR_FUSED_ROWS) != 0 || a->n % s.group != 0)
+    return fail(SKYRL_ERR_INVALID_ARGUMENT, "split linear: a linear with a LoRA term whose N is whole groups of the parts");
+  return linear_forward(a, s, stream);
 }
 
 // ---- group-wise scales ---------------------------------------------------------

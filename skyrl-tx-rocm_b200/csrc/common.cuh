@@ -104,6 +104,33 @@ int launch_lora_a_proj(const void* x, int m, int k, const void* a_packed, const 
                        cudaStream_t stream, int row_lo = 0, int row_hi = -1, void* const* extra_dests = nullptr,
                        int extra_count = 0, int list_row0 = -1,  // extra copies of the rows written
                        int table_rows = SKYRL_LORA_RANK_PAD, int table_k = 0);  // rows and columns of a table (0: k)
+// Output columns dealt to several matrices: every run of `group` columns is off[1] - off[0] columns of part 0, then
+// off[2] - off[1] of part 1, ... (the fused q / k / v layout); count 0: one matrix.  Parts are multiples of 32 columns.
+struct ColumnSplit {
+  int count, group;
+  int off[5];
+  void* base[4];
+};
+#ifdef __CUDACC__
+// the part of column nc, its row length and the column in it; a run of 32 columns from a multiple of 32 stays in one part
+__device__ __forceinline__ void split_column(const ColumnSplit& s, int n, int nc, void*& out, int64_t& stride, int& col) {
+  const int g = nc / s.group, c = nc - g * s.group;
+  int part = 0;
+#pragma unroll
+  for (int i = 1; i < 4; ++i)
+    if (i < s.count && c >= s.off[i]) part = i;
+  int lo = 0, hi = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (i == part) {
+      out = s.base[i];
+      lo = s.off[i];
+      hi = s.off[i + 1];
+    }
+  stride = static_cast<int64_t>(n / s.group) * (hi - lo);
+  col = g * (hi - lo) + c - lo;
+}
+#endif
 // Tile width and K split the GEMM launcher chooses for a shape (deterministic per device).
 struct GemmPlan {
   int bn_eff;
@@ -113,7 +140,8 @@ struct GemmPlan {
 GemmPlan plan_gemm(int m, int n, int k, int epilogue, int max_slabs);
 constexpr int MAX_SPLIT_K_SLABS = 16;
 // `src`: the M tiles, where they are not the two-adapter list in `a` (nullptr: a.tiles / a.num_tiles).
-int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic = false, const TileSource* src = nullptr);
+int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic = false, const TileSource* src = nullptr,
+                const ColumnSplit* split = nullptr);  // split: SKYRL_EPI_LINEAR only
 // `programmatic`: launch with programmatic stream serialization (small-batch chain of short kernels)
 // Adapter ids outside [0, num_adapters) are clamped and STATUS_BAD_ADAPTER_ID is recorded in `status`.
 int launch_rms_quant_rows(const void* x, int64_t x_row_stride, const void* rms_delta, float eps, const int32_t* ids,
@@ -123,7 +151,7 @@ int launch_rms_quant_rows(const void* x, int64_t x_row_stride, const void* rms_d
 int launch_finalize_rows(int epilogue, const int32_t* acc, int slabs, const float* sx, const float* sw, const float* z_rows,
                          const int32_t* ids, int num_adapters, const void* b_table, int64_t b_adapter_stride,
                          int b_row_stride, int rank, int m, int n, const void* residual, int64_t res_stride, void* out,
-                         int64_t out_stride, int32_t* status, cudaStream_t stream, bool programmatic = false);
+                         int64_t out_stride, int32_t* status, cudaStream_t stream, bool programmatic, const ColumnSplit& split);
 // Linear on group-wise scales (grouped_gemm_sm100.cu): a scale per row and group, a weight scale per group and column.
 int launch_group_quant(const void* x, int64_t x_row_stride, const int32_t* row_map, int m, int k, int group, void* xq,
                        float* sx, void* xn, cudaStream_t stream);

@@ -221,7 +221,7 @@ finalize_rows_kernel(const int32_t* __restrict__ acc, int slabs, int64_t slab_st
                      const float* __restrict__ z_rows, const int32_t* __restrict__ ids, int num_adapters,
                      const __nv_bfloat16* __restrict__ b_table, int64_t b_adapter_stride, int b_row_stride,
                      int rank_vecs, int n, const __nv_bfloat16* __restrict__ residual, int64_t res_stride,
-                     void* __restrict__ out, int64_t out_stride, int32_t* status) {
+                     void* __restrict__ out, int64_t out_stride, int32_t* status, ColumnSplit split) {
   __shared__ float zs[SKYRL_LORA_RANK_PAD];
   const int m = blockIdx.y;
   if (rank_vecs > 0 && threadIdx.x < SKYRL_LORA_RANK_PAD)
@@ -318,8 +318,11 @@ finalize_rows_kernel(const int32_t* __restrict__ acc, int slabs, int64_t slab_st
       *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(out) + static_cast<int64_t>(m) * out_stride + n0) =
           pack_bf16x2(__fadd_rn(round_bf16(f0), bf16_lo(rv[j])), __fadd_rn(round_bf16(f1), bf16_hi(rv[j])));
     } else {
-      *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(out) + static_cast<int64_t>(m) * out_stride + n0) =
-          pack_bf16x2(f0, f1);
+      void* to = out;
+      int64_t stride = out_stride;
+      int col = n0;
+      if (split.count > 0) split_column(split, n, n0, to, stride, col);
+      *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(to) + static_cast<int64_t>(m) * stride + col) = pack_bf16x2(f0, f1);
     }
   }
 }
@@ -374,7 +377,7 @@ int launch_finalize_rows(int epilogue, const int32_t* acc, int slabs, const floa
                          const float* z_rows, const int32_t* ids, int num_adapters, const void* b_table,
                          int64_t b_adapter_stride, int b_row_stride, int rank, int m, int n, const void* residual,
                          int64_t res_stride, void* out, int64_t out_stride, int32_t* status, cudaStream_t stream,
-                         bool programmatic) {
+                         bool programmatic, const ColumnSplit& split) {
   if (acc == nullptr || sx == nullptr || sw == nullptr || out == nullptr || status == nullptr || m <= 0 || n <= 0 ||
       n % 2 != 0 || m > 65535 || num_adapters <= 0)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "finalize_rows: null buffer or bad shape");
@@ -394,7 +397,7 @@ int launch_finalize_rows(int epilogue, const int32_t* acc, int slabs, const floa
 #define SKYRL_FINALIZE_P(E, PP, RR)                                                                                  \
   le = launch_kernel(finalize_rows_kernel<E, PP, RR>, grid, dim3(256), 0, stream, programmatic, acc, slabs,          \
                      static_cast<int64_t>(m) * n, sx, sw, z_rows, ids, num_adapters, bt, b_adapter_stride, b_row_stride, \
-                     rank_vecs, n, res, res_stride, out, out_stride, status)
+                     rank_vecs, n, res, res_stride, out, out_stride, status, split)
 #define SKYRL_FINALIZE(E)                                \
   if (wide_rank) {                                       \
     SKYRL_FINALIZE_P(E, 1, 8);                           \

@@ -23,9 +23,8 @@
 // pipeline depth (the main loop is bound by bytes in flight per SM).
 //
 // Rows live in the adapter-sorted space: every 128-row M tile comes from the
-// tile list and holds rows of at most two adapters (each row's z is zero in the
-// slot of the adapter that is not its own); rows past the tile's count are
-// computed but never stored.  Every wait is bounded (see ptx_sm100.cuh).
+// tile list, whatever adapters its rows belong to (tiles.cuh); rows past the tile's
+// count are computed but never stored.  Every wait is bounded (see ptx_sm100.cuh).
 #include <stdlib.h>
 
 #include <mutex>
@@ -110,6 +109,7 @@ struct GemmParams {
   int profile;                 // 1: the MMA issuer of CTA 0 adds the cycles it spent waiting to status[1..3]
   int lterm_off;               // byte offset of the l tile inside the stage area
   int lterm_pitch;             // floats per row of the l tile (odd, so that a column is conflict-free)
+  ColumnSplit split;           // linear epilogue: the output columns of several matrices
   const unsigned char* prefetch;  // bytes another kernel will stream soon: requested into L2 once the own loads are out
   long long prefetch_bytes;
 };
@@ -371,8 +371,12 @@ __device__ __forceinline__ void epi_store_chunk(const GemmParams& p, uint32_t ta
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j) o[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
-      epi_staged_store(stage, lane, o, 16, row_valid, orow, static_cast<__nv_bfloat16*>(p.out), p.out_stride, nc,
-                       n_end - nc, EPI == SKYRL_EPI_RESIDUAL ? p.residual : nullptr, p.res_stride);
+      void* to = p.out;
+      int64_t stride = p.out_stride;
+      int col = nc;
+      if (EPI == SKYRL_EPI_LINEAR && p.split.count > 0 && nc < n_end) split_column(p.split, p.n, nc, to, stride, col);
+      epi_staged_store(stage, lane, o, 16, row_valid, orow, static_cast<__nv_bfloat16*>(to), stride, col, n_end - nc,
+                       EPI == SKYRL_EPI_RESIDUAL ? p.residual : nullptr, p.res_stride);
     }
     return;
   }
@@ -1625,7 +1629,8 @@ static bool pair_is_faster(int mt, int n, int kblocks, int bn, int sms, int rank
   return pair < single;
 }
 
-int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic, const TileSource* src) {
+int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmatic, const TileSource* src,
+                const ColumnSplit* split) {
   if (a.struct_size != sizeof(SkyrlW8A8GemmArgs))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: struct_size %u does not match ABI v%d (%zu)", a.struct_size,
                 SKYRL_W8A8_ABI_VERSION, sizeof(SkyrlW8A8GemmArgs));
@@ -1689,7 +1694,7 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   // stores from registers, which NVLink carries poorly).
   const bool wide = !rows && k_splits == 1 && a.scatter_rows == 0 && a.n >= 256;
   const bool big = wide && bn_eff == 256 && static_cast<int64_t>(mt_est) * ((a.n + 255) / 256) >= 4 * sms;
-  bool pair2 = wide && a.cta_limit <= 0 && mt_est >= 2 && a.epilogue != SKYRL_EPI_ACC_I32 &&
+  bool pair2 = wide && a.cta_limit <= 0 && mt_est >= 2 && (a.epilogue != SKYRL_EPI_ACC_I32 || big) &&
                pair_is_faster(mt_est, a.n, kblocks_of(a.k), bn_eff, sms, lora ? a.rank : 0, a.num_adapters);
   bool paired = big && kblocks_of(a.k) >= 64 && a.cta_limit > 0;
   const int forced = a.variant & 3;
@@ -1697,6 +1702,11 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   if (forced == SKYRL_GEMM_VARIANT_TWO_TILES) paired = big, pair2 = false;
   if (forced == SKYRL_GEMM_VARIANT_CTA_PAIR) pair2 = big && a.cta_limit <= 0, paired = paired && !pair2;
   if (pair2) bn_eff = PAIR2_BN;
+  if (split != nullptr) {
+    if (a.epilogue != SKYRL_EPI_LINEAR || rows) return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: split columns need the linear epilogue");
+    paired = false;                      // its stores come straight from registers
+    bn_eff = (bn_eff + 31) / 32 * 32;    // chunks of 32 columns stay inside a part
+  }
   const int bn = bn_eff > 128 ? 256 : 128;
   const int w_box_rows = pair2 ? 128 : bn_eff;   // a CTA of a pair stages half of the weight (and LoRA-B) tile
 
@@ -1726,6 +1736,7 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
     p.tm_z = p.tm_xq;
     p.tm_b = p.tm_xq;
   }
+  p.split = split != nullptr ? *split : ColumnSplit{};
   p.sx = a.sx;
   p.sw = a.sw;
   p.src = src != nullptr ? *src : TileSource{reinterpret_cast<const int4*>(a.tiles), nullptr, nullptr, a.num_tiles, 0, 0, a.m};

@@ -511,7 +511,7 @@ def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids
 
 
 def _run_linear(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids, epilogue, *, rms_delta=None, eps=RMS_EPS,
-                residual=None, out=None, timing_events=None, fused_rows=False, gemm_variant=0):
+                residual=None, out=None, timing_events=None, fused_rows=False, gemm_variant=0, parts=None):
     if weight.group_size:
         if epilogue != EPI_LINEAR or rms_delta is not None or residual is not None:
             raise SkyrlKernelError("grouped weights (group_size < K) are served by w8a8_lora_linear and "
@@ -530,6 +530,11 @@ def _run_linear(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids, epilog
         out_cols, out_dtype = npad, torch.float32
     else:
         out_cols, out_dtype = npad, torch.bfloat16
+    outs = None
+    if parts is not None:
+        groups = npad // sum(parts)
+        outs = tuple(torch.empty((m, groups * g), dtype=out_dtype, device=dev) for g in parts)
+        out = outs[0]
     if out is None:
         out = torch.empty((m, out_cols), dtype=out_dtype, device=dev)
     na = lora.num_adapters if lora is not None else 1
@@ -560,10 +565,15 @@ def _run_linear(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids, epilog
         a.residual = residual.data_ptr()
         a.residual_row_stride = residual.stride(0)
     a.out = out.data_ptr()
-    a.out_row_stride = out.stride(0)
+    a.out_row_stride = out_cols if outs is not None else out.stride(0)
     a.workspace = ws.data_ptr()
     a.workspace_bytes = nbytes
     a.status = st.data_ptr()
+    if outs is not None:
+        _lib.check(lib.skyrl_w8a8_lora_forward_split_sm100_v1(
+            C.byref(a), len(parts), (C.c_int32 * len(parts))(*parts), (C.c_void_p * len(parts))(*[o.data_ptr() for o in outs]),
+            _stream()), "w8a8_lora_forward_split")
+        return outs
     if timing_events is not None:
         a.timing_events[0], a.timing_events[1] = timing_events[0].cuda_event, timing_events[1].cuda_event
     # every fused variant has its own exported target (one symbol per operator, as a custom-call layer binds them)
@@ -623,6 +633,22 @@ def w8a8_lora_linear(x, weight, lora_a, lora_b=None, lora_scaling=None, adapter_
     ids = _check_ids(adapter_ids, x2.shape[0], lora)
     y = _run_linear(x2, w, lora, ids, EPI_LINEAR, timing_events=timing_events, fused_rows=fused_rows, gemm_variant=gemm_variant)
     return y[:, : w.out_features].reshape(*x.shape[:-1], w.out_features)
+
+
+def can_split_columns(weight, lora, parts) -> bool:
+    """Whether the projection kernels can write a fused projection's components themselves: whole 32-column chunks,
+    no padded columns, per-channel scales, a LoRA term."""
+    return (isinstance(weight, PackedW8Weight) and isinstance(lora, PackedLoRA) and not weight.group_size and 1 <= len(parts) <= 4
+            and all(g > 0 and g % 32 == 0 for g in parts) and weight.out_features == weight.padded_out_features
+            and weight.out_features % sum(parts) == 0)
+
+
+def w8a8_lora_linear_split(x, weight: PackedW8Weight, lora: PackedLoRA, adapter_ids, parts):
+    """`w8a8_lora_linear` with the output columns dealt to one contiguous tensor per component."""
+    x2 = _check_x(x, weight.in_features)
+    lora = _lora_of(weight, lora, None, None)
+    outs = _run_linear(x2, weight, lora, _check_ids(adapter_ids, x2.shape[0], lora), EPI_LINEAR, parts=parts)
+    return tuple(o.reshape(*x.shape[:-1], o.shape[1]) for o in outs)
 
 
 def w8a8_lora_linear_f32(x, weight, lora_a=None, lora_b=None, lora_scaling=None, adapter_ids=None, *,

@@ -92,4 +92,7 @@ class FusedLoRALinearW8(LoRALinearW8):
         self.group_sizes = tuple(int(g) for g in group_sizes)
 
     def __call__(self, x, adapter_indices=None):
+        if self.enabled and x.ndim >= 2 and ops.can_split_columns(self.weight, self.lora, self.group_sizes):
+            # the GEMM writes the components: splitting its output was three strided copies, 28 of 121 us at 2048 rows
+            return ops.w8a8_lora_linear_split(x, self.weight, self.lora, self._token_ids(x, adapter_indices), self.group_sizes)
         return split_components(super().__call__(x, adapter_indices), self.group_sizes)

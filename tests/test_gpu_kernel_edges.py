@@ -129,3 +129,27 @@ def test_cta_pairs_below_four_waves(S, m, k, n, rank, na):
     S.check_status()
     assert torch.equal(y, one)
     assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), what=f"{m} rows")
+
+
+@pytest.mark.parametrize("m,k,parts,groups,rank,na", [
+    (1, 64, (32,), 1, 8, 1),                # the row-wise route; a single part
+    (100, 256, (64, 32, 32), 3, 16, 5),     # parts that end inside a tile
+    (129, 512, (96, 32), 5, 32, 3),         # the sorted route, narrow column tiles
+    (900, 2048, (512, 128, 128), 6, 8, 2),  # CTA pairs; parts wider than a chunk
+    (300, 256, (160, 32, 64, 96), 4, 48, 1),
+])
+def test_components_written_by_the_projection(S, m, k, parts, groups, rank, na):
+    from skyrl_tx_rocm_b200 import projections
+
+    n = groups * sum(parts)
+    x, w, a, b, s, ids = make_case(41 + m, m, k, n, rank, na, w_std=0.05)
+    _, pw = device_weight(S, w)
+    lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=pw.in_features, padded_out_features=pw.padded_out_features)
+    idd = to_dev(ids) if na > 1 else None
+    layer = projections.FusedLoRALinearW8(pw, lora, components=tuple("qkvg")[:len(parts)], group_sizes=parts, enabled=True)
+    got = layer(to_dev(x), idd)
+    want = projections.split_components(S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=idd, enabled=True), parts)
+    S.check_status()
+    assert len(got) == len(want)
+    for g, h in zip(got, want):
+        assert g.is_contiguous() and g.shape == h.shape and torch.equal(g, h)
