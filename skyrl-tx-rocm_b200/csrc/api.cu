@@ -405,8 +405,9 @@ static int run_projection(const Projection& q, cudaStream_t stream) {
     g.scatter_rows = q.scatter_rows;
   }
   if (q.ev_begin != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_begin), stream);
-  // launched programmatically behind this call's own quantiser stage: what it reads before its wait (the tile list)
-  // then comes from at least two kernels back
+  // Launched programmatically behind this call's own quantiser stage: what it touches before its wait (the tile list and
+  // the claim counter) must come from at least two kernels back.  The routing kernel clears the counter, or the quantiser
+  // with the LoRA-A projection behind it; without either the caller passes no counter (fixed stride).
   rc = launch_gemm(g, stream, !q.skip_quant && q.ev_begin == nullptr && q.ev_end == nullptr, &q.src,
                    q.split.count > 0 ? &q.split : nullptr);
   if (q.ev_end != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(q.ev_end), stream);
@@ -493,8 +494,8 @@ static int linear_forward(const SkyrlW8A8LinearArgs* a, const ColumnSplit& split
   q.out = a->out;
   q.out_stride = a->out_row_stride;
   q.status = a->status;
-  if (!rows_path) q.sched = w.sched;
-  if (!routed && !rows_path) q.zero_words = w.sched;
+  if (!rows_path && (routed || a->rank > 0)) q.sched = w.sched;
+  if (!rows_path && !routed) q.zero_words = q.sched;
   q.ev_begin = a->timing_events[0];
   q.ev_end = a->timing_events[1];
   return run_projection(q, stream);
@@ -948,9 +949,11 @@ static Projection front_projection(const SkyrlW8A8MlpArgs* a, const MlpPlan& pl)
   q.status = a->status;
   // odd and even chunks claim tiles through counter pairs of their own, so that two chunks of one block may run
   // on two streams at the same time
-  // (Without adapter ids no routing kernel runs to clear the words: a whole block's quantiser does, the chunks of a
-  // block without ids take their tiles with a fixed stride.)
-  if (pl.routed || (!pl.rows_path && !pl.chunked)) q.sched = w.sched + (pl.chunked ? (a->chunk_index & 1) * 4 : 0);
+  // (Without adapter ids no routing kernel runs to clear the words: a whole block's quantiser does, with the projection
+  // between it and the GEMM; the chunks of a block without ids, and a block without LoRA, take their tiles with a fixed
+  // stride.)
+  if (pl.routed || (!pl.rows_path && !pl.chunked && a->rank > 0))
+    q.sched = w.sched + (pl.chunked ? (a->chunk_index & 1) * 4 : 0);
   q.ev_begin = a->timing_events[0];
   q.ev_end = a->timing_events[1];
   return q;
@@ -979,7 +982,7 @@ extern "C" int skyrl_w8a8_mlp_block_sm100_v1(const SkyrlW8A8MlpArgs* a, skyrl_st
   q.zero_amax = q.row_amax;
   if (!pl.routed && !pl.rows_path && !pl.chunked) {
     if (prepared) q.sched = nullptr;  // the rows were prepared by a call of their own
-    else q.zero_words = w.sched;
+    else q.zero_words = q.sched;
   }
   if (pl.rows_path && a->prefetch_down_bytes > 0) {
     // the down weights travel to L2 while the row-wise kernels behind gate_up run

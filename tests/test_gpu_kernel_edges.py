@@ -153,3 +153,41 @@ def test_components_written_by_the_projection(S, m, k, parts, groups, rank, na):
     assert len(got) == len(want)
     for g, h in zip(got, want):
         assert g.is_contiguous() and g.shape == h.shape and torch.equal(g, h)
+
+
+@pytest.fixture
+def dirty_workspace(S):
+    """Scratch that starts as large positive int32 words: a tile-claim counter read before it is cleared claims no tile."""
+    buf = torch.full((96 << 20,), 0x5a, dtype=torch.uint8, device="cuda")
+    S.use_workspace(buf)
+    yield buf
+    S.use_workspace(None)
+
+
+@pytest.mark.parametrize("variant", [0, 1])   # the rule's choice; the single-tile kernel, which claims its tiles
+def test_projection_without_lora_on_a_dirty_workspace(S, dirty_workspace, variant):
+    m, k, n = 1000, 256, 8192                 # 256 tiles of 128 x 256: two waves
+    x, w, *_ = make_case(7, m, k, n, 8, 1, w_std=0.05)
+    q, pw = device_weight(S, w)
+    want = O.quantized_lora_linear(x, q).view(np.uint16)
+    for _ in range(3):
+        dirty_workspace.fill_(0x5a)
+        y = S.w8a8_lora_linear_f32(to_dev(x), pw, enabled=True, gemm_variant=variant)
+        np.testing.assert_array_equal(to_np(y.to(torch.bfloat16)).view(np.uint16), want)
+        dirty_workspace.fill_(0x5a)
+        np.testing.assert_array_equal(to_np(S.w8a8_frozen_linear(to_dev(x), pw, enabled=True)).view(np.uint16), want)
+    S.check_status()
+
+
+def test_block_without_lora_on_a_dirty_workspace(S, dirty_workspace):
+    m, hidden, inter = 700, 256, 4096
+    x, wgu, *_ = make_case(11, m, hidden, 2 * inter, 8, 1, w_std=0.05)
+    _, wd, *_ = make_case(13, m, inter, hidden, 8, 1, w_std=0.05)
+    (_, pgu), (_, pd) = device_weight(S, wgu), device_weight(S, wd)
+    xd = to_dev(x)
+    h = S.w8a8_rms_gate_up_lora_swiglu(xd, None, pgu, None, enabled=True)
+    want = S.w8a8_down_lora_residual(h, pd, None, residual=xd, enabled=True)
+    for variant in (0, 1):
+        dirty_workspace.fill_(0x5a)
+        assert torch.equal(S.w8a8_mlp_block(xd, None, pgu, None, pd, None, enabled=True, gemm_variant=variant), want)
+    S.check_status()
