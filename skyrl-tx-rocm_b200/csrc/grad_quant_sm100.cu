@@ -17,8 +17,8 @@ namespace skyrl {
 namespace {
 
 __global__ void __launch_bounds__(QUANT_THREADS)
-grad_quant_kernel(const __nv_bfloat16* __restrict__ dy, int64_t dy_row_stride, const float* __restrict__ col_scale,
-                  const int32_t* __restrict__ row_map, int n, int8_t* __restrict__ q1, float* __restrict__ s1,
+grad_quant_kernel(const __nv_bfloat16* dy, int64_t dy_row_stride, const float* __restrict__ col_scale,
+                  const int32_t* row_map, int n, int8_t* __restrict__ q1, float* __restrict__ s1,
                   int8_t* __restrict__ q2, float* __restrict__ s2, uint4* __restrict__ rows) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float4* g = reinterpret_cast<float4*>(smem_raw);  // n / 4 vectors
@@ -27,14 +27,14 @@ grad_quant_kernel(const __nv_bfloat16* __restrict__ dy, int64_t dy_row_stride, c
   pdl_wait();
   pdl_trigger();
   const int out_row = blockIdx.x;
-  const int64_t src_row = row_map != nullptr ? row_map[out_row] : out_row;
+  const int64_t src_row = row_map != nullptr ? __ldcg(row_map + out_row) : out_row;
   const uint4* src = reinterpret_cast<const uint4*>(dy + src_row * dy_row_stride);
   const float4* cs = reinterpret_cast<const float4*>(col_scale);
   const int nvec = n >> 3;
 
   float amax = 0.f;
   for (int v = threadIdx.x; v < nvec; v += QUANT_THREADS) {
-    const uint4 u = __ldg(src + v);
+    const uint4 u = ld_stream16(src + v);
     if (rows != nullptr) rows[static_cast<int64_t>(out_row) * nvec + v] = u;  // for the LoRA projection of the sorted rows
     const float4 c0 = __ldg(cs + 2 * v), c1 = __ldg(cs + 2 * v + 1);
     float4 a, b;

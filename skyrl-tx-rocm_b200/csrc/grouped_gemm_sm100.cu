@@ -27,13 +27,12 @@ namespace skyrl {
 // shuffles only.  Otherwise a warp takes a whole group and reads it twice.
 template <bool POW2>
 __global__ void __launch_bounds__(QUANT_THREADS)
-group_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* __restrict__ row_map, int m,
-                   int k, int group_vecs, int8_t* __restrict__ xq, float* __restrict__ sx,
-                   __nv_bfloat16* __restrict__ xn) {
+group_quant_kernel(const __nv_bfloat16* x, int64_t x_row_stride, const int32_t* row_map, int m, int k, int group_vecs,
+                   int8_t* __restrict__ xq, float* __restrict__ sx, __nv_bfloat16* __restrict__ xn) {
   pdl_wait();
   pdl_trigger();
   const int row = blockIdx.x, lane = threadIdx.x & 31;
-  const int64_t src_row = row_map != nullptr ? row_map[row] : row;
+  const int64_t src_row = row_map != nullptr ? __ldcg(row_map + row) : row;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * x_row_stride);
   uint2* dst = reinterpret_cast<uint2*>(xq + static_cast<int64_t>(row) * k);
   uint4* copy = xn != nullptr ? reinterpret_cast<uint4*>(xn + static_cast<int64_t>(row) * k) : nullptr;
@@ -58,7 +57,7 @@ group_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, co
   if (POW2) {
     for (int v0 = threadIdx.x & ~31; v0 < nvec; v0 += QUANT_THREADS) {
       const int v = v0 + lane;
-      const uint4 u = v < nvec ? __ldg(src + v) : make_uint4(0u, 0u, 0u, 0u);
+      const uint4 u = v < nvec ? ld_stream16(src + v) : make_uint4(0u, 0u, 0u, 0u);
       float a = absmax(u);
       for (int o = 1; o < group_vecs; o <<= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
       const float scale = a > 0.f ? __fdiv_rn(a, 127.0f) : 1.0f;
@@ -71,12 +70,12 @@ group_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, co
   } else {
     for (int g = threadIdx.x >> 5; g * group_vecs < nvec; g += QUANT_THREADS / 32) {
       float a = 0.f;
-      for (int i = lane; i < group_vecs; i += 32) a = fmaxf(a, absmax(__ldg(src + g * group_vecs + i)));
+      for (int i = lane; i < group_vecs; i += 32) a = fmaxf(a, absmax(ld_stream16(src + g * group_vecs + i)));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
       const float scale = a > 0.f ? __fdiv_rn(a, 127.0f) : 1.0f;
       for (int i = lane; i < group_vecs; i += 32) {
-        const uint4 u = __ldg(src + g * group_vecs + i);
+        const uint4 u = ld_stream16(src + g * group_vecs + i);
         dst[g * group_vecs + i] = codes(u, scale, quant_rcp(scale));
         if (copy != nullptr) copy[g * group_vecs + i] = u;
       }

@@ -368,10 +368,9 @@ int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* per
 // rint(x / scale) with IEEE division (skyrl/tx/kernels/quantized_lora.py:207-211).
 // ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(QUANT_THREADS)
-rms_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const __nv_bfloat16* __restrict__ delta,
-                 float eps, const int32_t* __restrict__ row_map, int k, int8_t* __restrict__ xq,
-                 float* __restrict__ sx, __nv_bfloat16* __restrict__ xn, float* __restrict__ zero_amax,
-                 int32_t* __restrict__ zero_words) {
+rms_quant_kernel(const __nv_bfloat16* x, int64_t x_row_stride, const __nv_bfloat16* __restrict__ delta, float eps,
+                 const int32_t* row_map, int k, int8_t* __restrict__ xq, float* __restrict__ sx,
+                 __nv_bfloat16* __restrict__ xn, float* __restrict__ zero_amax, int32_t* __restrict__ zero_words) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* row = reinterpret_cast<uint4*>(smem_raw);  // k / 8 vectors of 8 bf16
   __shared__ float red[QUANT_THREADS / 32];
@@ -379,7 +378,7 @@ rms_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, cons
   pdl_wait();
   pdl_trigger();
   const int out_row = blockIdx.x;
-  const int64_t src_row = row_map != nullptr ? row_map[out_row] : out_row;
+  const int64_t src_row = row_map != nullptr ? __ldcg(row_map + out_row) : out_row;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * x_row_stride);
   const int nvec = k >> 3;
   const bool norm = delta != nullptr;
@@ -388,7 +387,7 @@ rms_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, cons
 
   float ss = 0.f, amax = 0.f;
   for (int v = threadIdx.x; v < nvec; v += QUANT_THREADS) {
-    const uint4 u = __ldg(src + v);
+    const uint4 u = ld_stream16(src + v);
     row[v] = u;
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -440,21 +439,21 @@ int launch_rms_quant(const void* x, int64_t x_row_stride, const void* rms_delta,
 // vectors, HBM in -> codes out, with no shared memory and no barrier.  Same arithmetic as
 // rms_quant_kernel (scale = amax / 127 or 1, exact rint(x / scale)).
 __global__ void __launch_bounds__(256)
-quant_stream_kernel(const uint4* __restrict__ x, const float* __restrict__ row_amax, int nvec, int64_t total_vecs,
-                    uint2* __restrict__ xq, float* __restrict__ sx) {
+quant_stream_kernel(const uint4* x, const float* row_amax, int nvec, int64_t total_vecs, uint2* __restrict__ xq,
+                    float* __restrict__ sx) {
   pdl_wait();
   pdl_trigger();
   const int64_t v0 = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * 2;
   if (v0 >= total_vecs) return;
   const bool two = v0 + 1 < total_vecs;
-  const uint4 u0 = __ldg(x + v0);
-  const uint4 u1 = two ? __ldg(x + v0 + 1) : make_uint4(0u, 0u, 0u, 0u);
+  const uint4 u0 = ld_stream16(x + v0);
+  const uint4 u1 = two ? ld_stream16(x + v0 + 1) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     if (i == 1 && !two) break;
     const int64_t v = v0 + i;
     const int64_t row = v / nvec;
-    const float amax = __ldg(row_amax + row);
+    const float amax = __ldcg(row_amax + row);
     const float scale = amax > 0.f ? __fdiv_rn(amax, 127.0f) : 1.0f;
     const float rcp = quant_rcp(scale);
     if (v - row * nvec == 0) sx[row] = scale;

@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) w8a8_gemm_pair_kernel(const _
       const int n_end = min(p.n, n0 + PAIR_BN);
       const bool row_valid = r < tile.y;
       const int srow = tile.x + r;
-      const float sxr = row_valid ? __ldg(p.sx + srow) : 0.f;
+      const float sxr = row_valid ? __ldcg(p.sx + srow) : 0.f;
       const int64_t orow = row_valid ? (p.out_row_map != nullptr ? __ldg(p.out_row_map + srow) : srow) : 0;
 
       ok = __all_sync(0xffffffffu, mbar_wait(tmem_full, it & 1u, abort_flag, p.status, STATUS_TIMEOUT_EPILOGUE));
@@ -1397,7 +1397,7 @@ w8a8_gemm_pair2_kernel(const __grid_constant__ GemmParams p) {
       const uint32_t s = it & 1u, aphase = (it >> 1) & 1u;
       const bool row_valid = r < tile.y;
       const int srow = tile.x + r;
-      const float sxr = row_valid ? __ldg(p.sx + srow) : 0.f;
+      const float sxr = row_valid ? __ldcg(p.sx + srow) : 0.f;
       const int64_t orow = row_valid ? (p.out_row_map != nullptr ? __ldg(p.out_row_map + srow) : srow) : 0;
 
       ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[s], aphase, abort_flag, p.status, STATUS_TIMEOUT_EPILOGUE));
