@@ -98,7 +98,7 @@ def w8a8_lora_linear_input_grad(dy: torch.Tensor, weight_bwd: PackedW8Backward, 
         a.adapter_ids = ids.data_ptr() if ids is not None else None
         dx = torch.empty((m, k), dtype=torch.bfloat16, device=dev)
         a.dx = dx.data_ptr()
-        _with_workspace(a, dev, True)
+        _owner = _with_scratch(a, dev, True)
         _lib.check(lib.skyrl_w8a8_train_backward_sm100_v1(C.byref(a), ops._stream()), "train_backward (input gradient)")
         return dx.reshape(*dy.shape[:-1], k)
     # one plane: the int8 step of the cotangent stays visible in dx; same kernels as the forward
@@ -151,10 +151,11 @@ def _train_args(m: int, n: int, k: int, n_logical: int, rank: int, adapters: int
     return a
 
 
-def _with_workspace(a, device, backward: bool) -> None:
-    nbytes = _lib.load().skyrl_w8a8_train_workspace_bytes(a.m, a.n, a.k, a.rank, a.num_adapters, backward)
-    ws = ops._workspace(device, nbytes)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
+def _with_scratch(a, device, backward: bool) -> torch.Tensor:
+    """Gives `a` scratch of its own and returns its owner, which has to live until the call is enqueued."""
+    a.workspace_bytes = _lib.load().skyrl_w8a8_train_workspace_bytes(a.m, a.n, a.k, a.rank, a.num_adapters, backward)
+    owner, a.workspace = ops._scratch(device, a.workspace_bytes)
+    return owner
 
 
 def _mm_f32(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
@@ -251,7 +252,7 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
         a.adapter_ids = ids.data_ptr() if ids is not None else None
         a.y = y.data_ptr()
         _with_saved(a, saved)
-        _with_workspace(a, dev, False)
+        _owner = _with_scratch(a, dev, False)
         _lib.check(lib.skyrl_w8a8_train_forward_sm100_v1(C.byref(a), ops._stream()), "train_forward")
         ctx.save_for_backward(x, lora_a, lora_b, lora_scaling, ids, saved)
         ctx.weight_bwd = weight_bwd
@@ -284,7 +285,7 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
         a.dx = dx.data_ptr() if dx is not None else None
         a.da, a.db = d_a.data_ptr(), d_b.data_ptr()
         _with_saved(a, saved)
-        _with_workspace(a, dev, True)
+        _owner = _with_scratch(a, dev, True)
         _lib.check(_lib.load().skyrl_w8a8_train_backward_sm100_v1(C.byref(a), ops._stream()), "train_backward")
         d_s = None
         if ctx.needs_input_grad[3]:   # rarely wanted (alpha / r is a constant): library matmuls

@@ -310,6 +310,15 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws[off: off + nbytes]
 
 
+def _scratch(device: torch.device, nbytes: int):
+    """(owner, address) of scratch for ONE call, from torch's caching allocator: calls on several streams or threads never
+    share it, a captured graph owns what its calls were given, and it is returned when the owner goes.  For operators whose
+    scratch nothing reads after the call."""
+    owner = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
+    base = owner.data_ptr()
+    return owner, base + -base % 1024
+
+
 def use_workspace(buffer: torch.Tensor | None, device=None) -> None:
     """Make the operators of `buffer`'s device carve their scratch from `buffer` (uint8, CUDA) instead of a
     tensor of their own: a tensor-parallel stack registers a piece of peer-mapped (symmetric) memory here so
@@ -443,7 +452,7 @@ def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids
     if g_size % 32 == 0:
         out = torch.empty((m, npad), dtype=torch.bfloat16, device=dev)
         nbytes = lib.skyrl_w8a8_grouped_workspace_bytes(m, npad, k, na, g_size)
-        ws = _workspace(dev, nbytes)
+        _owner, address = _scratch(dev, nbytes)
         a = _lib.LinearArgs()
         a.struct_size = C.sizeof(_lib.LinearArgs)
         a.epilogue = EPI_LINEAR
@@ -458,7 +467,7 @@ def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids
                 a.lora_b_rows, a.lora_b_rows_rank = lora.b_rows.data_ptr(), lora.b_rows.shape[2]
         a.adapter_ids = ids.data_ptr() if ids is not None else None
         a.out, a.out_row_stride = out.data_ptr(), npad
-        a.workspace, a.workspace_bytes, a.status = ws.data_ptr(), nbytes, st.data_ptr()
+        a.workspace, a.workspace_bytes, a.status = address, nbytes, st.data_ptr()
         _lib.check(lib.skyrl_w8a8_lora_forward_grouped_sm100_v1(C.byref(a), g_size, _stream()), "w8a8_lora_forward_grouped")
         return out
     perm, tiles, num = prepare_routing(ids, m, na)

@@ -191,3 +191,60 @@ def test_block_without_lora_on_a_dirty_workspace(S, dirty_workspace):
         dirty_workspace.fill_(0x5a)
         assert torch.equal(S.w8a8_mlp_block(xd, None, pgu, None, pd, None, enabled=True, gemm_variant=variant), want)
     S.check_status()
+
+
+def _grouped_call(S, seed):
+    m, k, n, g, na = 300, 512, 256, 64, 3
+    x, w, a, b, s, ids = make_case(seed, m, k, n, 8, na, w_std=0.05)
+    pw = S.PackedW8Weight(*_packed_grouped(S, O.quantize_frozen_weight(w, group_size=g), k, n, g))
+    lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=k, padded_out_features=pw.padded_out_features)
+    xd, idd = to_dev(x), to_dev(ids)
+    return lambda: [S.w8a8_lora_linear(xd, pw, lora, adapter_ids=idd, enabled=True)]
+
+
+def _training_call(S, seed):
+    from skyrl_tx_rocm_b200 import backward as B
+
+    m, k, n, na = 2048, 1024, 1024, 3
+    x, w, a, b, s, ids = make_case(seed, m, k, n, 8, na, w_std=0.05)
+    _, pw = device_weight(S, w)
+    wb, sd, idd = B.pack_weight_backward(pw), to_dev(s), to_dev(ids)
+    xd, ad, bd = to_dev(x).requires_grad_(), to_dev(a).requires_grad_(), to_dev(b).requires_grad_()
+    dy = to_dev((np.random.default_rng(seed).standard_normal((m, n)) * 0.3).astype(np.float32).astype(x.dtype))
+
+    def call():
+        y = B.w8a8_lora_linear_trainable(xd, pw, wb, ad, bd, sd, idd)
+        return [y.detach(), *torch.autograd.grad(y, (xd, ad, bd), dy)]
+
+    return call
+
+
+@pytest.mark.parametrize("make", [_grouped_call, _training_call])
+def test_scratch_of_training_and_grouped_calls_is_their_own(S, make):
+    calls = [make(S, 3), make(S, 4)]
+    want = [c() for c in calls]
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    # a registered buffer (other ranks store into it) is neither used nor too small for them
+    registered = torch.full((1 << 20,), 0x5a, dtype=torch.uint8, device="cuda")
+    S.use_workspace(registered)
+    try:
+        for c, w in zip(calls, want):
+            assert all(torch.equal(g, h) for g, h in zip(c(), w))
+        assert int((registered != 0x5a).sum()) == 0
+    finally:
+        S.use_workspace(None)
+    del registered
+    assert torch.cuda.memory_allocated() <= before    # nothing stays behind
+    # two streams: each call's kernels overlap the other's
+    streams = [torch.cuda.Stream() for _ in calls]
+    got = [None, None]
+    torch.cuda.synchronize()
+    for _ in range(8):
+        for i, c in enumerate(calls):
+            with torch.cuda.stream(streams[i]):
+                got[i] = c()
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        assert all(torch.equal(p, q) for p, q in zip(g, w))
+    S.check_status()
