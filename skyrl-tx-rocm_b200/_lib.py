@@ -127,6 +127,7 @@ class TpExchangeArgs(C.Structure):
 SYMBOLS = {
     "skyrl_w8a8_abi_version": (C.c_int, []),
     "skyrl_w8a8_last_error": (C.c_char_p, []),
+    "skyrl_w8a8_stream_capture_id": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64)]),
     "skyrl_w8a8_bounded_wait_selftest_sm100_v1": (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p]),
     "skyrl_lora_route_sm100_v1": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,
                                             C.c_int32, C.c_void_p, C.c_void_p]),

@@ -421,6 +421,16 @@ using namespace skyrl;
 extern "C" int skyrl_w8a8_abi_version(void) { return SKYRL_W8A8_ABI_VERSION; }
 extern "C" const char* skyrl_w8a8_last_error(void) { return g_last_error; }
 
+extern "C" int skyrl_w8a8_stream_capture_id(skyrl_stream_t stream, uint64_t* id) {
+  if (id == nullptr) return fail(SKYRL_ERR_INVALID_ARGUMENT, "stream_capture_id: id is null");
+  cudaStreamCaptureStatus state = cudaStreamCaptureStatusNone;
+  unsigned long long capture = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &state, &capture);
+  if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "stream_capture_id: %s", cudaGetErrorString(e));
+  *id = state == cudaStreamCaptureStatusActive ? capture : 0;
+  return SKYRL_OK;
+}
+
 extern "C" size_t skyrl_w8a8_linear_workspace_bytes(int32_t m, int32_t n, int32_t k, int32_t num_adapters) {
   if (m <= 0 || n <= 0 || k <= 0) return 0;
   return carve_linear(nullptr, m, n, k, num_adapters).bytes;

@@ -18,6 +18,8 @@ runs in the hand-written CUDA library behind the C ABI
 from __future__ import annotations
 
 import ctypes as C
+import threading
+from collections import OrderedDict
 from dataclasses import dataclass
 
 import torch
@@ -107,6 +109,11 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
 
 def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
+
+
+def _stream_of(idx: int) -> int:
+    """Handle of device `idx`'s current stream, without the Stream object `torch.cuda.current_stream` makes (2 us a call)."""
+    return torch._C._cuda_getCurrentRawStream(idx)
 
 
 def _ptr(t):
@@ -290,22 +297,106 @@ def pack_lora(lora_a: torch.Tensor, lora_b: torch.Tensor, lora_scaling, *, in_fe
 
 
 # --------------------------------------------------------------------------- #
-# per-device scratch (torch owns the memory; the C ABI never allocates)
+# scratch (torch owns the memory; the C ABI never allocates)
 # --------------------------------------------------------------------------- #
-_workspaces: dict[int, torch.Tensor] = {}
-_pinned_workspaces: set[int] = set()
+# MLP blocks keep their scratch between calls: a call may reuse the routing of the one before, run on rows another call
+# prepared, or have its stages read back.  Every stream has a buffer of its own, so calls on two streams never share one;
+# a call that CONTINUES an earlier one (`fresh=False`) takes the buffer of this thread's last call, whatever its stream.
+# While a stream is captured the buffers come from the graph's memory pool and belong to the graph: its replays must not
+# write into memory that a later, larger call gave back.
+MAX_STREAM_WORKSPACES = 16
+_stream_workspaces: OrderedDict = OrderedDict()      # (device, stream) -> buffer, least recently used first
+_registered_workspaces: dict[int, torch.Tensor] = {}  # use_workspace()
+_last_workspaces: dict[int, torch.Tensor] = {}        # of any thread
+_replayed_workspaces: list = []                       # eager buffers that a captured call continues on: never given back
+_thread = threading.local()
 _status: dict[int, torch.Tensor] = {}
 
 
-def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+class _Capture:
+    """Buffers one thread handed out during one stream capture."""
+
+    def __init__(self, ident: int, stream: int):
+        self.ident, self.stream = ident, stream
+        self.by_stream: dict = {}
+        self.last: dict[int, torch.Tensor] = {}
+
+
+def _capture_id(stream: int) -> int:
+    ident = C.c_uint64(0)
+    _lib.check(_lib.load().skyrl_w8a8_stream_capture_id(stream, C.byref(ident)), "stream_capture_id")
+    return ident.value
+
+
+def _holds(buffer, nbytes: int) -> bool:
+    return buffer is not None and buffer.numel() >= nbytes + 1024
+
+
+def _captured_workspace(device, idx: int, stream: int, nbytes: int, fresh: bool) -> torch.Tensor:
+    ident = _capture_id(stream)
+    held = getattr(_thread, "capture", None)
+    if held is None or held.ident != ident:
+        held = _thread.capture = _Capture(ident, stream)
+    if fresh:
+        ws = held.by_stream.get((idx, stream))
+    else:
+        ws = held.last.get(idx)
+        if ws is None:   # continues a call from before the capture
+            ws = _current_workspace(idx)
+            if _holds(ws, nbytes) and all(ws is not kept for kept in _replayed_workspaces):
+                _replayed_workspaces.append(ws)
+    if not _holds(ws, nbytes):
+        ws = held.by_stream[idx, stream] = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
+    held.last[idx] = ws
+    return ws
+
+
+def _current_workspace(idx: int):
+    own = getattr(_thread, "last", {}).get(idx)
+    return own if own is not None else _last_workspaces.get(idx)
+
+
+def _eager_workspace(device, idx: int, stream: int, nbytes: int, fresh: bool) -> torch.Tensor:
+    held = getattr(_thread, "capture", None)
+    if held is not None and _capture_id(held.stream) != held.ident:
+        _thread.capture = None   # that capture is over: its buffers are the graph's alone
+    if not hasattr(_thread, "last"):
+        _thread.last = {}
+    ws = None if fresh else _current_workspace(idx)
+    if not _holds(ws, nbytes):
+        key = (idx, stream)
+        ws = _stream_workspaces.get(key)
+        if not _holds(ws, nbytes):
+            ws = _stream_workspaces[key] = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
+            while len(_stream_workspaces) > MAX_STREAM_WORKSPACES:
+                _stream_workspaces.popitem(last=False)
+        elif _thread.last.get(idx) is not ws:
+            _stream_workspaces.move_to_end(key)
+    _thread.last[idx] = _last_workspaces[idx] = ws
+    return ws
+
+
+def _workspace_buffer(device: torch.device, nbytes: int, fresh: bool = False) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    ws = _workspaces.get(idx)
-    if ws is None or ws.numel() < nbytes + 1024:
-        if idx in _pinned_workspaces:
+    ws = _registered_workspaces.get(idx)
+    if ws is not None:
+        if not _holds(ws, nbytes):
             raise SkyrlKernelError(f"the workspace registered with use_workspace() has {ws.numel()} bytes, this call needs "
                                    f"{nbytes + 1024}; register a larger one or release it with use_workspace(None)")
-        ws = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
-        _workspaces[idx] = ws
+        return ws
+    stream = _stream_of(idx)
+    if stream != 0 and torch.cuda.is_current_stream_capturing():   # the legacy default stream cannot be captured
+        return _captured_workspace(device, idx, stream, nbytes, fresh)
+    return _eager_workspace(device, idx, stream, nbytes, fresh)
+
+
+def _aligned_address(buffer: torch.Tensor) -> int:
+    base = buffer.data_ptr()
+    return base + -base % 1024
+
+
+def _workspace(device: torch.device, nbytes: int, fresh: bool = False) -> torch.Tensor:
+    ws = _workspace_buffer(device, nbytes, fresh)
     off = (-ws.data_ptr()) % 1024
     return ws[off: off + nbytes]
 
@@ -315,27 +406,32 @@ def _scratch(device: torch.device, nbytes: int):
     share it, a captured graph owns what its calls were given, and it is returned when the owner goes.  For operators whose
     scratch nothing reads after the call."""
     owner = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
-    base = owner.data_ptr()
-    return owner, base + -base % 1024
+    return owner, _aligned_address(owner)
 
 
 def use_workspace(buffer: torch.Tensor | None, device=None) -> None:
     """Make the operators of `buffer`'s device carve their scratch from `buffer` (uint8, CUDA) instead of a
-    tensor of their own: a tensor-parallel stack registers a piece of peer-mapped (symmetric) memory here so
+    memory of their own: a tensor-parallel stack registers a piece of peer-mapped (symmetric) memory here so
     that other ranks can store the rows they prepared straight into this rank's workspace.  The operators
     raise if a call needs more than the buffer holds.  `None` releases the registration."""
     if buffer is None:
         dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-        idx = dev.index if dev.index is not None else torch.cuda.current_device()
-        _pinned_workspaces.discard(idx)
-        _workspaces.pop(idx, None)
+        _drop_workspaces(dev.index if dev.index is not None else torch.cuda.current_device())
         return
     _require_cuda(buffer, "buffer")
     if buffer.dtype != torch.uint8 or buffer.ndim != 1 or not buffer.is_contiguous():
         raise TypeError("the workspace must be a contiguous one-dimensional uint8 tensor")
     idx = buffer.device.index if buffer.device.index is not None else torch.cuda.current_device()
-    _workspaces[idx] = buffer
-    _pinned_workspaces.add(idx)
+    _drop_workspaces(idx)
+    _registered_workspaces[idx] = buffer
+
+
+def _drop_workspaces(idx: int) -> None:
+    _registered_workspaces.pop(idx, None)
+    _last_workspaces.pop(idx, None)
+    getattr(_thread, "last", {}).pop(idx, None)
+    for key in [key for key in list(_stream_workspaces) if key[0] == idx]:
+        _stream_workspaces.pop(key, None)
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
@@ -548,7 +644,11 @@ def _run_linear(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids, epilog
         out = torch.empty((m, out_cols), dtype=out_dtype, device=dev)
     na = lora.num_adapters if lora is not None else 1
     nbytes = lib.skyrl_w8a8_linear_workspace_bytes(m, npad, k, na)
-    ws = _workspace(dev, nbytes)
+    if dev.index in _registered_workspaces:
+        _owner = _workspace_buffer(dev, nbytes)
+        address = _aligned_address(_owner)
+    else:
+        _owner, address = _scratch(dev, nbytes)
     st = _status_word(dev)
     a = _lib.LinearArgs()
     a.struct_size = C.sizeof(_lib.LinearArgs)
@@ -575,7 +675,7 @@ def _run_linear(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids, epilog
         a.residual_row_stride = residual.stride(0)
     a.out = out.data_ptr()
     a.out_row_stride = out_cols if outs is not None else out.stride(0)
-    a.workspace = ws.data_ptr()
+    a.workspace = address
     a.workspace_bytes = nbytes
     a.status = st.data_ptr()
     if outs is not None:
@@ -791,7 +891,7 @@ def w8a8_mlp_block(x, rms_delta, gate_up_weight: PackedW8Weight, gate_up_lora: P
     dev = x2.device
     na = gate_up_lora.num_adapters if gate_up_lora is not None else 1
     nbytes = lib.skyrl_w8a8_mlp_workspace_bytes(m, hidden, inter, na)
-    ws = _workspace(dev, nbytes)
+    ws = _workspace_buffer(dev, nbytes, fresh=not (reuse_routing or input_prepared))
     st = _status_word(dev)
     if out is None:
         out = torch.empty((m, hidden), dtype=torch.float32 if down_epilogue == EPI_PARTIAL_F32 else torch.bfloat16,
@@ -823,7 +923,7 @@ def w8a8_mlp_block(x, rms_delta, gate_up_weight: PackedW8Weight, gate_up_lora: P
             a.b_rows_rank = gate_up_lora.b_rows.shape[2]
     a.adapter_ids = ids.data_ptr() if ids is not None else None
     a.out = out.data_ptr()
-    a.workspace = ws.data_ptr()
+    a.workspace = _aligned_address(ws)
     a.workspace_bytes = nbytes
     a.status = st.data_ptr()
     if timing_events is not None:
@@ -855,15 +955,15 @@ def w8a8_mlp_block(x, rms_delta, gate_up_weight: PackedW8Weight, gate_up_lora: P
         for i, addr in enumerate(scatter[1]):
             a.tp_scatter_bases[i] = int(addr)
     if build_only:
-        return out, (a, x2, delta, ids, r2)
+        return out, (a, x2, delta, ids, r2, ws)
     if prepare_rows is not None:
         _lib.check(lib.skyrl_w8a8_mlp_tp_prepare_sm100_v1(C.byref(a), int(prepare_rows[0]), int(prepare_rows[1]),
                                                         _stream()), "w8a8_mlp_tp_prepare")
-        return out, (a, x2, delta, ids, r2)
+        return out, (a, x2, delta, ids, r2, ws)
     _lib.check(lib.skyrl_w8a8_mlp_block_sm100_v1(C.byref(a), _stream()), "w8a8_mlp_block")
     if return_call:
         # keeps the argument block (and through it the workspace layout) for the tensor-parallel finalize
-        return out, (a, x2, delta, ids, r2)
+        return out, (a, x2, delta, ids, r2, ws)
     return out.reshape(*x.shape[:-1], hidden) if out.shape[0] == m else out
 
 
@@ -982,12 +1082,13 @@ def w8a8_mlp_tp_unsort(call, sorted_rows: torch.Tensor, out: torch.Tensor):
     return out
 
 
-def w8a8_mlp_workspace_regions(m: int, hidden: int, inter: int, num_adapters: int, device):
+def w8a8_mlp_workspace_regions(m: int, hidden: int, inter: int, num_adapters: int, device, *, fresh: bool = False):
     """Views of the workspace regions a sequence-parallel gather moves, indexed by sorted row:
-    (codes int8 [m, hidden], scales fp32 [m], LoRA-A parts bf16 [m, 384])."""
+    (codes int8 [m, hidden], scales fp32 [m], LoRA-A parts bf16 [m, 384]).  Of the last block call's workspace, or, with
+    `fresh`, of the one the next call that continues no other will take on the current stream."""
     lib = _lib.load()
     na = max(int(num_adapters), 1)
-    ws = _workspace(device, lib.skyrl_w8a8_mlp_workspace_bytes(m, hidden, inter, na))
+    ws = _workspace(device, lib.skyrl_w8a8_mlp_workspace_bytes(m, hidden, inter, na), fresh=fresh)
     off = (C.c_size_t * 3)()
     _lib.check(lib.skyrl_w8a8_mlp_workspace_regions(m, hidden, inter, na, off), "w8a8_mlp_workspace_regions")
     xq = ws[off[0]: off[0] + m * hidden].view(torch.int8).view(m, hidden)

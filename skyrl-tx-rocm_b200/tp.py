@@ -331,7 +331,8 @@ class TensorParallelMLPStack:
         own, own_off, own_rows = plan["own"], plan["own_off"], plan["own_rows"]
         first = self.blocks[0]
         na = first.gate_up_lora.num_adapters if first.gate_up_lora is not None else 1
-        codes, scales, parts = ops.w8a8_mlp_workspace_regions(m, hidden, first.down_weight.in_features, na, x.device)
+        codes, scales, parts = ops.w8a8_mlp_workspace_regions(m, hidden, first.down_weight.in_features, na, x.device,
+                                                              fresh=True)
         lora = first.gate_up_lora is not None
         slab_ptrs = self._peer_slabs(x, tp) if self.peer_scatter else None
         mode = self.peer_scatter if slab_ptrs is not None else False
