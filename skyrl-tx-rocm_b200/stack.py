@@ -52,16 +52,20 @@ class MLPStack:
         return c
 
     def _buffers(self, x2):
+        if self._side is None or self._side.device != x2.device:
+            self._side = torch.cuda.Stream(device=x2.device)
+        if torch.cuda.is_current_stream_capturing():
+            # the graph's own: its replays must not write into buffers that a forward of another shape replaces
+            return [torch.empty(x2.shape, dtype=torch.bfloat16, device=x2.device) for _ in range(2)]
         key = (tuple(x2.shape), x2.device)
         if self._act is None or self._act[0] != key:
             self._act = (key, [torch.empty(x2.shape, dtype=torch.bfloat16, device=x2.device) for _ in range(2)])
-            self._side = torch.cuda.Stream(device=x2.device)
         return self._act[1]
 
     def forward(self, x, adapter_ids=None, *, out=None, timing_events=None):
         """x [..., hidden] bf16 -> the last block's output (a buffer of the stack that the next forward reuses,
-        unless `out` is given).  `timing_events[l]` = four CUDA events recorded around block l's two GEMM
-        launches (of chunk 0 when the rows are cut)."""
+        unless `out` is given; a buffer of the graph in a captured forward).  `timing_events[l]` = four CUDA events
+        recorded around block l's two GEMM launches (of chunk 0 when the rows are cut)."""
         ops._require_cuda(x, "x")
         x2 = x.reshape(-1, x.shape[-1])
         m = x2.shape[0]

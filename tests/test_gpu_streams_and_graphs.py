@@ -118,3 +118,25 @@ def test_two_captures_do_not_share_a_workspace(S):
         assert all(torch.equal(o, want) for o in outs[0])
     assert int((fill != 0x5a).sum()) == 0
     S.check_status()
+
+
+def test_a_captured_stack_owns_its_activations(S):
+    """A forward of another shape replaces the stack's buffers; the graph must not go on writing into the old ones."""
+    from skyrl_tx_rocm_b200.stack import MLPStack
+
+    x, ids, parts = _block(S, 13, 64, 1024, 512)
+    stack = MLPStack([parts] * 3, num_chunks=1)
+    want = stack(x, ids).clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = stack(x, ids)
+    stack(x[:16].contiguous(), ids[:16].contiguous())
+    torch.cuda.synchronize()
+    fill = [torch.full(x.shape, 3.0, dtype=torch.bfloat16, device="cuda") for _ in range(200)]
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert all(bool((f == 3.0).all()) for f in fill)
+    S.check_status()
