@@ -479,7 +479,10 @@ def _check_x(x: torch.Tensor, k_logical: int) -> torch.Tensor:
 
 
 def _pad_cols(x2: torch.Tensor, k: int) -> torch.Tensor:
-    if x2.shape[1] == k and x2.stride(1) == 1 and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0:
+    """Rows of k values the kernels can read where they are (a row pitch of at least k, 16-byte aligned), else a zero-padded
+    copy: broadcast rows, such as the cotangent of a sum, have a pitch of 0."""
+    if (x2.shape[1] == k and x2.stride(1) == 1 and x2.stride(0) >= k and x2.stride(0) % 8 == 0
+            and x2.data_ptr() % 16 == 0):
         return x2
     out = torch.zeros((x2.shape[0], k), dtype=x2.dtype, device=x2.device)
     out[:, : x2.shape[1]] = x2

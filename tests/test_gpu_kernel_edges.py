@@ -248,3 +248,44 @@ def test_scratch_of_training_and_grouped_calls_is_their_own(S, make):
     for g, w in zip(got, want):
         assert all(torch.equal(p, q) for p, q in zip(g, w))
     S.check_status()
+
+
+def _trainable(S, seed, m, k, n, rank, na):
+    from skyrl_tx_rocm_b200 import backward as B
+
+    x, w, a, b, s, ids = make_case(seed, m, k, n, rank, na, w_std=0.05)
+    _, pw = device_weight(S, w)
+    return B, (to_dev(x), pw, B.pack_weight_backward(pw), to_dev(a), to_dev(b), to_dev(s), to_dev(ids))
+
+
+def _gradients(B, x, pw, wb, a, b, s, ids, loss):
+    x, a, b = (t.detach().requires_grad_() for t in (x, a, b))
+    y = B.w8a8_lora_linear_trainable(x, pw, wb, a, b, s, ids)
+    return [y.detach(), *torch.autograd.grad(loss(y), (x, a, b))]
+
+
+@pytest.mark.parametrize("reduce", [lambda y: y.sum(0).float().pow(2).sum(), lambda y: y.float().sum(), lambda y: y.sum((0, 1))])
+@pytest.mark.parametrize("m", [1, 40, 300])
+def test_broadcast_cotangents(S, m, reduce):
+    """The cotangent of a sum over rows has a row stride of 0 (and of 0 along the columns of a full sum)."""
+    B, (x, pw, wb, a, b, s, ids) = _trainable(S, 17, m, 256, 96, 8, 3)
+    got = _gradients(B, x, pw, wb, a, b, s, ids, reduce)
+
+    def dense(y):   # the same value with a cotangent that is stored densely
+        return (y * torch.autograd.grad(reduce(y), y, retain_graph=True)[0].contiguous()).sum()
+
+    want = _gradients(B, x, pw, wb, a, b, s, ids, dense)
+    S.check_status()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("m", [5, 200])
+def test_broadcast_rows_and_residuals(S, m):
+    x, w, a, b, s, ids = make_case(19, m, 256, 96, 8, 3, w_std=0.05)
+    _, pw = device_weight(S, w)
+    lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=256, padded_out_features=96)
+    xe, re, idd = to_dev(x)[:1].expand(m, -1), to_dev(x)[:1, :96].expand(m, -1), to_dev(ids)
+    got = S.w8a8_down_lora_residual(xe, pw, lora, residual=re, adapter_ids=idd, enabled=True)
+    want = S.w8a8_down_lora_residual(xe.contiguous(), pw, lora, residual=re.contiguous(), adapter_ids=idd, enabled=True)
+    S.check_status()
+    assert torch.equal(got, want)
