@@ -317,7 +317,13 @@ def _tables(lora_a, lora_b, lora_scaling, k: int, n: int):
         scaling = scaling.to(device=lora_a.device, dtype=torch.float32)
     if scaling.numel() != na:
         raise ValueError(f"lora_scaling must have {na} entries, got {scaling.numel()}")
-    return lora_a.detach().contiguous(), lora_b.detach().contiguous(), scaling.contiguous()
+    return _dense(lora_a.detach()), _dense(lora_b.detach()), scaling.contiguous()
+
+
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and 16-byte aligned, as tensor maps need it: a table may be a view into a flat parameter buffer."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
 def _with_saved(a, saved: torch.Tensor) -> None:

@@ -289,3 +289,22 @@ def test_broadcast_rows_and_residuals(S, m):
     want = S.w8a8_down_lora_residual(xe.contiguous(), pw, lora, residual=re.contiguous(), adapter_ids=idd, enabled=True)
     S.check_status()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("offset", [1, 4])   # elements: 2 and 8 bytes past a 16-byte boundary
+def test_training_tables_inside_a_flat_parameter_buffer(S, offset):
+    B, (x, pw, wb, a, b, s, ids) = _trainable(S, 23, 150, 256, 96, 8, 3)
+    dy = to_dev((np.random.default_rng(1).standard_normal((150, 96)) * 0.3).astype(np.float32)).to(torch.bfloat16)
+
+    def flat(t):
+        buf = torch.empty(t.numel() + offset, dtype=t.dtype, device="cuda")
+        view = buf[offset:].view(t.shape)
+        view.copy_(t)
+        assert view.is_contiguous() and view.data_ptr() % 16
+        return view
+
+    loss = lambda y: (y * dy).sum()
+    want = _gradients(B, x, pw, wb, a, b, s, ids, loss)
+    got = _gradients(B, x, pw, wb, flat(a), flat(b), s, ids, loss)
+    S.check_status()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
