@@ -243,7 +243,7 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
             raise ValueError("adapter_ids is required when the LoRA tables hold more than one adapter")
         ids = ops._check_ids(adapter_ids, m, None)
         lib = _lib.load()
-        saved = torch.empty(lib.skyrl_w8a8_train_saved_bytes(m, na) + 1024, dtype=torch.uint8, device=dev)
+        saved = torch.empty(lib.skyrl_w8a8_train_saved_bytes(m, na), dtype=torch.uint8, device=dev)
         y = torch.empty((m, npad), dtype=torch.bfloat16, device=dev)
         a = _train_args(m, npad, k, n, rank, na, ops._status_word(dev))
         a.x, a.x_row_stride = x2.data_ptr(), x2.stride(0)
@@ -284,7 +284,7 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
         a.bwd_b, a.bwd_b_slots = table_b.data_ptr(), table_b.shape[2]
         a.dx = dx.data_ptr() if dx is not None else None
         a.da, a.db = d_a.data_ptr(), d_b.data_ptr()
-        _with_saved(a, saved)
+        saved = _with_saved(a, saved)
         _owner = _with_scratch(a, dev, True)
         _lib.check(_lib.load().skyrl_w8a8_train_backward_sm100_v1(C.byref(a), ops._stream()), "train_backward")
         d_s = None
@@ -326,10 +326,13 @@ def _dense(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
-def _with_saved(a, saved: torch.Tensor) -> None:
-    base = saved.data_ptr()
-    off = -base % 1024
-    a.saved, a.saved_bytes = base + off, saved.numel() - off
+def _with_saved(a, saved: torch.Tensor) -> torch.Tensor:
+    """Points `a` at the buffer the forward keeps.  Its layout starts at its first byte: between the passes it may have been
+    moved (hooks on saved tensors take it to the host and back).  Returns the tensor that has to live until the call is
+    enqueued."""
+    saved = _dense(saved)
+    a.saved, a.saved_bytes = saved.data_ptr(), saved.numel()
+    return saved
 
 
 def w8a8_lora_linear_trainable(x, weight, weight_bwd: PackedW8Backward, lora_a, lora_b, lora_scaling, adapter_ids=None):

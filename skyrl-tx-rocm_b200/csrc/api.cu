@@ -644,6 +644,15 @@ static TrainSaved carve_train_saved(void* base, int m, int num_adapters) {
   return s;
 }
 
+// What a forward keeps may lie elsewhere by the time of the backward (a host that moves activations out and back), so it
+// needs no more than the 16 bytes of its tensor map and its vector loads.
+static int check_saved(const SkyrlW8A8TrainArgs* a, size_t need, const char* who) {
+  if (a->saved == nullptr || !aligned16(a->saved))
+    return fail(SKYRL_ERR_WORKSPACE, "%s: saved must be non-null and 16-byte aligned", who);
+  if (a->saved_bytes < need) return fail(SKYRL_ERR_WORKSPACE, "%s: saved has %zu bytes, %zu needed", who, a->saved_bytes, need);
+  return SKYRL_OK;
+}
+
 struct TrainWs {
   int32_t* sched;
   int8_t* xq;        // forward
@@ -718,7 +727,7 @@ extern "C" int skyrl_w8a8_train_forward_sm100_v1(const SkyrlW8A8TrainArgs* a, sk
   const int na = a->num_adapters;
   const TrainSaved sv = carve_train_saved(a->saved, a->m, na);
   const TrainWs w = carve_train(a->workspace, a->m, a->n, a->k, a->rank, na, false);
-  if ((rc = check_ws(a->saved, a->saved_bytes, sv.bytes, "train_forward (saved)"))) return rc;
+  if ((rc = check_saved(a, sv.bytes, "train_forward"))) return rc;
   if ((rc = check_ws(a->workspace, a->workspace_bytes, w.bytes, "train_forward"))) return rc;
   const bool routed = a->adapter_ids != nullptr;
   if ((rc = launch_train_tables(a->lora_a, a->lora_b, na, a->k, a->n_logical, a->n, a->rank, w.at, w.bt, stream))) return rc;
@@ -776,7 +785,7 @@ extern "C" int skyrl_w8a8_train_backward_sm100_v1(const SkyrlW8A8TrainArgs* a, s
   const bool routed = lora && a->adapter_ids != nullptr;
   if (grads) {
     sv = carve_train_saved(a->saved, a->m, na);
-    if ((rc = check_ws(a->saved, a->saved_bytes, sv.bytes, "train_backward (saved)"))) return rc;
+    if ((rc = check_saved(a, sv.bytes, "train_backward"))) return rc;
   } else if (routed && (rc = launch_route_dense(a->adapter_ids, a->m, na, sv.route.perm, sv.route.tiles, sv.route.seg_mask,
                                                 sv.route.seg_adapter, a->status, stream, nullptr, 0, true, sv.adapter_start))) {
     return rc;

@@ -308,3 +308,26 @@ def test_training_tables_inside_a_flat_parameter_buffer(S, offset):
     got = _gradients(B, x, pw, wb, flat(a), flat(b), s, ids, loss)
     S.check_status()
     assert all(torch.equal(g, w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("m", [40, 300])
+@pytest.mark.parametrize("offset", [16, 512, 1008])
+def test_saved_tensors_may_move_between_the_passes(S, m, offset):
+    """Hooks on saved tensors (activations kept on the host, a memory pool of the trainer) give back copies at other addresses."""
+    B, (x, pw, wb, a, b, s, ids) = _trainable(S, 29, m, 256, 96, 8, 3)
+    dy = to_dev((np.random.default_rng(2).standard_normal((m, 96)) * 0.3).astype(np.float32)).to(torch.bfloat16)
+    loss = lambda y: (y * dy).sum()
+    want = _gradients(B, x, pw, wb, a, b, s, ids, loss)
+
+    def moved(t):
+        nbytes = t.numel() * t.element_size()
+        buf = torch.full((nbytes + 2048,), 0x33, dtype=torch.uint8, device="cuda")
+        at = -buf.data_ptr() % 1024 + offset
+        piece = buf[at:at + nbytes].view(t.dtype).view(t.shape)
+        piece.copy_(t)
+        return piece
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: moved(t.cuda())):
+        got = _gradients(B, x, pw, wb, a, b, s, ids, loss)
+    S.check_status()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
