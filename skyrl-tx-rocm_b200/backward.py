@@ -235,7 +235,8 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
         if w.group_size:
             raise ops.SkyrlKernelError("the backward path takes per-output-channel scales (one group over K)")
         k, npad, n = w.in_features, w.padded_out_features, w.out_features
-        x2 = ops._pad_cols(ops._check_x(x, weight_bwd.in_features), k)
+        k_logical = weight.original_in_features if isinstance(weight, ops.GroupQuantizedWeight) else k
+        x2 = ops._pad_cols(ops._check_x(x, k_logical), k)
         m, dev = x2.shape[0], x2.device
         a3, b3, scaling = _tables(lora_a, lora_b, lora_scaling, k, n)
         na, _, rank = a3.shape
@@ -291,12 +292,14 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
         if ctx.needs_input_grad[3]:   # rarely wanted (alpha / r is a constant): library matmuls
             d_s = lora_parameter_grads(x.detach(), dy.contiguous(), lora_a.detach(), lora_b.detach(), lora_scaling.detach(), ids)[2]
             d_s = d_s.reshape(lora_scaling.shape).to(lora_scaling.dtype)
-        return (dx.reshape(x.shape) if dx is not None else None, d_a.reshape(lora_a.shape), d_b.reshape(lora_b.shape), d_s,
-                None, None, None)
+        if dx is not None:
+            dx = dx[:, :x.shape[-1]].reshape(x.shape)
+        return (dx, d_a[:, :lora_a.shape[-2]].reshape(lora_a.shape), d_b.reshape(lora_b.shape), d_s, None, None, None)
 
 
 def _tables(lora_a, lora_b, lora_scaling, k: int, n: int):
-    """LoRA tables in the reference's layout (one adapter as matrices, or a stack) as contiguous [A, K, r], [A, r, N], [A]."""
+    """LoRA tables in the reference's layout (one adapter as matrices, or a stack) as contiguous [A, K, r], [A, r, N], [A].
+    K is the packed weight's, a multiple of 16: shorter tables are padded with zeros."""
     ops._require_cuda(lora_a, "lora_a")
     ops._require_cuda(lora_b, "lora_b")
     if lora_a.dtype != torch.bfloat16 or lora_b.dtype != torch.bfloat16:
@@ -308,7 +311,7 @@ def _tables(lora_a, lora_b, lora_scaling, k: int, n: int):
     na, ka, r = lora_a.shape
     if lora_b.shape[:2] != (na, r):
         raise ValueError(f"incompatible LoRA shapes: A={tuple(lora_a.shape)}, B={tuple(lora_b.shape)}")
-    if ka != k or lora_b.shape[2] != n:
+    if not ka <= k < ka + 16 or lora_b.shape[2] != n:
         raise ValueError(f"LoRA tables of {ka} and {lora_b.shape[2]} features do not match the weight's {k} and {n}")
     if r > ops.MAX_LORA_RANK:
         raise ValueError(f"LoRA rank must not exceed {ops.MAX_LORA_RANK}, got {r}")
@@ -317,7 +320,10 @@ def _tables(lora_a, lora_b, lora_scaling, k: int, n: int):
         scaling = scaling.to(device=lora_a.device, dtype=torch.float32)
     if scaling.numel() != na:
         raise ValueError(f"lora_scaling must have {na} entries, got {scaling.numel()}")
-    return _dense(lora_a.detach()), _dense(lora_b.detach()), scaling.contiguous()
+    lora_a = lora_a.detach()
+    if ka != k:
+        lora_a = torch.nn.functional.pad(lora_a, (0, 0, 0, k - ka))
+    return _dense(lora_a), _dense(lora_b.detach()), scaling.contiguous()
 
 
 def _dense(t: torch.Tensor) -> torch.Tensor:

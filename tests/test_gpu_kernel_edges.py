@@ -331,3 +331,24 @@ def test_saved_tensors_may_move_between_the_passes(S, m, offset):
         got = _gradients(B, x, pw, wb, a, b, s, ids, loss)
     S.check_status()
     assert all(torch.equal(g, w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("k", [50, 61, 64, 95])   # packed as 64, 64, 64 and 96 values of K
+def test_training_on_reference_storage_of_any_k(S, k):
+    from skyrl_tx_rocm_b200 import backward as B
+
+    m, n, na = 150, 96, 3
+    x, w, a, b, s, ids = make_case(37 + k, m, k, n, 8, na, w_std=0.05)
+    q = O.quantize_frozen_weight(w, group_size=k + k % 2)
+    stored = S.GroupQuantizedWeight(to_dev(q.codes), to_dev(q.scales), q.original_in_features, q.padded_in_features, 8, q.group_size)
+    dy = (np.random.default_rng(k).standard_normal((m, n)) * 0.3).astype(np.float32).astype(x.dtype)
+    for x_grad in (False, True):
+        xd, ad, bd = to_dev(x).requires_grad_(x_grad), to_dev(a).requires_grad_(), to_dev(b).requires_grad_()
+        y = B.w8a8_lora_linear_trainable(xd, stored, B.pack_weight_backward(stored), ad, bd, to_dev(s), to_dev(ids))
+        y.backward(to_dev(dy))
+        S.check_status()
+        assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), f"y of K {k}")
+        dx, da, db, _ = O.quantized_lora_linear_vjp(x, q, a, b, s, dy, ids)
+        assert O.relative_l2(to_np(ad.grad), da) < 2.0 ** -9 and O.relative_l2(to_np(bd.grad), db) < 2.0 ** -9
+        if x_grad:
+            assert O.relative_l2(to_np(xd.grad), dx) < 4e-3
