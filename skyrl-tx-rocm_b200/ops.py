@@ -550,6 +550,7 @@ def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids
     st = _status_word(dev)
     if g_size % 32 == 0:
         out = torch.empty((m, npad), dtype=torch.bfloat16, device=dev)
+        sw = weight.sw.contiguous()   # the kernel takes the scales of all groups in one piece
         nbytes = lib.skyrl_w8a8_grouped_workspace_bytes(m, npad, k, na, g_size)
         _owner, address = _scratch(dev, nbytes)
         a = _lib.LinearArgs()
@@ -558,7 +559,7 @@ def _run_linear_grouped(x2, weight: PackedW8Weight, lora: PackedLoRA | None, ids
         a.m, a.n, a.k = m, npad, k
         a.rank, a.num_adapters = (lora.rank if lora is not None else 0), na
         a.x, a.x_row_stride = x2.data_ptr(), x2.stride(0)
-        a.wq, a.sw = weight.wq.data_ptr(), weight.sw.data_ptr()
+        a.wq, a.sw = weight.wq.data_ptr(), sw.data_ptr()
         if lora is not None:
             a.lora_a_packed, a.lora_b_packed = lora.a.data_ptr(), lora.b.data_ptr()
             a.lora_scaling = lora.scaling.data_ptr()

@@ -352,3 +352,15 @@ def test_training_on_reference_storage_of_any_k(S, k):
         assert O.relative_l2(to_np(ad.grad), da) < 2.0 ** -9 and O.relative_l2(to_np(bd.grad), db) < 2.0 ** -9
         if x_grad:
             assert O.relative_l2(to_np(xd.grad), dx) < 4e-3
+
+
+def test_grouped_scales_with_a_row_pitch(S):
+    m, k, n, g = 200, 256, 96, 64
+    x, w, *_ = make_case(43, m, k, n, 8, 1, w_std=0.05)
+    q = O.quantize_frozen_weight(w, group_size=g)
+    wq, sw, *rest = _packed_grouped(S, q, k, n, g)
+    wide = torch.full((sw.shape[0], sw.shape[1] + 32), 7.0, device="cuda")   # the scales are columns of a wider table
+    wide[:, :sw.shape[1]] = sw
+    y = S.w8a8_frozen_linear(to_dev(x), S.PackedW8Weight(wq, wide[:, :sw.shape[1]], *rest), enabled=True)
+    S.check_status()
+    np.testing.assert_array_equal(to_np(y).view(np.uint16), O.quantized_lora_linear(x, q).view(np.uint16))
