@@ -884,8 +884,7 @@ def w8a8_mlp_block(x, rms_delta, gate_up_weight: PackedW8Weight, gate_up_lora: P
         raise ValueError("w8a8_mlp_block needs feature sizes that are multiples of 32")
     if down_weight.in_features != inter or down_weight.out_features != hidden:
         raise ValueError("down weight does not match gate_up weight")
-    x2 = _check_x(x, hidden)
-    x2 = _pad_cols(x2, hidden)
+    x2 = _pad_cols(_check_x(x, hidden).contiguous(), hidden)   # the block's argument block has no row strides
     m = x2.shape[0]
     if (gate_up_lora is None) != (down_lora is None):
         raise ValueError("give LoRA tables for both projections or for neither")
@@ -911,7 +910,7 @@ def w8a8_mlp_block(x, rms_delta, gate_up_weight: PackedW8Weight, gate_up_lora: P
     a.rms_delta = delta.data_ptr() if delta is not None else None
     r2 = None
     if residual is not None:
-        r2 = _pad_cols(residual.reshape(-1, residual.shape[-1]), hidden)
+        r2 = _pad_cols(residual.reshape(-1, residual.shape[-1]).contiguous(), hidden)
         a.residual = r2.data_ptr()
     a.gu_wq, a.gu_sw = gate_up_weight.wq.data_ptr(), gate_up_weight.sw.data_ptr()
     a.dn_wq, a.dn_sw = down_weight.wq.data_ptr(), down_weight.sw.data_ptr()

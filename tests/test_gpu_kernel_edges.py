@@ -364,3 +364,18 @@ def test_grouped_scales_with_a_row_pitch(S):
     y = S.w8a8_frozen_linear(to_dev(x), S.PackedW8Weight(wq, wide[:, :sw.shape[1]], *rest), enabled=True)
     S.check_status()
     np.testing.assert_array_equal(to_np(y).view(np.uint16), O.quantized_lora_linear(x, q).view(np.uint16))
+
+
+@pytest.mark.parametrize("m", [40, 300])
+def test_block_on_rows_of_a_wider_matrix(S, m):
+    hidden, inter = 256, 512
+    x, wgu, *_ = make_case(47, m, hidden, 2 * inter, 8, 1, w_std=0.05)
+    (_, pgu), (_, pd) = device_weight(S, wgu), device_weight(S, make_case(48, m, inter, hidden, 8, 1, w_std=0.05)[1])
+    xd, rd = to_dev(x), to_dev(make_case(49, m, hidden, 32, 8, 1)[0])
+    wide = torch.cat([xd, rd, xd], dim=1)
+    xs, rs = wide[:, :hidden], wide[:, hidden:2 * hidden]
+    assert not xs.is_contiguous() and torch.equal(xs, xd) and torch.equal(rs, rd)
+    want = S.w8a8_mlp_block(xd, None, pgu, None, pd, None, residual=rd, enabled=True)
+    got = S.w8a8_mlp_block(xs, None, pgu, None, pd, None, residual=rs, enabled=True)
+    S.check_status()
+    assert torch.equal(got, want)
