@@ -1694,13 +1694,14 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
   // stores from registers, which NVLink carries poorly).
   const bool wide = !rows && k_splits == 1 && a.scatter_rows == 0 && a.n >= 256;
   const bool big = wide && bn_eff == 256 && static_cast<int64_t>(mt_est) * ((a.n + 255) / 256) >= 4 * sms;
-  bool pair2 = wide && a.cta_limit <= 0 && mt_est >= 2 && (a.epilogue != SKYRL_EPI_ACC_I32 || big) &&
+  const bool pair_fits = wide && a.cta_limit <= 0 && mt_est >= 2;
+  bool pair2 = pair_fits && (a.epilogue != SKYRL_EPI_ACC_I32 || big) &&
                pair_is_faster(mt_est, a.n, kblocks_of(a.k), bn_eff, sms, lora ? a.rank : 0, a.num_adapters);
   bool paired = big && kblocks_of(a.k) >= 64 && a.cta_limit > 0;
   const int forced = a.variant & 3;
   if (forced == SKYRL_GEMM_VARIANT_SINGLE) paired = pair2 = false;
   if (forced == SKYRL_GEMM_VARIANT_TWO_TILES) paired = big, pair2 = false;
-  if (forced == SKYRL_GEMM_VARIANT_CTA_PAIR) pair2 = big && a.cta_limit <= 0, paired = paired && !pair2;
+  if (forced == SKYRL_GEMM_VARIANT_CTA_PAIR) pair2 = pair_fits, paired = paired && !pair2;
   if (pair2) bn_eff = PAIR2_BN;
   if (split != nullptr) {
     if (a.epilogue != SKYRL_EPI_LINEAR || rows) return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: split columns need the linear epilogue");

@@ -114,20 +114,27 @@ def test_training_step_against_the_oracle(S, m, k, n, rank, na):
     (900, 256, 4160, 0, 1),         # fewer K blocks than pipeline stages; a tile of four rows, a column tile of 64
     (773, 2048, 4608, 8, 1),        # an odd number of M tiles: the last pair has one
     (897, 4096, 4128, 16, 3),       # a tile of one row; adapters that change inside a pair
+    (129, 512, 256, 8, 2),          # the smallest problem the pair takes: one row in its second tile
+    (300, 1024, 1056, 64, 200),     # an adapter per row: many rounds of LoRA operands in a pair
 ])
 def test_cta_pairs_below_four_waves(S, m, k, n, rank, na):
     x, w, a, b, s, ids = make_case(77 + m, m, k, n, max(rank, 1), na, w_std=0.05)
     q, pw = device_weight(S, w)
     if rank == 0:
-        y = S.w8a8_frozen_linear(to_dev(x), pw, enabled=True)
-        np.testing.assert_array_equal(to_np(y).view(np.uint16), O.quantized_lora_linear(x, q).view(np.uint16))
+        want = O.quantized_lora_linear(x, q).view(np.uint16)
+        np.testing.assert_array_equal(to_np(S.w8a8_frozen_linear(to_dev(x), pw, enabled=True)).view(np.uint16), want)
+        for variant in (S.GEMM_VARIANT_SINGLE, S.GEMM_VARIANT_CTA_PAIR):
+            y = S.w8a8_lora_linear_f32(to_dev(x), pw, enabled=True, gemm_variant=variant)
+            np.testing.assert_array_equal(to_np(y.to(torch.bfloat16)).view(np.uint16), want)
         return
     lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=pw.in_features,
                        padded_out_features=pw.padded_out_features)
-    y = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids) if na > 1 else None, enabled=True)
-    one = S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids) if na > 1 else None, enabled=True, gemm_variant=1)
+    # the rule's choice, and both kernels whatever the rule picks
+    y, one, pair = [S.w8a8_lora_linear(to_dev(x), pw, lora, adapter_ids=to_dev(ids) if na > 1 else None, enabled=True,
+                                       gemm_variant=v)
+                    for v in (S.GEMM_VARIANT_AUTO, S.GEMM_VARIANT_SINGLE, S.GEMM_VARIANT_CTA_PAIR)]
     S.check_status()
-    assert torch.equal(y, one)
+    assert torch.equal(pair, one) and torch.equal(y, one)
     assert_one_step(to_np(y), O.quantized_lora_linear(x, q, a, b, s, ids), what=f"{m} rows")
 
 
