@@ -386,3 +386,52 @@ def test_block_on_rows_of_a_wider_matrix(S, m):
     got = S.w8a8_mlp_block(xs, None, pgu, None, pd, None, residual=rs, enabled=True)
     S.check_status()
     assert torch.equal(got, want)
+
+
+def test_a_second_backward_over_the_same_graph(S):
+    B, (x, pw, wb, a, b, s, ids) = _trainable(S, 53, 300, 256, 96, 8, 3)
+    x, a, b = (t.requires_grad_() for t in (x, a, b))
+    y = B.w8a8_lora_linear_trainable(x, pw, wb, a, b, s, ids)
+    dy = torch.randn(y.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).to(torch.bfloat16)
+    first = torch.autograd.grad(y, (x, a, b), dy, retain_graph=True)
+    B.w8a8_lora_linear_trainable(x, pw, wb, a, b, s, ids.flip(0).contiguous())   # another forward in between
+    second = torch.autograd.grad(y, (x, a, b), dy)
+    S.check_status()
+    assert all(torch.equal(f, g) for f, g in zip(first, second))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("m", [40, 200, 700])
+def test_non_finite_rows_stay_with_their_adapter(S, m, bad):
+    """Rows, tables and scaling of one adapter go bad; in the tiles it shares every other row keeps its bits."""
+    B, (x, pw, wb, a, b, s, ids) = _trainable(S, 59 + m, m, 256, 512, 16, 4)
+    dy = torch.randn((m, 512), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).to(torch.bfloat16)
+    hit = ids == 1
+    x2, a2, b2, s2, dy2 = x.clone(), a.clone(), b.clone(), s.clone(), dy.clone()
+    x2[hit, 3], a2[1, 5], b2[1, 2], s2[1], dy2[hit, 7] = bad, bad, bad, bad, bad
+    pack = lambda a, b, s: S.pack_lora(a, b, s, in_features=pw.in_features, padded_out_features=pw.padded_out_features)
+    want = S.w8a8_lora_linear(x, pw, pack(a, b, s), adapter_ids=ids, enabled=True)
+    got = S.w8a8_lora_linear(x2, pw, pack(a2, b2, s2), adapter_ids=ids, enabled=True)
+    assert torch.equal(got[~hit], want[~hit]) and bool(torch.isnan(got[hit]).any())
+    clean = _gradients(B, x, pw, wb, a, b, s, ids, lambda y: (y * dy).sum())
+    dirty = _gradients(B, x2, pw, wb, a2, b2, s2, ids, lambda y: (y * dy2).sum())
+    S.check_status()
+    for c, d in zip(clean[:2], dirty[:2]):     # y, dx
+        assert torch.equal(c[~hit], d[~hit])
+    others = torch.tensor([0, 2, 3], device="cuda")
+    for c, d in zip(clean[2:], dirty[2:]):     # dA, dB
+        assert torch.equal(c[others], d[others]) and not bool(torch.isfinite(d[1]).all())
+
+
+def test_non_finite_rows_of_a_group_scale_linear_stay_with_their_adapter(S):
+    for m in (100, 300):
+        x, w, a, b, s, ids = make_case(61 + m, m, 256, 96, 16, 4, w_std=0.05)
+        pw = S.PackedW8Weight(*_packed_grouped(S, O.quantize_frozen_weight(w, group_size=64), 256, 96, 64))
+        lora = S.pack_lora(to_dev(a), to_dev(b), to_dev(s), in_features=256, padded_out_features=96)
+        xd, idd = to_dev(x), to_dev(ids)
+        want = S.w8a8_lora_linear(xd, pw, lora, adapter_ids=idd, enabled=True)
+        hit = idd == 2
+        xd[hit, 9] = float("nan")
+        got = S.w8a8_lora_linear(xd, pw, lora, adapter_ids=idd, enabled=True)
+        S.check_status()
+        assert torch.equal(got[~hit], want[~hit])
