@@ -83,10 +83,9 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, int bytes, bool (&done)[MA
 #endif
 
 // kernel launchers implemented in the .cu files
-// `zero_words` (nullable): `zero_count` int32 words the routing kernel clears (the workspace's tile-claim counters).
 int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* num_tiles,
-                 int max_tiles, int32_t* status, cudaStream_t stream, int chunk_rows = 0, int chunk_cap = 0,
-                 int32_t* zero_words = nullptr, int zero_count = 0);
+                 int max_tiles, int32_t* status, cudaStream_t stream);
+// `zero_words` (nullable): `zero_count` int32 words the kernel clears (the workspace's tile-claim counters).
 int launch_route_dense(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* seg_mask,
                        int32_t* seg_adapter, int32_t* status, cudaStream_t stream, int32_t* zero_words, int zero_count,
                        bool always_sort = false, int32_t* adapter_start = nullptr);

@@ -1,7 +1,9 @@
 // HBM-bound front-end kernels of the W8A8 multi-LoRA path:
-//   * route_kernel ....... stable counting sort of token rows by adapter id and
-//                          the list of 128-row M tiles (at most two adapters per tile)
+//   * route_dense_kernel . stable counting sort of token rows by adapter id, the 128-row M tiles and the
+//                          row masks of their adapters (the operators)
+//   * route_kernel ....... the same order with tiles of at most two adapters (the public routing entry point)
 //   * rms_quant_kernel ... optional RMSNorm(1 + delta), per-token absmax, int8 codes
+//   * quant_stream_kernel  int8 codes of rows whose absmax the producing GEMM collected
 //   * pack kernels ....... one-time layout changes of weights and LoRA tables
 #include "common.cuh"
 #include "ptx_sm100.cuh"
@@ -10,47 +12,30 @@
 namespace skyrl {
 
 // ----------------------------------------------------------------------------
-// Routing.  One CTA; the histogram is parallel, the stable scatter is done by a
+// Routing entry point.  One CTA; the histogram is parallel, the stable scatter is done by a
 // single warp with match_any so that rows of an adapter keep their order
 // (the reference's argsort is used the same way: skyrl/tx/layers/util.py:82-87).
 // ----------------------------------------------------------------------------
 constexpr int ROUTE_THREADS = 1024;
 constexpr int ROUTE_MAX_ADAPTERS = 4096;
 
-// Tile lists.  With chunk_rows == 0 there is one list at `tiles` and its length at num_tiles[0].
-// With chunk_rows > 0 (a multiple of 128) the sorted row space is cut at multiples of chunk_rows and
-// chunk c gets its own list at tiles + 4 * c * chunk_cap with its length at num_tiles[c]; no tile
-// crosses a chunk boundary, so the chunks of a block can be computed and reduced independently.
 __global__ void __launch_bounds__(ROUTE_THREADS)
 route_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int32_t* __restrict__ perm,
-             int32_t* __restrict__ tiles, int32_t* __restrict__ num_tiles, int max_tiles, int chunk_rows,
-             int chunk_cap, int32_t* status, int32_t* __restrict__ zero_words, int zero_count) {
+             int32_t* __restrict__ tiles, int32_t* __restrict__ num_tiles, int max_tiles, int32_t* status) {
   __shared__ int counts[ROUTE_MAX_ADAPTERS];
   __shared__ int cursor[ROUTE_MAX_ADAPTERS];
   const int tid = threadIdx.x;
-  if (zero_words != nullptr && tid < zero_count) zero_words[tid] = 0;
-  const int num_chunks = chunk_rows > 0 ? (m + chunk_rows - 1) / chunk_rows : 1;
-  const int cap = chunk_rows > 0 ? chunk_cap : max_tiles;
-  const int span = chunk_rows > 0 ? chunk_rows : m;
 
   if (ids == nullptr) {
     for (int i = tid; i < m; i += ROUTE_THREADS) perm[i] = i;
-    const int per_chunk = (span + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS;
-    if (per_chunk > cap) {
-      if (tid == 0) atomicCAS(status, 0, STATUS_TILE_OVERFLOW);
-      for (int c = tid; c < num_chunks; c += ROUTE_THREADS) num_tiles[c] = 0;
-      return;
-    }
     const int nt = (m + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS;
-    for (int t = tid; t < nt; t += ROUTE_THREADS) {
-      const int r0 = t * SKYRL_TILE_ROWS;
-      const int c = r0 / span;  // chunk_rows is a multiple of the tile height, so tiles never straddle
-      const int slot = c * cap + (r0 - c * span) / SKYRL_TILE_ROWS;
-      reinterpret_cast<int4*>(tiles)[slot] = make_int4(r0, min(SKYRL_TILE_ROWS, m - r0), 0, 0);
+    if (tid == 0) {
+      num_tiles[0] = nt <= max_tiles ? nt : 0;
+      if (nt > max_tiles) atomicCAS(status, 0, STATUS_TILE_OVERFLOW);
     }
-    for (int c = tid; c < num_chunks; c += ROUTE_THREADS) {
-      const int rows = min(span, m - c * span);
-      num_tiles[c] = (rows + SKYRL_TILE_ROWS - 1) / SKYRL_TILE_ROWS;
+    for (int t = tid; t < nt && nt <= max_tiles; t += ROUTE_THREADS) {
+      const int r0 = t * SKYRL_TILE_ROWS;
+      reinterpret_cast<int4*>(tiles)[t] = make_int4(r0, min(SKYRL_TILE_ROWS, m - r0), 0, 0);
     }
     return;
   }
@@ -74,43 +59,27 @@ route_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int32_t* 
     }
     // Greedy packing of the sorted rows into tiles of up to 128 rows and at most two adapters: where an
     // adapter's run ends inside a tile, the tile is filled up with rows of the next adapter.
-    int chunk = 0, in_chunk = 0, pos = 0, a = 0;
-    bool overflow = false;
+    int count = 0, pos = 0, a = 0;
     while (a < num_adapters && counts[a] == 0) ++a;
     while (pos < m && a < num_adapters) {
-      while (pos >= (chunk + 1) * span) {  // close the chunks this row has passed
-        num_tiles[chunk] = in_chunk;
-        ++chunk;
-        in_chunk = 0;
-      }
-      const int cend = min(m, (chunk + 1) * span);
       const int aend = cursor[a] + counts[a];
-      const int take = min(SKYRL_TILE_ROWS, min(aend, cend) - pos);
+      const int take = min(SKYRL_TILE_ROWS, aend - pos);
       int rows = take, second = 0;
-      if (take < SKYRL_TILE_ROWS && pos + take == aend && pos + take < cend) {
+      if (take < SKYRL_TILE_ROWS && pos + take == aend && aend < m) {
         int b = a + 1;
         while (b < num_adapters && counts[b] == 0) ++b;
         if (b < num_adapters) {
-          const int bend = cursor[b] + counts[b];
-          rows = take + min(SKYRL_TILE_ROWS - take, min(bend, cend) - (pos + take));
+          rows = take + min(SKYRL_TILE_ROWS - take, counts[b]);
           second = (b + 1) | (take << 16);
         }
       }
-      if (in_chunk < cap) {
-        reinterpret_cast<int4*>(tiles)[chunk * cap + in_chunk] = make_int4(pos, rows, a, second);
-      } else {
-        overflow = true;
-      }
-      ++in_chunk;
+      if (count < max_tiles) reinterpret_cast<int4*>(tiles)[count] = make_int4(pos, rows, a, second);
+      ++count;
       pos += rows;
       while (a < num_adapters && pos >= cursor[a] + counts[a]) ++a;  // the adapter that owns row `pos`
     }
-    num_tiles[chunk] = in_chunk;
-    for (int c = chunk + 1; c < num_chunks; ++c) num_tiles[c] = 0;
-    if (overflow) {
-      atomicCAS(status, 0, STATUS_TILE_OVERFLOW);
-      for (int c = 0; c < num_chunks; ++c) num_tiles[c] = 0;
-    }
+    num_tiles[0] = count <= max_tiles ? count : 0;
+    if (count > max_tiles) atomicCAS(status, 0, STATUS_TILE_OVERFLOW);
   }
   __syncthreads();
   if (tid < 32) {
@@ -131,8 +100,7 @@ route_kernel(const int32_t* __restrict__ ids, int m, int num_adapters, int32_t* 
 }
 
 int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int32_t* tiles, int32_t* num_tiles,
-                 int max_tiles, int32_t* status, cudaStream_t stream, int chunk_rows, int chunk_cap, int32_t* zero_words,
-                 int zero_count) {
+                 int max_tiles, int32_t* status, cudaStream_t stream) {
   if (m <= 0 || perm == nullptr || tiles == nullptr || num_tiles == nullptr || status == nullptr)
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: m must be positive and perm/tiles/num_tiles/status non-null");
   if (ids != nullptr && (num_adapters <= 0 || num_adapters > ROUTE_MAX_ADAPTERS))
@@ -140,14 +108,7 @@ int launch_route(const int32_t* ids, int m, int num_adapters, int32_t* perm, int
                 num_adapters);
   if (max_tiles <= 0 || !aligned16(tiles))
     return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: tiles must be 16-byte aligned with max_tiles > 0");
-  if (chunk_rows < 0 || chunk_rows % SKYRL_TILE_ROWS != 0 || (chunk_rows > 0 && chunk_cap <= 0))
-    return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: chunk_rows must be a multiple of %d", SKYRL_TILE_ROWS);
-  if (chunk_rows > 0 && static_cast<int64_t>((m + chunk_rows - 1) / chunk_rows) * chunk_cap > max_tiles)
-    return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: chunk lists do not fit in max_tiles");
-  if (zero_count < 0 || zero_count > ROUTE_THREADS)
-    return fail(SKYRL_ERR_INVALID_ARGUMENT, "route: at most %d words can be cleared", ROUTE_THREADS);
-  route_kernel<<<1, ROUTE_THREADS, 0, stream>>>(ids, m, num_adapters, perm, tiles, num_tiles, max_tiles, chunk_rows,
-                                                chunk_cap, status, zero_words, zero_count);
+  route_kernel<<<1, ROUTE_THREADS, 0, stream>>>(ids, m, num_adapters, perm, tiles, num_tiles, max_tiles, status);
   cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return fail(SKYRL_ERR_LAUNCH, "route launch: %s", cudaGetErrorString(e));
   return SKYRL_OK;
@@ -818,7 +779,7 @@ extern "C" int skyrl_lora_route_sm100_v1(const int32_t* adapter_ids, int32_t m, 
                                          int32_t* tiles, int32_t* num_tiles, int32_t max_tiles, int32_t* status,
                                          skyrl_stream_t stream) {
   return launch_route(adapter_ids, m, num_adapters, perm, tiles, num_tiles, max_tiles, status,
-                      static_cast<cudaStream_t>(stream), 0, 0, nullptr, 0);
+                      static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int skyrl_rms_quant_sm100_v1(const void* x, int64_t x_row_stride, const void* rms_delta, float eps,

@@ -82,7 +82,6 @@ struct GemmParams {
   int64_t slab_stride;  // elements between slabs of the int32 output
   int a_rows;       // rows of the activation TMA box (64 when the batch has at most 64 rows, else 128)
   int* sched;       // {tile claim counter, finished-CTA counter} of this launch, both zero on entry
-  int direct_stores;  // tuning aid: 1 = bf16 epilogues store from registers instead of through the staging tile
   // Row scatter of the fp32 partial sums (tensor-parallel reduce-scatter folded into the epilogue): row i of
   // the sorted order belongs to owner o = (i - scatter_row0) / scatter_rows and is written to
   // scatter_base[o] + (i - scatter_row0 - o * scatter_rows) * out_stride, which may be another GPU's memory
@@ -717,8 +716,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
     const int c_begin = warp < 4 ? 0 : (nchunks + 1) / 2;  // column chunks [c_begin, c_end) of the tile
     const int c_end = warp < 4 ? (nchunks + 1) / 2 : nchunks;
     const int r = quad * 32 + lane;  // row of the tile == TMEM lane
-    unsigned char* store_stage =
-        p.direct_stores ? nullptr : smem + SINGLE_STAGE_AREA + (warp < 4 ? warp : warp - 2) * EPI_STAGE_BYTES;
+    unsigned char* store_stage = smem + SINGLE_STAGE_AREA + (warp < 4 ? warp : warp - 2) * EPI_STAGE_BYTES;
     float* lterm = reinterpret_cast<float*>(smem + p.lterm_off);
     const bool rows_lora = ROWS && p.lora_rank_vecs > 0;
     const int ew = warp < 4 ? warp : warp - 2;  // 0 ... 7 among the epilogue warps
@@ -1808,7 +1806,6 @@ int launch_gemm(const SkyrlW8A8GemmArgs& a, cudaStream_t stream, bool programmat
       return fail(SKYRL_ERR_INVALID_ARGUMENT, "gemm: row_amax needs the SwiGLU epilogue and rows left in sorted order");
     p.row_amax = a.row_amax;
   }
-  p.direct_stores = 0;
   if (p.num_stages > MAX_STAGES) p.num_stages = MAX_STAGES;
   p.lora = LoraGeom{};
   if (lora)
