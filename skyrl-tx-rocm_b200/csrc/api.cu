@@ -230,7 +230,7 @@ struct Projection {
   bool keep_xn;           // sorted route: x must be re-laid out (gathered / normalised) for the projection MMA
   int m, n, k, rank, na;
   int q_row0, q_rows;     // sorted rows the quantiser stage covers (a chunk of the block, or all m rows)
-  int list_row0;          // first sorted row of the tile list `tiles` (0, or the first row of the call's chunk)
+  int list_row0;          // first sorted row of `src` (0, or the first row of the call's chunk)
   bool skip_quant;        // the quantiser stage of these rows already ran (its outputs are in xq / sx / z_parts)
   int gemm_variant;       // SKYRL_GEMM_VARIANT_* forced on the GEMM (0: the library chooses)
   bool two_step_rows;     // row-wise route: GEMM to an int32 accumulator in memory + finalize kernel (default)

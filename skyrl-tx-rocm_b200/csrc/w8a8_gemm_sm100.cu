@@ -17,10 +17,12 @@
 // the epilogue rewrites the int32 accumulator in place as dequantised fp32,
 // the MMA warp then issues the rank-r bf16 MMAs that accumulate z @ B^T onto
 // it, and the tile is read back a second time for the final cast.  The LoRA
-// operands (three z planes, one B tile) have no shared memory of their own
-// either: they travel through two slots of the same TMA pipeline, injected
-// into the stream of the NEXT tile's K blocks, so the whole buffer serves
-// pipeline depth (the main loop is bound by bytes in flight per SM).
+// operands have no shared memory of their own either: they travel through
+// slots of the same TMA pipeline, injected into the stream of the NEXT tile's
+// K blocks, so the whole buffer serves pipeline depth.  They come in rounds of
+// three z planes and the B tiles of as many adapters as there are slots left:
+// z slots + B slots of a round never exceed the pipeline's stages (LoraGeom),
+// so the planes can stay until the round's last MMA.
 //
 // Rows live in the adapter-sorted space: every 128-row M tile comes from the
 // tile list, whatever adapters its rows belong to (tiles.cuh); rows past the tile's
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
   uint64_t* empty_bar = bars + MAX_STAGES;
   uint64_t* tmem_full = bars + 2 * MAX_STAGES;        // [2]
   uint64_t* tmem_empty = tmem_full + 2;               // [2]
-  uint64_t* conv_done = tmem_empty + 2;               // 128 epilogue threads rewrote the accumulator
+  uint64_t* conv_done = tmem_empty + 2;               // all EPI_THREADS epilogue threads rewrote the accumulator
   uint64_t* lora_done = conv_done + 1;                // LoRA MMAs accumulated into TMEM
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + Cfg::NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
@@ -808,7 +810,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) w8a8_gemm_kernel(const __grid
 // (2 x 256 columns), so the epilogue of a pair is not overlapped with the next pair's main loop; it is
 // kept short instead by sixteen epilogue warps (two tiles x four lane quadrants x two column halves).
 // The two tiles of a pair are neighbours in the tile list and may belong to different adapters: each
-// gets its own LoRA operands (two pipeline slots per tile, issued right after the pair's K loop).
+// gets its own LoRA operands (rounds of pipeline slots as in the single-tile kernel, right after the pair's K loop).
 // ---------------------------------------------------------------------------------------------------
 constexpr int PAIR_THREADS = 576;      // warps 0-15 epilogue, warp 16 TMA producer, warp 17 MMA issuer
 constexpr int PAIR_EPI_THREADS = 512;
