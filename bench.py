@@ -667,7 +667,8 @@ def measure(args, workload, steps, rank, local_rank, world, device, dist, sub=Fa
     if wl["bound"] == "tensor":
         achieved = gu_ops_launch / (gu_avg * 1e-3) / 1e12
         traffic, traffic_note = load_traffic(workload, m_launch if kind == "mlp" else m) if tp == 1 else (None, None)
-        roofline = dict(bound="tensor", kernel="w8a8_gemm_kernel<gate_up/SwiGLU epilogue>" if kind in ("mlp", "gate_up") else "w8a8_gemm_kernel",
+        # the library chooses the kernel: CTA pair (w8a8_gemm_pair2_kernel) or single tile (w8a8_gemm_kernel)
+        roofline = dict(bound="tensor", kernel="w8a8_gemm_pair2_kernel or w8a8_gemm_kernel" + (" (gate_up, SwiGLU epilogue)" if kind in ("mlp", "gate_up") else ""),
                         achieved=achieved, peak=i8_peak, unit="TFLOP/s", frac=achieved / i8_peak,
                         traffic=traffic, traffic_unit="bytes per launch" + (f" ({traffic_note})" if traffic_note else ""),
                         algorithmic_bytes=gu_bytes_launch,
