@@ -12,6 +12,7 @@
 // of small bulk copies of their own.  The LoRA term has tensor-memory columns of its own (the accumulators never are
 // the sum it could be added to) and is added once, before the single cast.
 //
+// (ncu: the tensor pipe is busy 10 % of the time, ten warps issue on 42 % of the cycles, in dependent chains.)
 // Before, every group was a launch of its own into an fp32 slab: 262 launches and 3.16 ms for 512 x 4096 -> 4096 at
 // group 64; now four launches and 66 us, 48 of them in the GEMM.
 #include "common.cuh"

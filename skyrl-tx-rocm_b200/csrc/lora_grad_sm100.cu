@@ -4,7 +4,7 @@
 //   dB[a][j, n] = sum over the rows i of adapter a of  dy[i, n] * z[i, j]      z  = s (x A)
 //
 // (skyrl/tx/kernels/quantized_lora.py:374-389, the scaling already inside z and zb).  Both are tall contractions over
-// rows with a result of rank columns, so x and dy are read once and the work is HBM-bound: one CTA takes 128 columns of
+// rows with a result of rank columns, so x and dy are read once and the floor is their bytes: one CTA takes 128 columns of
 // x (or dy) and the rows of one adapter, multiplies 64 rows at a time on the tensor cores (both operands with the row
 // as the slow index in shared memory, i.e. MN-major) and keeps the 128 x rank result in tensor memory.  z and zb are
 // the bf16 parts the projection kernel leaves: the three parts sit side by side as one operand of 3 x rank columns and
@@ -15,7 +15,9 @@
 // last are filled with zeros.  Where tables and blocks are too few for the GPU, a cluster shares the rows of a block and
 // adds its partial sums in rank order through distributed shared memory.
 //
-// Before, a training step of eight adapters spent 150 launches of library matmuls, casts and additions here.
+// Before, a training step of eight adapters spent 150 launches of library matmuls, casts and additions here.  Now one launch,
+// 197 us at 4096 rows, K 12288, N 4096, rank 32, 8 adapters, for 138 MB (21 us): no unit is near its limit (DRAM 9 %, issue
+// 8 %), the loads of a stage wait for its row indices, and 1024 short CTAs pay fill and drain one after the other.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 
