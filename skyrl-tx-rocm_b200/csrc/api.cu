@@ -1251,7 +1251,10 @@ extern "C" int skyrl_w8a8_mlp_tp_finalize_slabs_sm100_v1(const SkyrlW8A8MlpArgs*
 // a handle for the symbol; the address kernels can use is looked up once per
 // device with cudaGetSymbolAddress and cached.
 // ---------------------------------------------------------------------------
-static __device__ __align__(256) unsigned char g_noalloc_scratch[SKYRL_NOALLOC_SCRATCH_BYTES];
+// Beside the documented size there is room for what the segments of dense tiles take more than the two-adapter tile list
+// they replaced (20 bytes a tile and 4 an adapter, at most 27 KB): whatever fitted before still does.
+constexpr size_t NOALLOC_ARRAY_BYTES = SKYRL_NOALLOC_SCRATCH_BYTES + (64u << 10);
+static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_ARRAY_BYTES];
 
 namespace skyrl {
 
@@ -1274,7 +1277,7 @@ static int noalloc_scratch(unsigned char** base, size_t* bytes) {
   const uintptr_t raw = reinterpret_cast<uintptr_t>(cached[dev]);
   const uintptr_t aligned = (raw + 1023u) & ~static_cast<uintptr_t>(1023u);
   *base = reinterpret_cast<unsigned char*>(aligned);
-  *bytes = SKYRL_NOALLOC_SCRATCH_BYTES - static_cast<size_t>(aligned - raw);
+  *bytes = NOALLOC_ARRAY_BYTES - static_cast<size_t>(aligned - raw);
   return SKYRL_OK;
 }
 

@@ -77,6 +77,27 @@ def test_noalloc_entry_point_matches_workspace_entry_point_twice():
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
 
 
+def test_noalloc_entry_point_takes_what_fitted_the_two_adapter_tile_lists():
+    """A need of 32 MiB less 1 KB then, 2 KB more than 32 MiB with the segments of dense tiles."""
+    import skyrl_tx_rocm_b200 as S
+    from skyrl_tx_rocm_b200 import _lib
+
+    lib = _lib.load()
+    m, k, n, adapters = 8717, 1024, 64, 256
+    x, w, lora, ids = _case(S, 5, m, k, n, 8, adapters)
+    nbytes = lib.skyrl_w8a8_linear_workspace_bytes(m, n, k, adapters)
+    assert nbytes > _lib.NOALLOC_SCRATCH_BYTES
+    want, got = (torch.empty((m, n), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    ws = torch.empty(nbytes + 1024, dtype=torch.uint8, device="cuda")
+    ws = ws[(-ws.data_ptr()) % 1024:][:nbytes]
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.skyrl_w8a8_lora_forward_sm100_v1(C.byref(_args(_lib, x, w, lora, ids, want, status, ws)), stream), "workspace")
+    _lib.check(lib.skyrl_w8a8_lora_forward_noalloc_sm100_v1(C.byref(_args(_lib, x, w, lora, ids, got, status)), stream), "noalloc")
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0] and torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 def test_noalloc_entry_point_rejects_oversized_requests():
     import skyrl_tx_rocm_b200 as S
     from skyrl_tx_rocm_b200 import _lib
