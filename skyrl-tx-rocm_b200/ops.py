@@ -410,8 +410,8 @@ def _scratch(device: torch.device, nbytes: int):
 
 
 def use_workspace(buffer: torch.Tensor | None, device=None) -> None:
-    """Make the operators of `buffer`'s device carve their scratch from `buffer` (uint8, CUDA) instead of a
-    memory of their own: a tensor-parallel stack registers a piece of peer-mapped (symmetric) memory here so
+    """Make the block calls and single projections of `buffer`'s device, on every stream, carve their scratch from
+    `buffer` (uint8, CUDA) instead of memory of their own: a tensor-parallel stack registers a piece of peer-mapped (symmetric) memory here so
     that other ranks can store the rows they prepared straight into this rank's workspace.  The operators
     raise if a call needs more than the buffer holds.  `None` releases the registration."""
     if buffer is None:
