@@ -292,9 +292,11 @@ class W8A8LoRALinearFunction(torch.autograd.Function):
         if ctx.needs_input_grad[3]:   # rarely wanted (alpha / r is a constant): library matmuls
             d_s = lora_parameter_grads(x.detach(), dy.contiguous(), lora_a.detach(), lora_b.detach(), lora_scaling.detach(), ids)[2]
             d_s = d_s.reshape(lora_scaling.shape).to(lora_scaling.dtype)
+        if lora_a.shape[-2] != k:   # a K that the packed weight rounds up to a multiple of 16
+            d_a = d_a[:, :lora_a.shape[-2]]
         if dx is not None:
-            dx = dx[:, :x.shape[-1]].reshape(x.shape)
-        return (dx, d_a[:, :lora_a.shape[-2]].reshape(lora_a.shape), d_b.reshape(lora_b.shape), d_s, None, None, None)
+            dx = (dx if x.shape[-1] == k else dx[:, :x.shape[-1]]).reshape(x.shape)
+        return (dx, d_a.reshape(lora_a.shape), d_b.reshape(lora_b.shape), d_s, None, None, None)
 
 
 def _tables(lora_a, lora_b, lora_scaling, k: int, n: int):
